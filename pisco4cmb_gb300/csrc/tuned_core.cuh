@@ -100,17 +100,24 @@ struct HasOutside<A, std::void_t<decltype(&A::outside)>> : std::true_type {};
 // over a workload is measured by pisco_tuned_calibrate and must stay well
 // below this bound.
 constexpr float kMarginRel = 1.2e-6f;
+// A ring batch whose longitude offsets all stay within this (radians) takes
+// the short series of sin and 1 - cos (short_sin_versin).
+constexpr float kShortOffset = 0.125f;
 // Pairs with 1 - cos(rho) below this take the reference's degenerate branch
 // (rho <= 1e-6, sphtrigo.cpp:40-48) and are done in FP64.
 constexpr float kTinyQ = 4.0e-12f;
 
 // One disc ring of the current batch: FP32 offset constants and the pixel
-// range(s), 64 bytes, read with four 16-byte loads.
+// range, 64 bytes, read with four 16-byte loads.  The sample's rotation by
+// psi and the beam grid's scale are in the constants, so a pair forms its
+// rotated beam-frame components with two multiply-adds each.
 struct alignas(16) RingC {
-    float dc, dphi, si, Di;  // anchor offset, pixel spacing, s, sin(dec - dec0)
-    float Ki, Zs, Wz, Pp;    // 1 - cos(dec - dec0), s z0, s0 z, s s0
-    int s1, s2, b1, b2;      // range starts, anchor offsets of the ranges (second: minus n1)
-    int n1, nr, incl, base;  // first range length, ring pixels, inclusive scan, first index
+    float dc, dphi, Ki, Pp;  // anchor offset, pixel spacing; R^2 (1 - cos(dec - dec0)), R^2 s s0
+    float Xs, Xh, Xc, Wz;    // s sin psi, -s z0 cos psi, -Di cos psi; s0 z
+    float Ys, Yh, Yc, Di;    // s cos psi, s z0 sin psi, Di sin psi; Di = sin(dec - dec0)
+    int j0;                  // ring index of flattened pair t: (j0 + t) mod nr
+    int nr, start;           // ring pixels, first pixel
+    int kc;                  // bits of 1.5 2^23 less the anchor's ring index
 };
 
 // Samples in flight per warp (a sample keeps its slot until its queued
@@ -145,7 +152,8 @@ struct alignas(16) SamplePlan {
     double phi_f, dec0;       // frame: longitude reduced mod 2 pi, latitude
     double cosr;              // disc: cos(radius) (the beam's, as evaluated on the device)
     float z0f, s0f;           // frame: sin and |cos| of the latitude
-    float sps, cps, c2p, s2p; // psi phasors (negated with the frame's flip)
+    float sps, cps;           // sin and cos of psi times a common factor (psi_phasor),
+                              // negated with the frame's flip
     int ring_lo, ring_hi;     // rings on the edge formula
     int full_lo, full_hi;     // rings touched
     int flags;                // kPlanBad: non-finite pointing; kPlanAllSky
@@ -159,6 +167,7 @@ constexpr int kPlanAllSky = 2;
 struct WarpSmem {
     SamplePlan plan;
     RingC r[32];
+    int incl[32];  // inclusive scan of the batch's pixel counts
     Pend p[kPend];
     int q[kQCap];
     unsigned char qs[kQCap];
@@ -213,11 +222,6 @@ __device__ __forceinline__ Beam make_beam(const F8* beam, int nside, int npix, d
     return b;
 }
 
-struct Frame {
-    double ra, dec, psi;
-    float s0, sps, cps, c2p, s2p;
-};
-
 __device__ __forceinline__ void record(unsigned int* err, unsigned int code)
 {
     if (err) atomicCAS(err, 0u, code);
@@ -232,28 +236,64 @@ __device__ __forceinline__ void two_sum(float& s, float& c, float x)
     c += e;
 }
 
-// x within m of an integer (x - rint(x) is exact for |x| < 2^23).
-__device__ __forceinline__ bool near_int(float x, float m)
+// Two FP32 values in one 64-bit register pair, added and subtracted by one
+// instruction each (the packed FP32 forms round every half as the scalar ones
+// do; they take one issue slot where two scalar instructions take two).
+using F32x2 = unsigned long long;
+__device__ __forceinline__ F32x2 pack2(float lo, float hi)
 {
-    return fabsf(x - rintf(x)) < m;
+    F32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(F32x2 v, float& lo, float& hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ F32x2 add2(F32x2 a, F32x2 b)
+{
+    F32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F32x2 sub2(F32x2 a, F32x2 b)
+{
+    F32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// two_sum of both halves
+__device__ __forceinline__ void two_sum2(F32x2& s, F32x2& c, F32x2 x)
+{
+    const F32x2 t = add2(s, x);
+    const F32x2 bp = sub2(t, s);
+    c = add2(c, add2(sub2(s, sub2(t, bp)), sub2(x, bp)));
+    s = t;
 }
 
-#ifndef PISCO_FAST_FLOOR
-#define PISCO_FAST_FLOOR 1
-#endif
 constexpr float kTwo23 = 8388608.0f;
 constexpr int kTwo23Bits = 0x4B000000;  // the bits of 2^23
 
 // floor(x) and its fractional part f = x - floor(x) for 0 <= x < 2^23 by
 // FP32 additions: x + 2^23 rounded down is 2^23 + floor(x) exactly (the
 // spacing of floats in [2^23, 2^24) is 1), and x - floor(x) is exact
-// (Sterbenz).  f < m or 1 - f < m is |x - rint(x)| < m (1 - f is exact for
-// f >= 1/2, and above 1/2 > m otherwise), so the decisions are near_int's.
+// (Sterbenz).
 __device__ __forceinline__ int split_floor(float x, float& f)
 {
     const float t = __fadd_rd(x, kTwo23);
     f = x - (t - kTwo23);
     return __float_as_int(t) - kTwo23Bits;
+}
+
+// The same with h = floor(x) + 1/2 (exact below 2^22) and f = x - h in
+// [-1/2, 1/2]: x lies within m of an integer exactly when |f| > 1/2 - m, one
+// comparison for both sides.  Returns the bits of 2^23 + floor(x).
+__device__ __forceinline__ int split_half(float x, float& h, float& f)
+{
+    const float t = __fadd_rd(x, kTwo23);
+    h = t - 8388607.5f;
+    f = x - h;
+    return __float_as_int(t);
 }
 
 // (float)k for |k| < 2^22 by FP32 addition: 1.5 * 2^23 + k lies in
@@ -276,6 +316,14 @@ __device__ __forceinline__ float rcp_approx(float x)
 {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// 1/sqrt(x) by the MUFU approximation (relative error below 2^-22).
+__device__ __forceinline__ float rsqrt_approx(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
@@ -337,18 +385,22 @@ __device__ __forceinline__ F8 load_beam_stencil(const F8* p)
 #endif
 }
 
-// The disc's pixel range(s) on one ring: FP32 edge angle, FP64 positions,
-// exact FP64 HEALPix formula (disc_ring) whenever an edge decision is within
-// the FP32 angle's error of a pixel boundary.  Same result as disc_ring.
-__device__ __forceinline__ RingSpan fast_disc_ring(const Hpx& h, const SamplePlan& p, double cosr,
-                                                   long long ring, const RingT& rt)
+// The disc's pixels on one ring, as ring indices lo .. lo + n - 1 (0 <= lo <
+// npix, wrapping at npix).
+struct RingRange {
+    int lo, n;
+};
+
+// FP32 edge angle, FP64 positions, exact FP64 HEALPix formula (disc_ring)
+// whenever an edge decision is within the FP32 angle's error of a pixel
+// boundary.  Same pixels as disc_ring.
+__device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePlan& p, double cosr,
+                                                    int ring, const RingT& rt)
 {
-    RingSpan s = {0, 0, 0, 0};
-    if (ring < p.full_lo || ring > p.full_hi) return s;
-    const long long npix = rt.npix2 >> 1;
+    RingRange s = {0, 0};
+    const int npix = rt.npix2 >> 1;
     if ((p.flags & kPlanAllSky) || ring < p.ring_lo || ring > p.ring_hi) {
-        s.start1 = rt.start;
-        s.n1 = npix;
+        s.n = npix;
         return s;
     }
     const double x = PD_MUL(PD_SUB(cosr, PD_MUL(rt.z, p.z0)), p.xa);
@@ -373,24 +425,16 @@ __device__ __forceinline__ RingSpan fast_disc_ring(const Hpx& h, const SamplePla
         d.full_lo = p.full_lo;
         d.full_hi = p.full_hi;
         d.all_sky = (p.flags & kPlanAllSky) != 0;
-        return disc_ring(h, d, ring);
+        const RingSpan e = disc_ring(h, d, ring);
+        s.lo = (int)((e.n2 > 0 ? e.start2 : e.start1) - rt.start);
+        s.n = (int)(e.n1 + e.n2);
+        if (s.n <= 0) s = RingRange{0, 0};
+        return s;
     }
-    long long lo = (long long)floor(vlo) + 1;
-    long long hi = (long long)floor(vhi);
+    const int lo = (int)floor(vlo) + 1, hi = (int)floor(vhi);
     if (lo > hi) return s;
-    if (hi >= npix) {
-        lo -= npix;
-        hi -= npix;
-    }
-    if (lo < 0) {
-        s.start1 = rt.start;
-        s.n1 = hi + 1;
-        s.start2 = rt.start + lo + npix;
-        s.n2 = -lo;
-    } else {
-        s.start1 = rt.start + lo;
-        s.n1 = hi - lo + 1;
-    }
+    s.lo = lo < 0 ? lo + npix : (lo >= npix ? lo - npix : lo);
+    s.n = hi - lo + 1;
     return s;
 }
 
@@ -706,27 +750,69 @@ __device__ __forceinline__ void sin_versin(float x, float& sn, float& h)
     }
 }
 
-// atan2(y, x) / (pi/2) for y, x >= 0, in [0, 1]: the arctangent of the
-// ratio min/max by the minimax polynomial of Abramowitz & Stegun 4.4.49
-// (|error| <= 2e-8 on [0, 1]; 1e-7 when evaluated in FP32), reflected for
-// y > x.  y = x = 0 gives 0 (such pairs are re-done in FP64 anyway).
-__device__ __forceinline__ float quarter_turns(float y, float x)
+// The same for |x| <= kShortOffset, two terms fewer each (truncation below
+// 8e-10 relative, an eightieth of an FP32 ulp).
+__device__ __forceinline__ void short_sin_versin(float x, float& sn, float& h)
 {
-    const bool swap = y > x;
-    const float mn = swap ? x : y, mx = swap ? y : x;
-    const float t = mx > 0.0f ? __fdividef(mn, mx) : 0.0f;
+    const float x2 = x * x;
+    sn = x * fmaf(x2, fmaf(x2, 8.33333333e-3f, -1.66666667e-1f), 1.0f);
+    h = x2 * fmaf(x2, fmaf(x2, 1.38888889e-3f, -4.16666667e-2f), 0.5f);
+}
+
+// Fraction of the quadrant, atan2(yy, xx) / (pi/2) in [0, 1], of the
+// direction (X, Y): yy, xx = |Y|, |X| where the signs agree (quadrants 0 and
+// 2) and |X|, |Y| where they differ (1 and 3); sgn is the sign bit of X Y.
+// As 1/2 + (2/pi) atan(t), t = (yy - xx) / (yy + xx) in [-1, 1]: no swap of
+// numerator and denominator, so no comparison or selection.  The arctangent
+// is the minimax polynomial of Abramowitz & Stegun 4.4.49 (|error| <= 2e-8),
+// its coefficients times 2/pi; clamped to [0, 1].  X = Y = 0 gives a NaN
+// (such pairs are re-done in FP64 anyway).
+__device__ __forceinline__ float quarter_turns(float X, float Y, unsigned sgn)
+{
+    const float d = __uint_as_float(__float_as_uint(fabsf(Y) - fabsf(X)) ^ sgn);
+    const float t = d * rcp_approx(fabsf(X) + fabsf(Y));
     const float t2 = t * t;
-    float p = 0.0028662257f;
-    p = fmaf(p, t2, -0.0161657367f);
-    p = fmaf(p, t2, 0.0429096138f);
-    p = fmaf(p, t2, -0.0752896400f);
-    p = fmaf(p, t2, 0.1065626393f);
-    p = fmaf(p, t2, -0.1420889944f);
-    p = fmaf(p, t2, 0.1999355085f);
-    p = fmaf(p, t2, -0.3333314528f);
-    p = fmaf(p, t2, 1.0f);
-    const float a = t * p * 0.63661977236758134f;  // atan(t) / (pi/2)
-    return swap ? 1.0f - a : a;
+    constexpr double q = 0.63661977236758134;
+    float p = (float)(q * 0.0028662257);
+    p = fmaf(p, t2, (float)(q * -0.0161657367));
+    p = fmaf(p, t2, (float)(q * 0.0429096138));
+    p = fmaf(p, t2, (float)(q * -0.0752896400));
+    p = fmaf(p, t2, (float)(q * 0.1065626393));
+    p = fmaf(p, t2, (float)(q * -0.1420889944));
+    p = fmaf(p, t2, (float)(q * 0.1999355085));
+    p = fmaf(p, t2, (float)(q * -0.3333314528));
+    p = fmaf(p, t2, (float)q);
+    return __saturatef(fmaf(t, p, 0.5f));
+}
+
+// (sin psi, cos psi) times a common factor near 1, in FP32, with the angle
+// kept to about 2e-9: the rotation by psi multiplies every pair of a sample,
+// so the rounding error of its angle is coherent over the sample's sum (an
+// FP32 pair rounded once is off by up to 4e-8).  The uses are ratios, so the
+// factor drops out.  The larger component runs over eight FP32 values; the
+// one whose partner rounds best is kept.
+__device__ __forceinline__ void psi_phasor(double s, double c, float& sf, float& cf)
+{
+    const bool swap = fabs(s) > fabs(c);
+    const double big = swap ? s : c, small = swap ? c : s;
+    const double ratio = small / big;
+    const float b0 = (float)big;
+    float bb = b0, bs = (float)(ratio * (double)b0);
+    float best = 1.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float b = b0 * (1.0f - 0.03125f * (float)i);
+        const double p = ratio * (double)b;
+        const float r = (float)p;
+        const float e = fabsf((float)(p - (double)r)) / fabsf(b);
+        if (e < best) {
+            best = e;
+            bb = b;
+            bs = r;
+        }
+    }
+    sf = swap ? bb : bs;
+    cf = swap ? bs : bb;
 }
 
 __device__ __forceinline__ SamplePlan make_plan(const Hpx& hs, const Beam& B, double ra,
@@ -769,14 +855,9 @@ __device__ __forceinline__ SamplePlan make_plan(const Hpx& hs, const Beam& B, do
     }
     sp.z0f = (float)z0d;
     sp.s0f = (float)s0d;
-    // psi phasors in FP64, rounded once: exp(2i psi) multiplies every pair
-    // of the sample, so its rounding error is coherent over the sample sum.
     double spsi, cpsi;
     sincos(psi, &spsi, &cpsi);
-    sp.sps = (float)(flip ? -spsi : spsi);
-    sp.cps = (float)(flip ? -cpsi : cpsi);
-    sp.c2p = (float)__fma_rn(cpsi, cpsi, -__dmul_rn(spsi, spsi));
-    sp.s2p = (float)__dmul_rn(__dmul_rn(2.0, spsi), cpsi);
+    psi_phasor(flip ? -spsi : spsi, flip ? -cpsi : cpsi, sp.sps, sp.cps);
     sp.z0 = P.z0;
     sp.xa = P.xa;
     sp.phi = P.phi;
@@ -806,10 +887,6 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
 {
     RingC* W = S.r;
     const unsigned lt_mask = (1u << lane) - 1u;
-    Frame F;
-    F.ra = ra;
-    F.dec = dec;
-    F.psi = -pa;
     if (SP.flags & kPlanBad) {
         if (Action::kSums && lane == 0) {
             store_out(o.a, o.f64, o.idx, CUDART_NAN);
@@ -825,9 +902,9 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
     if (lane == 0) {
         Pend& Ps = S.p[slot];
         Ps.hb = hb;
-        Ps.ra = F.ra;
-        Ps.dec = F.dec;
-        Ps.psi = F.psi;
+        Ps.ra = ra;
+        Ps.dec = dec;
+        Ps.psi = -pa;
         Ps.fb_a = Ps.fb_b = 0.0;
         Ps.beam = B.beam;
         Ps.out_a = o.a;
@@ -846,36 +923,32 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
     if constexpr (Action::kSums) act.reset();
     const SamplePlan& PL = S.plan;
     // what the pair loop reads on every pair, in registers
-    F.s0 = PL.s0f;
-    F.sps = PL.sps;
-    F.cps = PL.cps;
-    F.c2p = PL.c2p;
-    F.s2p = PL.s2p;
-    const Beam& Bh = B;
+    const float s0 = PL.s0f;
+    const float tiny = kTinyQ * (B.rscale * B.rscale);
 
-    for (long long r0 = PL.full_lo; r0 <= PL.full_hi; r0 += 32) {
-        const long long ring = r0 + lane;
+    for (int r0 = PL.full_lo; r0 <= PL.full_hi; r0 += 32) {
+        const int ring = r0 + lane;
         int cnt = 0;
+        bool wide = false;
         RingC rc;
-        rc.n1 = 0;
         if (ring <= PL.full_hi) {
             const RingT rt = rings[ring - 1];
-            RingSpan sp = fast_disc_ring(hs, PL, PL.cosr, ring, rt);
-            // every pixel of the ring's range(s) must lie in the sky map:
+            RingRange sp = fast_disc_ring(hs, PL, PL.cosr, ring, rt);
+            const int nr = rt.npix2 >> 1;
+            // every pixel of the ring's range must lie in the sky map:
             // checked here, once per ring, instead of once per pair
-            if (sp.start1 < 0 || sp.start1 + sp.n1 > hs.npix ||
-                (sp.n2 > 0 && (sp.start2 < 0 || sp.start2 + sp.n2 > hs.npix))) {
+            if (sp.lo < 0 || sp.lo >= nr || sp.n < 0 || sp.n > nr || rt.start < 0 ||
+                rt.start + (long long)nr > hs.npix) {
                 record(err, kCheckSkyIndex);
-                sp = RingSpan{0, 0, 0, 0};
+                sp = RingRange{0, 0};
             }
-            cnt = (int)(sp.n1 + sp.n2);
+            cnt = sp.n;
             if (cnt) {
                 const double sh = (rt.npix2 & 1) ? 0.5 : 0.0;
                 const double phi_f = PL.phi_f;
                 const double jc = floor(phi_f * rt.fr - sh + 0.5);
                 rc.dc = (float)((jc + sh) * rt.dphi - phi_f);
                 rc.dphi = rt.dphif;
-                rc.si = rt.s;
                 // sin and 1 - cos of the latitude offset D: FP32 series at the
                 // rounded offset, first-order correction by its rounding error
                 const double dd = rt.dec - PL.dec0;
@@ -883,18 +956,37 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 const float de = (float)(dd - (double)df);
                 float sD, hD;
                 sin_versin(df, sD, hD);
-                rc.Di = fmaf(de, 1.0f - hD, sD);
-                rc.Ki = fmaf(de, sD, hD);
-                rc.Zs = rt.s * PL.z0f;
+                const float Di = fmaf(de, 1.0f - hD, sD);
+                const float Zs = rt.s * PL.z0f;
+                const float R2 = B.rscale * B.rscale;
+                rc.Ki = R2 * fmaf(de, sD, hD);
+                rc.Pp = R2 * (rt.s * PL.s0f);
                 rc.Wz = PL.s0f * rt.zf;
-                rc.Pp = rt.s * PL.s0f;
-                rc.nr = rt.npix2 >> 1;
-                rc.b1 = (int)(sp.start1 - rt.start) - (int)jc;
-                rc.b2 = (int)(sp.start2 - rt.start) - (int)jc - (int)sp.n1;
+                rc.Di = Di;
+                rc.Xs = rt.s * PL.sps;
+                rc.Xh = -Zs * PL.cps;
+                rc.Xc = -Di * PL.cps;
+                rc.Ys = rt.s * PL.cps;
+                rc.Yh = Zs * PL.sps;
+                rc.Yc = Di * PL.sps;
+                rc.nr = nr;
+                rc.start = rt.start;
+                // offsets from the anchor, the range centred on it; a whole
+                // ring starts half a turn from it
+                if (cnt == nr) {
+                    int lo = (int)jc - (nr >> 1);
+                    lo += lo < 0 ? nr : 0;
+                    sp.lo = lo >= nr ? lo - nr : lo;
+                }
+                int kk = sp.lo - (int)jc;
+                const int mid = kk + (cnt >> 1);
+                if (mid >= (nr >> 1) + 1) kk -= nr;
+                else if (mid < -(nr >> 1)) kk += nr;
+                rc.kc = 0x4B400000 + kk - sp.lo;
+                rc.j0 = sp.lo;
+                const int far = max(-kk, kk + cnt);
+                wide = (float)far * rt.dphif > kShortOffset - rt.dphif;
             }
-            rc.n1 = (int)sp.n1;
-            rc.s1 = (int)sp.start1;
-            rc.s2 = (int)sp.start2 - (int)sp.n1;
         }
         int incl = cnt;
 #pragma unroll
@@ -903,9 +995,10 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
             if (lane >= o) incl += v;
         }
         const int total = __shfl_sync(kFull, incl, 31);
-        rc.incl = incl;
-        rc.base = incl - cnt;
+        rc.j0 -= incl - cnt;
         W[lane] = rc;
+        S.incl[lane] = incl;
+        const bool narrow = !__any_sync(kFull, wide);
         __syncwarp();
         if (lane == 0) npairs += (unsigned long long)total;
         int k = 0;  // lane slot (ring) owning the current pair; only moves forward
@@ -915,56 +1008,45 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
             bool fb = false;
             int pix = 0;
             if (t < total) {
-                while (W[k].incl <= t) ++k;
-                const int4 R2 = *reinterpret_cast<const int4*>(&W[k].s1);
-                const int4 R3 = *reinterpret_cast<const int4*>(&W[k].n1);
-                const int u = t - R3.w;  // index within the ring's pixels
-                const bool first = u < R3.x;
-                pix = (first ? R2.x : R2.y) + u;
-                int kk = (first ? R2.z : R2.w) + u;
-                const int nr = R3.y;
-                if (kk >= (nr >> 1)) kk -= nr;
-                if (kk < -(nr >> 1)) kk += nr;
+                while (S.incl[k] <= t) ++k;
+                const int4 R3 = *reinterpret_cast<const int4*>(&W[k].j0);
+                const int j = R3.x + t;  // ring index, below 2 nr
+                pix = R3.z + (int)min((unsigned)j, (unsigned)(j - R3.y));
+                const float kf = __int_as_float(R3.w + j) - 12582912.0f;  // offset from the anchor
                 {
                     const float4 R0 = *reinterpret_cast<const float4*>(&W[k].dc);
-                    const float4 R1 = *reinterpret_cast<const float4*>(&W[k].Ki);
-                    const float dl = fmaf(small_int_to_float(kk), R0.y, R0.x);
+                    const float4 R1 = *reinterpret_cast<const float4*>(&W[k].Xs);
+                    const float4 R2 = *reinterpret_cast<const float4*>(&W[k].Ys);
+                    const float dl = fmaf(kf, R0.y, R0.x);
                     float sn, h;
-                    sin_versin(dl, sn, h);
-                    const float u_e = R0.z * sn;
-                    const float v_n = fmaf(R1.y, h, R0.w);
-                    const float q = fmaf(R1.w, h, R1.x);
-                    const float nb = F.s0 * sn;
-                    const float db = fmaf(R1.z, h, -R0.w);
-                    const float X = fmaf(u_e, F.sps, -v_n * F.cps);
-                    const float Y = fmaf(u_e, F.cps, v_n * F.sps);
-                    int qd;
-                    float yy, xx;
-                    if (Y >= 0.0f) {
-                        if (X > 0.0f) { qd = 0; yy = Y; xx = X; }
-                        else { qd = 1; yy = -X; xx = Y; }
-                    } else {
-                        if (X <= 0.0f) { qd = 2; yy = -Y; xx = -X; }
-                        else { qd = 3; yy = X; xx = -Y; }
-                    }
-                    const float tp = quarter_turns(yy, xx);
-                    const float r = Bh.rscale * (q * rsqrtf(q));
-                    // exp(2i (beta + alpha)) = w^2 / |w|^2, w = (db + i nb)(v + i u),
-                    // then rotated by exp(2i psi)
+                    if (narrow) short_sin_versin(dl, sn, h);
+                    else sin_versin(dl, sn, h);
+                    const float q = fmaf(R0.w, h, R0.z);  // R^2 (1 - cos rho)
+                    const float X = fmaf(sn, R1.x, fmaf(h, R1.y, R1.z));
+                    const float Y = fmaf(sn, R2.x, fmaf(h, R2.y, R2.z));
+                    const unsigned sgn =
+                        (__float_as_uint(X) ^ __float_as_uint(Y)) & 0x80000000u;
+                    const int qd = (int)(2u * (__float_as_uint(Y) >> 31) + (sgn >> 31));
+                    const float tp = quarter_turns(X, Y, sgn);
+                    const float r = q * rsqrt_approx(q);
+                    // exp(2i chi) = w^2 / |w|^2, w = (db + i nb)(X - i Y): the
+                    // direction to the boresight times the rotated beam-frame
+                    // direction (an overall sign drops out)
                     auto phasor = [&](float& c2, float& s2) {
-                        const float wr = fmaf(db, v_n, -nb * u_e);
-                        const float wi = fmaf(db, u_e, nb * v_n);
-                        const float iw = rcp_approx(fmaf(wr, wr, wi * wi));
-                        const float er = fmaf(wr, wr, -wi * wi) * iw;
-                        const float ei = 2.0f * wr * wi * iw;
-                        c2 = fmaf(er, F.c2p, -ei * F.s2p);
-                        s2 = fmaf(ei, F.c2p, er * F.s2p);
+                        const float nb = s0 * sn;
+                        const float db = fmaf(R1.w, h, -R2.w);
+                        const float wr = fmaf(db, X, nb * Y);
+                        const float wi = fmaf(nb, X, -(db * Y));
+                        const float ww = wr * wr;
+                        const float iw = rcp_approx(fmaf(wi, wi, ww));
+                        c2 = fmaf(-wi, wi, ww) * iw;
+                        s2 = wr * wi * (iw + iw);
                     };
                     if constexpr (kBil && Action::kStencil) {
-                        fb = q < kTinyQ;
+                        fb = q < tiny;
                         int px[4];
                         float w[4];
-                        if (!fb && stencil_f32(Bh, qd, tp, r, px, w)) {
+                        if (!fb && stencil_f32(B, qd, tp, r, px, w)) {
                             float c2, s2;
                             phasor(c2, s2);
                             act.pair_stencil(pix, act.fetch(pix), px, w, c2, s2);
@@ -972,9 +1054,9 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                             if (!fb) act.outside(pix, -1);
                         }
                     } else if constexpr (kBil) {
-                        fb = q < kTinyQ;
+                        fb = q < tiny;
                         F8 Bv;
-                        if (!fb && bilinear_f32(Bh, qd, tp, r, Bv)) {
+                        if (!fb && bilinear_f32(B, qd, tp, r, Bv)) {
                             float c2, s2;
                             phasor(c2, s2);
                             act.pair(pix, act.fetch(pix), Bv, -1, c2, s2);
@@ -982,48 +1064,39 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                             if (!fb) act.outside(pix, -1);
                         }
                     } else {
+                        // ang2pix of the polar cap: jp = floor(tp r), jm =
+                        // floor((1 - tp) r), ring ir = jp + jm + 1, position
+                        // floor(tp ir) in the quadrant; a value within the
+                        // margin of an integer sends the pair to FP64
                         const float av = tp * r;
-                        const float bv = (1.0f - tp) * r;
-#if PISCO_FAST_FLOOR
-                        // floors and fractional parts by FP32 additions (no
-                        // conversion instructions), the same values as the
-                        // conversions: see split_floor
-                        float fa, fbv, fc;
-                        const int jp = split_floor(av, fa), jm = split_floor(bv, fbv);
-                        const int ir = jp + jm + 1;
-                        const float irf = __int_as_float(ir + kTwo23Bits) - kTwo23;
+                        const float bv = fmaf(-tp, r, r);
+                        float ha, fa, hv, fv, hc, fc;
+                        const int ja = split_half(av, ha, fa), jb = split_half(bv, hv, fv);
+                        const float irf = ha + hv;
                         const float cv = tp * irf;
-                        const int ipr = split_floor(cv, fc);
-                        const float m = kMarginRel * (r + 1.0f);
-                        const float mc = kMarginRel * (irf + 1.0f);
-                        fb = q < kTinyQ || fa < m || 1.0f - fa < m || fbv < m ||
-                             1.0f - fbv < m || fc < mc || 1.0f - fc < mc;
-#else
-                        const int jp = (int)av, jm = (int)bv;
-                        const int ir = jp + jm + 1;
-                        const float cv = tp * (float)ir;
-                        const int ipr = (int)cv;
-                        const float m = kMarginRel * (r + 1.0f);
-                        fb = q < kTinyQ || near_int(av, m) || near_int(bv, m) ||
-                             near_int(cv, kMarginRel * ((float)ir + 1.0f));
-#endif
+                        const int jc = split_half(cv, hc, fc);
+                        // 1/2 less kMarginRel (r + 2), and r + 1 >= ir
+                        const float edge = fmaf(-kMarginRel, r, 0.5f - 2.0f * kMarginRel);
+                        fb = q < tiny || fmaxf(fmaxf(fabsf(fa), fabsf(fv)), fabsf(fc)) > edge;
+                        const int ir = (ja - kTwo23Bits) + (jb - kTwo23Bits) + 1;
                         if (kCalib && !fb) {
                             double rho, sig, chi;
-                            (void)pair_beam_pixel(hs, hb, pix, F.ra, F.dec, F.psi, &rho, &sig, &chi);
+                            (void)pair_beam_pixel(hs, hb, pix, ra, dec, -pa, &rho, &sig, &chi);
                             const double tt = fmodulo(sig * kInvHalfPi, 4.0);
                             const double tpd = tt - floor(tt);
-                            const double rd = (double)Bh.nside * sqrt(3.0 * (1.0 - cos(rho)));
+                            const double rd = (double)B.nside * sqrt(3.0 * (1.0 - cos(rho)));
                             const double e1 = fabs(av - tpd * rd) / (r + 1.0);
                             const double e2 = fabs(bv - (1.0 - tpd) * rd) / (r + 1.0);
                             const double e3 = fabs(cv - tpd * (double)ir) / ((double)ir + 1.0);
                             cmax = fmaxf(cmax, (float)fmax(fmax(e1, e2), e3) / kMarginRel);
                         }
                         if (!fb) {
-                            const int bp = 2 * ir * (ir - 1) + qd * ir + ipr;
-                            if ((unsigned)bp < (unsigned)Bh.npix) {  // 0 <= bp < npix
+                            // 2 ir (ir - 1) + qd ir + position
+                            const int bp = ir * (2 * ir - 2 + qd) + (jc - kTwo23Bits);
+                            if ((unsigned)bp < (unsigned)B.npix) {  // 0 <= bp < npix
                                 float c2, s2;
                                 phasor(c2, s2);
-                                act.pair(pix, act.fetch(pix), load_beam(Bh.beam + bp), bp, c2, s2);
+                                act.pair(pix, act.fetch(pix), load_beam(B.beam + bp), bp, c2, s2);
                             } else if constexpr (HasOutside<Action>::value) {
                                 act.outside(pix, bp);
                             }
@@ -1078,28 +1151,28 @@ __device__ __forceinline__ void sample(const Hpx& hs, const RingT* rings, const 
                                  S, Qs, lane, err, act, nfall, cmax, npairs);
 }
 
-// Forward action: gather the sky, multiply by the beam, compensated sums.
+// Forward action: gather the sky, multiply by the beam, compensated sums of
+// both detectors side by side (two_sum2).
 struct Gather {
     static constexpr bool kSums = true;
     static constexpr bool kStencil = false;
     const float4* sky;
-    float sa, ca, sb, cb;
-    __device__ __forceinline__ void reset() { sa = ca = sb = cb = 0.0f; }
+    F32x2 sum, cmp;  // halves: detector a, detector b
+    __device__ __forceinline__ void reset() { sum = cmp = pack2(0.0f, 0.0f); }
     __device__ __forceinline__ float4 fetch(int pix) const { return __ldg(&sky[pix]); }
+    // the sky's polarisation turned into the beam's frame once for both detectors
     __device__ __forceinline__ static void contrib(const float4& S, const F8& B, float c2, float s2,
                                                   float& ta, float& tb)
     {
-        ta = S.x * B.a.x + S.y * (B.a.y * c2 - B.a.z * s2) + S.z * (B.a.z * c2 + B.a.y * s2) +
-             S.w * B.a.w;
-        tb = S.x * B.b.x + S.y * (-B.b.y * c2 + B.b.z * s2) + S.z * (-B.b.z * c2 - B.b.y * s2) +
-             S.w * B.b.w;
+        const float q = fmaf(S.y, c2, S.z * s2), u = fmaf(S.z, c2, -(S.y * s2));
+        ta = fmaf(u, B.a.z, fmaf(q, B.a.y, fmaf(S.w, B.a.w, S.x * B.a.x)));
+        tb = fmaf(-u, B.b.z, fmaf(-q, B.b.y, fmaf(S.w, B.b.w, S.x * B.b.x)));
     }
     __device__ __forceinline__ void pair(int, const float4& S, const F8& B, int, float c2, float s2)
     {
         float ta, tb;
         contrib(S, B, c2, s2, ta, tb);
-        two_sum(sa, ca, ta);
-        two_sum(sb, cb, tb);
+        two_sum2(sum, cmp, pack2(ta, tb));
     }
     __device__ __forceinline__ void stash(Pend&) const {}
     __device__ __forceinline__ void deferred(const Pend&, int pix, const F8& B, int, float c2, float s2,
@@ -1110,6 +1183,9 @@ struct Gather {
     // warp total (fixed shuffle tree: deterministic)
     __device__ __forceinline__ void total(double& a, double& b) const
     {
+        float sa, sb, ca, cb;
+        unpack2(sum, sa, sb);
+        unpack2(cmp, ca, cb);
         a = (double)sa + (double)ca;
         b = (double)sb + (double)cb;
 #pragma unroll
