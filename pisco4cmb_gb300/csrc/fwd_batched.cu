@@ -82,23 +82,22 @@ __global__ void batched_plan_kernel(BatchArgs a)
     }
 }
 
-// Warps per SM of an instance: the planned nearest lookup runs 32 (register
-// cap 64: its per-sample plan and the descriptors are in shared memory, as in
-// the single-detector launch), the others 16 (cap 128).
-template <bool kBil, bool kPlanned>
+// Warps per SM of an instance.  The planned nearest lookup takes two pixels
+// per lane (tuned_core.cuh): 20 warps at 96 registers in blocks of 4, 24 at 80
+// in blocks of 8 (two blocks of 8 would leave 16: 48 pairs, 1.2M samples,
+// 22.4 ms against 25.3 ms), one block of 16.  The others run 16 (cap 128).
+template <bool kBil, bool kPlanned, int kW>
 constexpr int warps_per_sm()
 {
-    return kPlanned && !kBil ? 32 : 16;
+    return kPlanned && !kBil ? (kW == 4 ? 20 : (kW == 8 ? 24 : 16)) : 16;
 }
 
 // kBil: bilinear beam lookup (tuned_core.cuh bilinear_f32).  kW: warps per
-// block, the tile the autotuner picks with the chunk size; every tile of an
-// instance keeps the same warps per SM (warps_per_sm / kW blocks), so all
-// compile to the same register cap and differ in how many warps share an
-// item (and its samples' discs).  kPlanned: the samples' plans come from
-// batched_plan_kernel.
+// block, the tile the autotuner picks with the chunk size: how many warps
+// share an item (and its samples' discs).  kPlanned: the samples' plans come
+// from batched_plan_kernel.
 template <bool kBil, int kW, bool kPlanned>
-__global__ void __launch_bounds__(kW * 32, warps_per_sm<kBil, kPlanned>() / kW)
+__global__ void __launch_bounds__(kW * 32, warps_per_sm<kBil, kPlanned, kW>() / kW)
     batched_kernel(BatchArgs a)
 {
     constexpr int kBW = kW;
@@ -113,8 +112,9 @@ __global__ void __launch_bounds__(kW * 32, warps_per_sm<kBil, kPlanned>() / kW)
     const Hpx& hs = s_hs;
     unsigned long long nfall = 0, npairs = 0;
     float cmax = 0.0f;
-    tuned::Gather g;
+    tuned::Gather<(warps_per_sm<kBil, kPlanned, kW>() <= 20)> g;
     g.sky = a.sky32;
+    g.wide = (reinterpret_cast<size_t>(a.sky32) & 31) == 0;
     tuned::Queue Q{0, 0};
     for (int round = 0;; ++round) {
         // double-buffered: a slot is rewritten only after the next barrier,

@@ -14,22 +14,17 @@
 namespace pisco {
 namespace {
 
-// Launch shape: the nearest lookup runs one block of 32 warps per SM
-// (register cap 64).  The kernel is latency-bound, and with each sample's
-// plan (WarpSmem::plan) and the grids' and beam's descriptors in shared
-// memory, read where needed, its pair loop fits 64 registers with little
-// spilling, so eight warps per scheduler hide what four could not (c2
-// forward: 129.9 ms, against 169.7 ms for 16 warps at 128 registers; with
-// the descriptors in registers 20 warps gave 162.1 ms and 24 warps, spilling
-// inside the loop, 174.6 ms).  The 32 warps work on consecutive samples,
-// whose discs overlap, so their sky reads share L1.  Its 169 KB of per-warp
-// shared state is a static allocation, which sm_103a allows beyond 48 KB.
-// The bilinear lookup, which needs more registers per pair, runs 8 x 2 with
-// its descriptors in registers (296.3 ms; from shared memory 374.1 ms).  For
-// the nearest lookup the beam's descriptor in registers (its pointer and size
-// then come from the kernel parameters) is slower: 133.4 against 120.4 ms.
+// Launch shape: the nearest lookup runs one block of 20 warps per SM (register
+// cap 96, no spills), two pixels per lane: its pair loop is bound by the L1
+// pipe (94 % busy at 1.1 MB of beam: the beam gather, the sky and the rings'
+// constants), and 20 warps leave L1 156 KB.  100,000 samples of nside 1024 and
+// a 3 degree beam: 16 warps 4.53 ms, 20 warps 4.31 ms, 24 warps (80 registers,
+// spilling) 4.47 ms; one pixel per lane at 32 warps of 64 registers took 5.2
+// ms.  The warps of a block work on consecutive samples, whose discs overlap,
+// so their sky reads share L1.  The bilinear lookup, which needs more
+// registers per pair, runs 8 x 2 with its descriptors in registers.
 #ifndef PISCO_FWD_WARPS
-#define PISCO_FWD_WARPS 32
+#define PISCO_FWD_WARPS 20
 #endif
 #ifndef PISCO_BIL_WARPS
 #define PISCO_BIL_WARPS 8
@@ -39,12 +34,12 @@ namespace {
 // kTW: warps per block (fwd_warps_per_sm / kTW blocks per SM).
 // Positions [pos0, pos1) of the launch.  kPlanned: plans holds their sample
 // plans (index position - pos0); otherwise each warp builds its own.
-// Warps per SM: 32 for the planned nearest lookup (register cap 64), 16 for
+// Warps per SM: 20 for the planned nearest lookup (register cap 96), 16 for
 // the others (cap 128).
 template <bool kCalib, bool kBil, bool kPlanned>
 constexpr int fwd_warps_per_sm()
 {
-    return kPlanned && !kBil && !kCalib ? 32 : 16;
+    return kPlanned && !kBil && !kCalib ? PISCO_FWD_WARPS : 16;
 }
 
 template <bool kCalib, bool kBil, int kTW, bool kPlanned>
@@ -56,10 +51,10 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
     const int lane = threadIdx.x & 31;
     tuned::WarpSmem& S = sm[threadIdx.x >> 5];
     // The nearest lookup keeps the grids' and the beam's descriptors in
-    // shared memory, read where needed rather than held in registers across
-    // the pair loop: at its 64-register cap (32 warps per SM) that leaves the
-    // registers to the pair geometry.  The bilinear lookup, which reads the
-    // beam descriptor on every stencil pixel, keeps them in registers.
+    // shared memory, read once per sample rather than held in registers across
+    // the pair loop, which leaves those to the pair geometry.  The bilinear
+    // lookup, which reads the beam descriptor on every stencil pixel, keeps
+    // them in registers.
     constexpr bool kDescSmem = !kBil;
     __shared__ Hpx s_hs, s_hb;
     __shared__ tuned::Beam s_B;
@@ -81,8 +76,9 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
     const long long nw = (long long)gridDim.x * kTW;
     unsigned long long nfall = 0, npairs = 0;
     float cmax = 0.0f;
-    tuned::Gather g;
+    tuned::Gather<true> g;
     g.sky = a.sky32;
+    g.wide = (reinterpret_cast<size_t>(a.sky32) & 31) == 0;
     tuned::Queue Q{0, 0};
     for (long long i = pos0 + gw; i < pos1; i += nw) {
         const long long j = a.order ? (long long)a.order[i] : i;  // sample of position i
@@ -178,10 +174,10 @@ void launch_shape(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib,
 }
 
 // kTW: the planned launch's block; without plans the warps build their own
-// (FP64 disc plan in the loop's registers), which spills at 64 registers, so
-// that launch keeps 16 warps per SM.  A planned launch of fewer than four
-// samples per resident warp uses blocks of 8 warps (4 per SM), so that its
-// samples spread over every SM (32-warp blocks would fill n / 32 SMs).
+// (FP64 disc plan in the loop's registers), and that launch keeps 16 warps per
+// SM.  A planned launch of fewer than four samples per resident warp uses
+// blocks of 8 warps (2 per SM), so that its samples spread over every SM
+// (20-warp blocks would fill n / 20 SMs).
 template <bool kBil, int kTW>
 void launch_lookup(const FwdArgs& a, int sm_count, cudaStream_t st, tuned::SamplePlan* plans,
                    long long plan_cap)

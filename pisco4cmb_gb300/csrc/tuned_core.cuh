@@ -95,6 +95,11 @@ template <class A, class = void>
 struct HasOutside : std::false_type {};
 template <class A>
 struct HasOutside<A, std::void_t<decltype(&A::outside)>> : std::true_type {};
+// Does the action take two pixels per lane?
+template <class A, class = void>
+struct HasPair2 : std::false_type {};
+template <class A>
+struct HasPair2<A, std::void_t<decltype(&A::pair2)>> : std::true_type {};
 // Decisions whose FP32 value lies within kMarginRel * (value + 1) of an
 // integer are redone in FP64 (about 20 FP32 ulps).  The observed worst case
 // over a workload is measured by pisco_tuned_calibrate and must stay well
@@ -108,16 +113,26 @@ constexpr float kShortOffset = 0.125f;
 constexpr float kTinyQ = 4.0e-12f;
 
 // One disc ring of the current batch: FP32 offset constants and the pixel
-// range, 64 bytes, read with four 16-byte loads.  The sample's rotation by
-// psi and the beam grid's scale are in the constants, so a pair forms its
-// rotated beam-frame components with two multiply-adds each.
+// range, 48 bytes, read with three 16-byte loads.  A broadcast shared-memory
+// read costs the L1 pipe a cycle per word all the same, and that pipe is the
+// busiest unit of the pair loop, so what a pair can form from the sample's
+// own constants (Frame) is not stored per ring.
 struct alignas(16) RingC {
-    float dc, dphi, Ki, Pp;  // anchor offset, pixel spacing; R^2 (1 - cos(dec - dec0)), R^2 s s0
-    float Xs, Xh, Xc, Wz;    // s sin psi, -s z0 cos psi, -Di cos psi; s0 z
-    float Ys, Yh, Yc, Di;    // s cos psi, s z0 sin psi, Di sin psi; Di = sin(dec - dec0)
-    int j0;                  // ring index of flattened pair t: (j0 + t) mod nr
-    int nr, start;           // ring pixels, first pixel
-    int kc;                  // bits of 1.5 2^23 less the anchor's ring index
+    float dc, dphi;  // anchor offset, pixel spacing
+    float Ki, s;     // R^2 (1 - cos(dec - dec0)); sin of the colatitude
+    float Wz, Di;    // s0 z, sin(dec - dec0)
+    int j0;          // ring index of flattened pair t: (j0 + t) mod nr; with two
+                     // pixels per lane (j0 + 2 t) mod nr, even
+    int kc;          // bits of 1.5 2^23 less the anchor's ring index
+    int nr, start;   // ring pixels, first pixel
+    int ends;        // ring indices of the range's ends, first | last << 16
+    int pad;
+};
+
+// The sample's constants of the pair loop: z0, s0, R^2 s0, sin and cos of psi
+// (times their common factor).
+struct Frame {
+    float z0, s0, R2s0, sps, cps;
 };
 
 // Samples in flight per warp (a sample keeps its slot until its queued
@@ -167,7 +182,6 @@ constexpr int kPlanAllSky = 2;
 struct WarpSmem {
     SamplePlan plan;
     RingC r[32];
-    int incl[32];  // inclusive scan of the batch's pixel counts
     Pend p[kPend];
     int q[kQCap];
     unsigned char qs[kQCap];
@@ -262,6 +276,37 @@ __device__ __forceinline__ F32x2 sub2(F32x2 a, F32x2 b)
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ F32x2 mul2(F32x2 a, F32x2 b)
+{
+    F32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F32x2 fma2(F32x2 a, F32x2 b, F32x2 c)
+{
+    F32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ F32x2 add2_rd(F32x2 a, F32x2 b)  // rounded down
+{
+    F32x2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F32x2 both(float x) { return pack2(x, x); }
+__device__ __forceinline__ float lo2(F32x2 v)
+{
+    float a, b;
+    unpack2(v, a, b);
+    return a;
+}
+__device__ __forceinline__ float hi2(F32x2 v)
+{
+    float a, b;
+    unpack2(v, a, b);
+    return b;
+}
 // two_sum of both halves
 __device__ __forceinline__ void two_sum2(F32x2& s, F32x2& c, F32x2 x)
 {
@@ -328,35 +373,29 @@ __device__ __forceinline__ float rsqrt_approx(float x)
 }
 
 // One beam pixel, both detectors (32 bytes, one sector): a single 256-bit
-// load through the read-only path that does not allocate in L1, so the
-// scattered beam reads (a beam of 10^4 - 10^6 pixels, L2-resident) leave L1
-// to the sky pixels, which neighbouring samples re-read (measured on the
-// c2 forward: 176.2 ms against 177.2 ms allocating in L1).  PISCO_BEAM_LOAD
-// 0: the compiler's own loads (two 128-bit ones); 1: 256-bit, allocating in
-// L1; 3: 256-bit, L2 only (.cg).
-#ifndef PISCO_BEAM_LOAD
-#define PISCO_BEAM_LOAD 2
-#endif
+// load through the read-only path.  kL1: allocating in L1.  A warp's gather
+// of 32 scattered pixels takes the L1 34 cycles when L2 serves it (a sector a
+// cycle; 57 from a table of 64 KB, whose few L2 slices are hot) and 19 when L1
+// hits, so a kernel whose shared memory leaves L1 150 KB or more keeps beam
+// pixels there (20 warps with two pixels per lane: 4.31 ms against 4.93 ms for
+// 100,000 samples of a 1.1 MB beam); one that leaves less gives L1 to the
+// sky, which neighbouring samples re-read (back-projection, 32 warps: 2.36 ms
+// without allocation, 2.47 ms with).
+template <bool kL1 = false>
 __device__ __forceinline__ F8 load_beam(const F8* p)
 {
-#if PISCO_BEAM_LOAD == 0
-    return *p;
-#else
     F8 r;
-#if PISCO_BEAM_LOAD == 2
-#define PISCO_LDB "ld.global.nc.L1::no_allocate.v8.f32"
-#elif PISCO_BEAM_LOAD == 3
-#define PISCO_LDB "ld.global.cg.v8.f32"
-#else
-#define PISCO_LDB "ld.global.nc.v8.f32"
-#endif
-    asm(PISCO_LDB " {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y),
-          "=f"(r.b.z), "=f"(r.b.w)
-        : "l"(p));
-#undef PISCO_LDB
+    if constexpr (kL1)
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y),
+              "=f"(r.b.z), "=f"(r.b.w)
+            : "l"(p));
+    else
+        asm("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y),
+              "=f"(r.b.z), "=f"(r.b.w)
+            : "l"(p));
     return r;
-#endif
 }
 
 // A beam pixel of the bilinear stencil: its four pixels are two pairs of
@@ -785,6 +824,189 @@ __device__ __forceinline__ float quarter_turns(float X, float Y, unsigned sgn)
     return __saturatef(fmaf(t, p, 0.5f));
 }
 
+// A pair's place in the beam's frame: sin D and 1 - cos D of its longitude
+// offset, R^2 (1 - cos rho), the rotated components (X, Y), the beam grid's
+// polar-cap coordinates (quadrant qd, fraction tp, r = R sqrt(1 - cos rho)).
+struct Spot {
+    float sn, h, q, X, Y, tp, r;
+    int qd;
+};
+
+// The pair kf pixels from its ring's anchor, R0 = (dc, dphi, Ki, s) and Di its
+// ring's.  East u = s sin D, north v = Di + z0 s (1 - cos D), turned by psi.
+__device__ __forceinline__ Spot locate(float kf, const Frame& F, const float4& R0, float Di,
+                                       bool narrow)
+{
+    Spot p;
+    const float dl = fmaf(kf, R0.y, R0.x);
+    if (narrow) short_sin_versin(dl, p.sn, p.h);
+    else sin_versin(dl, p.sn, p.h);
+    const float sh = R0.w * p.h, u = R0.w * p.sn;
+    const float v = fmaf(F.z0, sh, Di);
+    p.q = fmaf(F.R2s0, sh, R0.z);
+    p.X = fmaf(u, F.sps, -v * F.cps);
+    p.Y = fmaf(u, F.cps, v * F.sps);
+    const unsigned sgn = (__float_as_uint(p.X) ^ __float_as_uint(p.Y)) & 0x80000000u;
+    p.qd = (int)(2u * (__float_as_uint(p.Y) >> 31) + (sgn >> 31));
+    p.tp = quarter_turns(p.X, p.Y, sgn);
+    p.r = p.q * rsqrt_approx(p.q);
+    return p;
+}
+
+// exp(2i chi) = w^2 / |w|^2, w = (db + i nb)(X - i Y): the direction to the
+// boresight (nb = s0 sin D, db = Wz h - Di) times the rotated beam-frame
+// direction (an overall sign drops out).
+__device__ __forceinline__ void phasor(const Spot& p, float s0, float Wz, float Di, float& c2,
+                                       float& s2)
+{
+    const float nb = s0 * p.sn;
+    const float db = fmaf(Wz, p.h, -Di);
+    const float wr = fmaf(db, p.X, nb * p.Y);
+    const float wi = fmaf(nb, p.X, -(db * p.Y));
+    const float ww = wr * wr;
+    const float iw = rcp_approx(fmaf(wi, wi, ww));
+    c2 = fmaf(-wi, wi, ww) * iw;
+    s2 = wr * wi * (iw + iw);
+}
+
+// The nearest beam pixel, ang2pix of the polar cap: jp = floor(tp r), jm =
+// floor((1 - tp) r), ring ir = jp + jm + 1, position floor(tp ir) in the
+// quadrant.  near: one of the three lies within its margin of an integer, and
+// the pair goes to FP64.
+struct CapPixel {
+    float av, bv, cv;
+    int ir, bp;
+    bool near;
+};
+__device__ __forceinline__ CapPixel cap_pixel(const Spot& p)
+{
+    CapPixel c;
+    c.av = p.tp * p.r;
+    c.bv = fmaf(-p.tp, p.r, p.r);
+    float ha, fa, hb, fb, hc, fc;
+    const int ja = split_half(c.av, ha, fa), jb = split_half(c.bv, hb, fb);
+    const float irf = ha + hb;
+    c.cv = p.tp * irf;
+    const int jc = split_half(c.cv, hc, fc);
+    // 1/2 less kMarginRel (r + 2), and r + 1 >= ir
+    const float edge = fmaf(-kMarginRel, p.r, 0.5f - 2.0f * kMarginRel);
+    c.near = fmaxf(fmaxf(fabsf(fa), fabsf(fb)), fabsf(fc)) > edge;
+    c.ir = (ja - kTwo23Bits) + (jb - kTwo23Bits) + 1;
+    // 2 ir (ir - 1) + qd ir + position
+    c.bp = c.ir * (2 * c.ir - 2 + p.qd) + (jc - kTwo23Bits);
+    return c;
+}
+
+// Two pairs of one ring, side by side: locate, cap_pixel and phasor with
+// every operation that has no ring constant packed.
+struct Spot2 {
+    float sn0, sn1, h0, h1, q0, q1;
+    F32x2 X, Y, tp, r;
+    int qd0, qd1;
+};
+__device__ __forceinline__ unsigned sign_of(float x, float y)
+{
+    return (__float_as_uint(x) ^ __float_as_uint(y)) & 0x80000000u;
+}
+__device__ __forceinline__ Spot2 locate2(float kf, const Frame& F, const float4& R0, float Di,
+                                         bool narrow)
+{
+    Spot2 p;
+    const float d0 = fmaf(kf, R0.y, R0.x), d1 = fmaf(kf + 1.0f, R0.y, R0.x);
+    if (narrow) {
+        const F32x2 x = pack2(d0, d1), x2 = mul2(x, x);
+        const F32x2 sn = mul2(x, fma2(x2, fma2(x2, both(8.33333333e-3f), both(-1.66666667e-1f)),
+                                      both(1.0f)));
+        const F32x2 h = mul2(x2, fma2(x2, fma2(x2, both(1.38888889e-3f), both(-4.16666667e-2f)),
+                                      both(0.5f)));
+        unpack2(sn, p.sn0, p.sn1);
+        unpack2(h, p.h0, p.h1);
+    } else {
+        sin_versin(d0, p.sn0, p.h0);
+        sin_versin(d1, p.sn1, p.h1);
+    }
+    const float g0 = R0.w * p.h0, g1 = R0.w * p.h1;
+    const float u0 = R0.w * p.sn0, u1 = R0.w * p.sn1;
+    const float w0 = fmaf(F.z0, g0, Di), w1 = fmaf(F.z0, g1, Di);
+    p.q0 = fmaf(F.R2s0, g0, R0.z);
+    p.q1 = fmaf(F.R2s0, g1, R0.z);
+    const float X0 = fmaf(u0, F.sps, -w0 * F.cps), X1 = fmaf(u1, F.sps, -w1 * F.cps);
+    const float Y0 = fmaf(u0, F.cps, w0 * F.sps), Y1 = fmaf(u1, F.cps, w1 * F.sps);
+    p.X = pack2(X0, X1);
+    p.Y = pack2(Y0, Y1);
+    const unsigned m0 = sign_of(X0, Y0), m1 = sign_of(X1, Y1);
+    p.qd0 = (int)(2u * (__float_as_uint(Y0) >> 31) + (m0 >> 31));
+    p.qd1 = (int)(2u * (__float_as_uint(Y1) >> 31) + (m1 >> 31));
+    // quarter_turns
+    const F32x2 d = pack2(__uint_as_float(__float_as_uint(fabsf(Y0) - fabsf(X0)) ^ m0),
+                          __uint_as_float(__float_as_uint(fabsf(Y1) - fabsf(X1)) ^ m1));
+    const F32x2 t = mul2(d, pack2(rcp_approx(fabsf(X0) + fabsf(Y0)),
+                                  rcp_approx(fabsf(X1) + fabsf(Y1))));
+    const F32x2 t2 = mul2(t, t);
+    constexpr double q = 0.63661977236758134;
+    F32x2 a = both((float)(q * 0.0028662257));
+    a = fma2(a, t2, both((float)(q * -0.0161657367)));
+    a = fma2(a, t2, both((float)(q * 0.0429096138)));
+    a = fma2(a, t2, both((float)(q * -0.0752896400)));
+    a = fma2(a, t2, both((float)(q * 0.1065626393)));
+    a = fma2(a, t2, both((float)(q * -0.1420889944)));
+    a = fma2(a, t2, both((float)(q * 0.1999355085)));
+    a = fma2(a, t2, both((float)(q * -0.3333314528)));
+    a = fma2(a, t2, both((float)q));
+    p.tp = pack2(__saturatef(fmaf(lo2(t), lo2(a), 0.5f)), __saturatef(fmaf(hi2(t), hi2(a), 0.5f)));
+    p.r = mul2(pack2(p.q0, p.q1), pack2(rsqrt_approx(p.q0), rsqrt_approx(p.q1)));
+    return p;
+}
+__device__ __forceinline__ void cap_pixel2(const Spot2& p, int& bp0, int& bp1, bool& near0,
+                                           bool& near1)
+{
+    const F32x2 k23 = both(kTwo23), khalf = both(8388607.5f);
+    const F32x2 av = mul2(p.tp, p.r), bv = sub2(p.r, av);
+    const F32x2 ta = add2_rd(av, k23), tb = add2_rd(bv, k23);
+    const F32x2 ha = sub2(ta, khalf), hb = sub2(tb, khalf);
+    const F32x2 fa = sub2(av, ha), fb = sub2(bv, hb);
+    const F32x2 cv = mul2(p.tp, add2(ha, hb));
+    const F32x2 tc = add2_rd(cv, k23);
+    const F32x2 fc = sub2(cv, sub2(tc, khalf));
+    const F32x2 edge = fma2(p.r, both(-kMarginRel), both(0.5f - 2.0f * kMarginRel));
+    near0 = fmaxf(fmaxf(fabsf(lo2(fa)), fabsf(lo2(fb))), fabsf(lo2(fc))) > lo2(edge);
+    near1 = fmaxf(fmaxf(fabsf(hi2(fa)), fabsf(hi2(fb))), fabsf(hi2(fc))) > hi2(edge);
+    const int i0 = (__float_as_int(lo2(ta)) - kTwo23Bits) + (__float_as_int(lo2(tb)) - kTwo23Bits) + 1;
+    const int i1 = (__float_as_int(hi2(ta)) - kTwo23Bits) + (__float_as_int(hi2(tb)) - kTwo23Bits) + 1;
+    bp0 = i0 * (2 * i0 - 2 + p.qd0) + (__float_as_int(lo2(tc)) - kTwo23Bits);
+    bp1 = i1 * (2 * i1 - 2 + p.qd1) + (__float_as_int(hi2(tc)) - kTwo23Bits);
+}
+// (the signs of wr and of its factors are turned around: no packed negation)
+__device__ __forceinline__ void phasor2(const Spot2& p, float s0, float Wz, float Di, F32x2& c2,
+                                        F32x2& s2)
+{
+    const F32x2 nb = pack2(s0 * p.sn0, s0 * p.sn1), mb = pack2(-s0 * p.sn0, -s0 * p.sn1);
+    const F32x2 db = pack2(fmaf(-Wz, p.h0, Di), fmaf(-Wz, p.h1, Di));
+    const F32x2 wr = fma2(db, p.X, mul2(mb, p.Y));
+    const F32x2 wi = fma2(nb, p.X, mul2(db, p.Y));
+    const F32x2 rr = mul2(wr, wr), ii = mul2(wi, wi);
+    const F32x2 n = add2(rr, ii);
+    const F32x2 iw = pack2(rcp_approx(lo2(n)), rcp_approx(hi2(n)));
+    c2 = mul2(sub2(rr, ii), iw);
+    s2 = mul2(mul2(wr, wi), mul2(iw, both(-2.0f)));
+}
+
+// Two pairs: the values loaded for them and their phasors.
+struct Unit {
+    F8 B0, B1;
+    float4 S0, S1;
+    F32x2 c, s;  // cos 2chi, sin 2chi
+    bool in0, in1;
+};
+
+// 1 << x, 0 for x outside [0, 32).
+__device__ __forceinline__ unsigned bit_or_0(int x)
+{
+    unsigned r;
+    asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(x));
+    return r;
+}
+
 // (sin psi, cos psi) times a common factor near 1, in FP32, with the angle
 // kept to about 2e-9: the rotation by psi multiplies every pair of a sample,
 // so the rounding error of its angle is coherent over the sample's sum (an
@@ -886,7 +1108,9 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                                                unsigned long long& npairs)
 {
     RingC* W = S.r;
-    const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned lt_mask = (1u << lane) - 1u, le_mask = 2u * lt_mask + 1u;
+    // two pixels per lane (actions with pair2, nearest lookup)
+    constexpr bool kUnits = HasPair2<Action>::value && !kBil && !kCalib;
     if (SP.flags & kPlanBad) {
         if (Action::kSums && lane == 0) {
             store_out(o.a, o.f64, o.idx, CUDART_NAN);
@@ -923,12 +1147,33 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
     if constexpr (Action::kSums) act.reset();
     const SamplePlan& PL = S.plan;
     // what the pair loop reads on every pair, in registers
-    const float s0 = PL.s0f;
-    const float tiny = kTinyQ * (B.rscale * B.rscale);
+    const float R2 = B.rscale * B.rscale;
+    const Frame F{PL.z0f, PL.s0f, R2 * PL.s0f, PL.sps, PL.cps};
+    const float tiny = kTinyQ * R2;
+    const F8* const beam = B.beam;
+    const unsigned npix_beam = (unsigned)B.npix;
+
+    // queues a near-edge pair per lane; redoes them 32 at a time in FP64
+    auto queue = [&](bool fb, int pix) {
+        const unsigned mk = __ballot_sync(kFull, fb);
+        if (!mk) return;
+        if (fb) {
+            const int at = Qs.n + __popc(mk & lt_mask);
+            S.q[at] = pix;
+            S.qs[at] = (unsigned char)slot;
+        }
+        Qs.n += __popc(mk);
+        if (lane == 0) {
+            nfall += __popc(mk);
+            S.p[slot].left += __popc(mk);
+        }
+        __syncwarp();
+        if (Qs.n >= 32) drain<kBil>(hs, 32, S, Qs, lane, err, act);
+    };
 
     for (int r0 = PL.full_lo; r0 <= PL.full_hi; r0 += 32) {
         const int ring = r0 + lane;
-        int cnt = 0;
+        int cnt = 0, items = 0;  // the ring's disc pixels; its lane slots
         bool wide = false;
         RingC rc;
         if (ring <= PL.full_hi) {
@@ -957,18 +1202,10 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 float sD, hD;
                 sin_versin(df, sD, hD);
                 const float Di = fmaf(de, 1.0f - hD, sD);
-                const float Zs = rt.s * PL.z0f;
-                const float R2 = B.rscale * B.rscale;
                 rc.Ki = R2 * fmaf(de, sD, hD);
-                rc.Pp = R2 * (rt.s * PL.s0f);
-                rc.Wz = PL.s0f * rt.zf;
+                rc.s = rt.s;
+                rc.Wz = F.s0 * rt.zf;
                 rc.Di = Di;
-                rc.Xs = rt.s * PL.sps;
-                rc.Xh = -Zs * PL.cps;
-                rc.Xc = -Di * PL.cps;
-                rc.Ys = rt.s * PL.cps;
-                rc.Yh = Zs * PL.sps;
-                rc.Yc = Di * PL.sps;
                 rc.nr = nr;
                 rc.start = rt.start;
                 // offsets from the anchor, the range centred on it; a whole
@@ -983,142 +1220,138 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 if (mid >= (nr >> 1) + 1) kk -= nr;
                 else if (mid < -(nr >> 1)) kk += nr;
                 rc.kc = 0x4B400000 + kk - sp.lo;
-                rc.j0 = sp.lo;
+                const int hi = sp.lo + cnt - 1;  // below 2^16: rings hold at most 2^15 pixels
+                rc.ends = sp.lo | hi << 16;
+                // two pixels per lane: ring indices 2m and 2m + 1, which are
+                // neighbours in memory as well (a ring's pixels and its first
+                // pixel are multiples of 4)
+                rc.j0 = kUnits ? sp.lo & ~1 : sp.lo;
+                items = kUnits ? (hi >> 1) - (sp.lo >> 1) + 1 : cnt;
                 const int far = max(-kk, kk + cnt);
                 wide = (float)far * rt.dphif > kShortOffset - rt.dphif;
             }
         }
-        int incl = cnt;
+        int incl = items;
+        int all = cnt;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(kFull, incl, o);
             if (lane >= o) incl += v;
         }
         const int total = __shfl_sync(kFull, incl, 31);
-        rc.j0 -= incl - cnt;
-        W[lane] = rc;
-        S.incl[lane] = incl;
+        if (kCalib) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(kFull, all, o);
+            if (lane == 0) npairs += (unsigned long long)all;
+        }
+        // the rings with pixels, packed in order: a lane's ring is then the
+        // number of ring starts up to its slot, counted with one warp
+        // reduction per iteration instead of a search through shared memory
+        const unsigned some = __ballot_sync(kFull, items > 0);
+        const int rings_here = __popc(some);
+        int first = items > 0 ? incl - items : 0x7fffffff;  // first slot less this iteration's
+        if (items > 0) {
+            rc.j0 -= (kUnits ? 2 : 1) * first;
+            W[__popc(some & lt_mask)] = rc;
+        }
         const bool narrow = !__any_sync(kFull, wide);
         __syncwarp();
-        if (lane == 0) npairs += (unsigned long long)total;
-        int k = 0;  // lane slot (ring) owning the current pair; only moves forward
+        int k0 = -1;  // ring of the slot before this iteration's
         const int iters = (total + 31) >> 5;
-        for (int it = 0; it < iters; ++it) {
+        for (int it = 0; it < iters; ++it, first -= 32) {
+            const unsigned starts = __reduce_or_sync(kFull, bit_or_0(first));
+            const int k = k0 + __popc(starts & le_mask);
+            k0 += __popc(starts);
             const int t = (it << 5) + lane;
+            if constexpr (kUnits) {
+                // the slots past the end repeat the last one, switched off
+                const int tt = min(t, total - 1);
+                const RingC& R = W[min(k, rings_here - 1)];
+                const float4 R0 = *reinterpret_cast<const float4*>(&R.dc);
+                const float4 R1 = *reinterpret_cast<const float4*>(&R.Wz);
+                const int4 R3 = *reinterpret_cast<const int4*>(&R.nr);
+                const int j = __float_as_int(R1.z) + 2 * tt;  // even, below 2 nr
+                const int pix = R3.y + (int)min((unsigned)j, (unsigned)(j - R3.x));
+                const float kf = __int_as_float(__float_as_int(R1.w) + j) - 12582912.0f;
+                const bool v0 = t < total && j >= (R3.z & 0xffff);
+                const bool v1 = t < total && j < (int)((unsigned)R3.z >> 16);
+                const Spot2 p = locate2(kf, F, R0, R1.y, narrow);
+                int bp0, bp1;
+                bool near0, near1;
+                cap_pixel2(p, bp0, bp1, near0, near1);
+                const bool fb0 = v0 && (near0 || p.q0 < tiny);
+                const bool fb1 = v1 && (near1 || p.q1 < tiny);
+                const bool in0 = v0 && !fb0 && (unsigned)bp0 < npix_beam;
+                const bool in1 = v1 && !fb1 && (unsigned)bp1 < npix_beam;
+                Unit U;
+                U.in0 = in0;
+                U.in1 = in1;
+                U.B0 = load_beam<Action::kL1>(beam + (in0 ? bp0 : 0));
+                U.B1 = load_beam<Action::kL1>(beam + (in1 ? bp1 : 0));
+                act.fetch2(pix, U.S0, U.S1);
+                phasor2(p, F.s0, R1.x, R1.y, U.c, U.s);
+                act.pair2(U);
+                if (__any_sync(kFull, fb0 || fb1)) {
+#pragma unroll 1
+                    for (int e = 0; e < 2; ++e) queue(e ? fb1 : fb0, pix + e);
+                }
+            } else {
             bool fb = false;
             int pix = 0;
             if (t < total) {
-                while (S.incl[k] <= t) ++k;
-                const int4 R3 = *reinterpret_cast<const int4*>(&W[k].j0);
-                const int j = R3.x + t;  // ring index, below 2 nr
-                pix = R3.z + (int)min((unsigned)j, (unsigned)(j - R3.y));
-                const float kf = __int_as_float(R3.w + j) - 12582912.0f;  // offset from the anchor
-                {
-                    const float4 R0 = *reinterpret_cast<const float4*>(&W[k].dc);
-                    const float4 R1 = *reinterpret_cast<const float4*>(&W[k].Xs);
-                    const float4 R2 = *reinterpret_cast<const float4*>(&W[k].Ys);
-                    const float dl = fmaf(kf, R0.y, R0.x);
-                    float sn, h;
-                    if (narrow) short_sin_versin(dl, sn, h);
-                    else sin_versin(dl, sn, h);
-                    const float q = fmaf(R0.w, h, R0.z);  // R^2 (1 - cos rho)
-                    const float X = fmaf(sn, R1.x, fmaf(h, R1.y, R1.z));
-                    const float Y = fmaf(sn, R2.x, fmaf(h, R2.y, R2.z));
-                    const unsigned sgn =
-                        (__float_as_uint(X) ^ __float_as_uint(Y)) & 0x80000000u;
-                    const int qd = (int)(2u * (__float_as_uint(Y) >> 31) + (sgn >> 31));
-                    const float tp = quarter_turns(X, Y, sgn);
-                    const float r = q * rsqrt_approx(q);
-                    // exp(2i chi) = w^2 / |w|^2, w = (db + i nb)(X - i Y): the
-                    // direction to the boresight times the rotated beam-frame
-                    // direction (an overall sign drops out)
-                    auto phasor = [&](float& c2, float& s2) {
-                        const float nb = s0 * sn;
-                        const float db = fmaf(R1.w, h, -R2.w);
-                        const float wr = fmaf(db, X, nb * Y);
-                        const float wi = fmaf(nb, X, -(db * Y));
-                        const float ww = wr * wr;
-                        const float iw = rcp_approx(fmaf(wi, wi, ww));
-                        c2 = fmaf(-wi, wi, ww) * iw;
-                        s2 = wr * wi * (iw + iw);
-                    };
-                    if constexpr (kBil && Action::kStencil) {
-                        fb = q < tiny;
-                        int px[4];
-                        float w[4];
-                        if (!fb && stencil_f32(B, qd, tp, r, px, w)) {
+                const float4 R0 = *reinterpret_cast<const float4*>(&W[k].dc);
+                const float4 R1 = *reinterpret_cast<const float4*>(&W[k].Wz);
+                const int2 R3 = *reinterpret_cast<const int2*>(&W[k].nr);
+                const int j = __float_as_int(R1.z) + t;  // ring index, below 2 nr
+                pix = R3.y + (int)min((unsigned)j, (unsigned)(j - R3.x));
+                const float kf = __int_as_float(__float_as_int(R1.w) + j) - 12582912.0f;
+                const Spot p = locate(kf, F, R0, R1.y, narrow);
+                fb = p.q < tiny;
+                if constexpr (kBil && Action::kStencil) {
+                    int px[4];
+                    float w[4];
+                    if (!fb && stencil_f32(B, p.qd, p.tp, p.r, px, w)) {
+                        float c2, s2;
+                        phasor(p, F.s0, R1.x, R1.y, c2, s2);
+                        act.pair_stencil(pix, act.fetch(pix), px, w, c2, s2);
+                    } else if constexpr (HasOutside<Action>::value) {
+                        if (!fb) act.outside(pix, -1);
+                    }
+                } else if constexpr (kBil) {
+                    F8 Bv;
+                    if (!fb && bilinear_f32(B, p.qd, p.tp, p.r, Bv)) {
+                        float c2, s2;
+                        phasor(p, F.s0, R1.x, R1.y, c2, s2);
+                        act.pair(pix, act.fetch(pix), Bv, -1, c2, s2);
+                    } else if constexpr (HasOutside<Action>::value) {
+                        if (!fb) act.outside(pix, -1);
+                    }
+                } else {
+                    const CapPixel c = cap_pixel(p);
+                    fb |= c.near;
+                    if (kCalib && !fb) {
+                        double rho, sig, chi;
+                        (void)pair_beam_pixel(hs, hb, pix, ra, dec, -pa, &rho, &sig, &chi);
+                        const double tt = fmodulo(sig * kInvHalfPi, 4.0);
+                        const double tpd = tt - floor(tt);
+                        const double rd = (double)B.nside * sqrt(3.0 * (1.0 - cos(rho)));
+                        const double e1 = fabs(c.av - tpd * rd) / (p.r + 1.0);
+                        const double e2 = fabs(c.bv - (1.0 - tpd) * rd) / (p.r + 1.0);
+                        const double e3 = fabs(c.cv - tpd * (double)c.ir) / ((double)c.ir + 1.0);
+                        cmax = fmaxf(cmax, (float)fmax(fmax(e1, e2), e3) / kMarginRel);
+                    }
+                    if (!fb) {
+                        if ((unsigned)c.bp < (unsigned)B.npix) {  // 0 <= bp < npix
                             float c2, s2;
-                            phasor(c2, s2);
-                            act.pair_stencil(pix, act.fetch(pix), px, w, c2, s2);
+                            phasor(p, F.s0, R1.x, R1.y, c2, s2);
+                            act.pair(pix, act.fetch(pix), load_beam(B.beam + c.bp), c.bp, c2, s2);
                         } else if constexpr (HasOutside<Action>::value) {
-                            if (!fb) act.outside(pix, -1);
-                        }
-                    } else if constexpr (kBil) {
-                        fb = q < tiny;
-                        F8 Bv;
-                        if (!fb && bilinear_f32(B, qd, tp, r, Bv)) {
-                            float c2, s2;
-                            phasor(c2, s2);
-                            act.pair(pix, act.fetch(pix), Bv, -1, c2, s2);
-                        } else if constexpr (HasOutside<Action>::value) {
-                            if (!fb) act.outside(pix, -1);
-                        }
-                    } else {
-                        // ang2pix of the polar cap: jp = floor(tp r), jm =
-                        // floor((1 - tp) r), ring ir = jp + jm + 1, position
-                        // floor(tp ir) in the quadrant; a value within the
-                        // margin of an integer sends the pair to FP64
-                        const float av = tp * r;
-                        const float bv = fmaf(-tp, r, r);
-                        float ha, fa, hv, fv, hc, fc;
-                        const int ja = split_half(av, ha, fa), jb = split_half(bv, hv, fv);
-                        const float irf = ha + hv;
-                        const float cv = tp * irf;
-                        const int jc = split_half(cv, hc, fc);
-                        // 1/2 less kMarginRel (r + 2), and r + 1 >= ir
-                        const float edge = fmaf(-kMarginRel, r, 0.5f - 2.0f * kMarginRel);
-                        fb = q < tiny || fmaxf(fmaxf(fabsf(fa), fabsf(fv)), fabsf(fc)) > edge;
-                        const int ir = (ja - kTwo23Bits) + (jb - kTwo23Bits) + 1;
-                        if (kCalib && !fb) {
-                            double rho, sig, chi;
-                            (void)pair_beam_pixel(hs, hb, pix, ra, dec, -pa, &rho, &sig, &chi);
-                            const double tt = fmodulo(sig * kInvHalfPi, 4.0);
-                            const double tpd = tt - floor(tt);
-                            const double rd = (double)B.nside * sqrt(3.0 * (1.0 - cos(rho)));
-                            const double e1 = fabs(av - tpd * rd) / (r + 1.0);
-                            const double e2 = fabs(bv - (1.0 - tpd) * rd) / (r + 1.0);
-                            const double e3 = fabs(cv - tpd * (double)ir) / ((double)ir + 1.0);
-                            cmax = fmaxf(cmax, (float)fmax(fmax(e1, e2), e3) / kMarginRel);
-                        }
-                        if (!fb) {
-                            // 2 ir (ir - 1) + qd ir + position
-                            const int bp = ir * (2 * ir - 2 + qd) + (jc - kTwo23Bits);
-                            if ((unsigned)bp < (unsigned)B.npix) {  // 0 <= bp < npix
-                                float c2, s2;
-                                phasor(c2, s2);
-                                act.pair(pix, act.fetch(pix), load_beam(B.beam + bp), bp, c2, s2);
-                            } else if constexpr (HasOutside<Action>::value) {
-                                act.outside(pix, bp);
-                            }
+                            act.outside(pix, c.bp);
                         }
                     }
                 }
             }
-            // queue near-edge pairs; redo them 32 at a time in FP64
-            const unsigned mk = __ballot_sync(kFull, fb);
-            if (mk) {
-                if (fb) {
-                    const int at = Qs.n + __popc(mk & lt_mask);
-                    S.q[at] = pix;
-                    S.qs[at] = (unsigned char)slot;
-                }
-                Qs.n += __popc(mk);
-                if (lane == 0) {
-                    nfall += __popc(mk);
-                    S.p[slot].left += __popc(mk);
-                }
-                __syncwarp();
-                if (Qs.n >= 32) drain<kBil>(hs, 32, S, Qs, lane, err, act);
+            queue(fb, pix);
             }
         }
         __syncwarp();
@@ -1153,10 +1386,13 @@ __device__ __forceinline__ void sample(const Hpx& hs, const RingT* rings, const 
 
 // Forward action: gather the sky, multiply by the beam, compensated sums of
 // both detectors side by side (two_sum2).
+template <bool kBeamL1>
 struct Gather {
+    static constexpr bool kL1 = kBeamL1;  // load_beam
     static constexpr bool kSums = true;
     static constexpr bool kStencil = false;
     const float4* sky;
+    bool wide;       // sky is 32-byte aligned
     F32x2 sum, cmp;  // halves: detector a, detector b
     __device__ __forceinline__ void reset() { sum = cmp = pack2(0.0f, 0.0f); }
     __device__ __forceinline__ float4 fetch(int pix) const { return __ldg(&sky[pix]); }
@@ -1173,6 +1409,32 @@ struct Gather {
         float ta, tb;
         contrib(S, B, c2, s2, ta, tb);
         two_sum2(sum, cmp, pack2(ta, tb));
+    }
+    // sky pixels pix (even) and pix + 1: one 256-bit load when the map is
+    // 32-byte aligned (a caller's own map need only be 16-byte aligned)
+    __device__ __forceinline__ void fetch2(int pix, float4& S0, float4& S1) const
+    {
+        const float4* p = sky + pix;
+        if (wide) {
+            asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                : "=f"(S0.x), "=f"(S0.y), "=f"(S0.z), "=f"(S0.w), "=f"(S1.x), "=f"(S1.y),
+                  "=f"(S1.z), "=f"(S1.w)
+                : "l"(p));
+        } else {
+            S0 = __ldg(p);
+            S1 = __ldg(p + 1);
+        }
+    }
+    // two pairs; one that is off adds nothing
+    __device__ __forceinline__ void pair2(const Unit& U)
+    {
+        float a0, b0, a1, b1;
+        contrib(U.S0, U.B0, lo2(U.c), lo2(U.s), a0, b0);
+        contrib(U.S1, U.B1, hi2(U.c), hi2(U.s), a1, b1);
+        if (!U.in0) a0 = b0 = 0.0f;
+        if (!U.in1) a1 = b1 = 0.0f;
+        two_sum2(sum, cmp, pack2(a0, b0));
+        two_sum2(sum, cmp, pack2(a1, b1));
     }
     __device__ __forceinline__ void stash(Pend&) const {}
     __device__ __forceinline__ void deferred(const Pend&, int pix, const F8& B, int, float c2, float s2,
