@@ -129,14 +129,14 @@ __global__ void ring_table_kernel(int nside, RingT* rings)
         const double z = ring2z(h, r);
         const double s = sqrt(PD_MUL(PD_SUB(1.0, z), PD_ADD(1.0, z)));
         RingT t;
-        t.z = z;
-        t.omz2 = PD_SUB(1.0, PD_MUL(z, z));
-        t.dec = atan2(z, s);
-        t.fr = PD_MUL((double)ri.npix, kInvTwoPi);
-        t.dphi = PD_DIV(kTwoPi, (double)ri.npix);
+        const double dec = atan2(z, s), fr = PD_MUL((double)ri.npix, kInvTwoPi);
+        t.dec_hi = (float)dec;
+        t.dec_lo = (float)(dec - (double)t.dec_hi);
+        t.fr_hi = (float)fr;
+        t.fr_lo = (float)(fr - (double)t.fr_hi);
         t.s = (float)s;
-        t.dphif = (float)t.dphi;
-        t.zf = (float)z;
+        t.dphi = (float)PD_DIV(kTwoPi, (double)ri.npix);
+        t.z = (float)z;
         t.start = (int)ri.start;
         t.npix2 = (int)(2 * ri.npix + (ri.shifted ? 1 : 0));
         rings[r - 1] = t;

@@ -30,21 +30,20 @@ struct alignas(64) D8 {
 };
 
 // Per-ring geometry of the sky grid, built once per nside on the device
-// (ring_table_kernel, fwd_tuned.cu) from hpx.cuh's ring_info and ring2z, so
-// every value is the one the HEALPix formulas give: rings 1 .. 4 nside - 1
-// at index ring - 1.  64 bytes, four 16-byte loads.  At most 32,767 rings
-// (nside 8192): 2.1 MB.
+// (ring_table_kernel, fwd_tuned.cu) from hpx.cuh's ring_info and ring2z, for
+// rings 1 .. 4 nside - 1 at index ring - 1.  What the ring set-up needs beyond
+// FP32 is kept as the sum of two FP32 values (hi + lo, to about 2^-49), so the
+// set-up runs in FP32.  48 bytes, three 16-byte loads.  At most 32,767 rings
+// (nside 8192): 1.6 MB.
 struct alignas(16) RingT {
-    double z;      // ring2z
-    double omz2;   // 1 - z*z, rounded as the disc-edge formula rounds it
-    double dec;    // latitude atan2(z, sqrt((1 - z)(1 + z)))
-    double fr;     // npix / (2 pi), rounded as the disc-edge formula rounds it
-    double dphi;   // 2 pi / npix
-    float s;       // sqrt(1 - z^2)
-    float dphif;   // 2 pi / npix
-    float zf;      // z
-    int start;     // first pixel
-    int npix2;     // 2 npix + (1 if the ring is shifted by half a pixel)
+    float dec_hi, dec_lo;  // latitude atan2(z, sqrt((1 - z)(1 + z)))
+    float fr_hi, fr_lo;    // npix / (2 pi)
+    float s;               // sqrt(1 - z^2)
+    float dphi;            // 2 pi / npix
+    float z;
+    int start;             // first pixel
+    int npix2;             // 2 npix + (1 if the ring is shifted by half a pixel)
+    int pad[3];
 };
 constexpr int kMaxRings = 4 * 8192 - 1;
 

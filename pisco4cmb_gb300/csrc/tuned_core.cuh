@@ -163,18 +163,22 @@ struct alignas(16) Pend {
 // it is FP64 work (about three hundred FP64 instructions), which GB300 runs
 // at a small fraction of its FP32 rate.  96 bytes.
 struct alignas(16) SamplePlan {
-    double z0, xa, phi;       // disc: cos(theta), 1 / sin(theta), longitude (disc_plan)
-    double phi_f, dec0;       // frame: longitude reduced mod 2 pi, latitude
-    double cosr;              // disc: cos(radius) (the beam's, as evaluated on the device)
+    // disc, for disc_ring's exact formula: cos(theta), 1 / sin(theta),
+    // cos(radius) (the beam's, as evaluated on the device), longitude
+    double z0, xa, cosr, phi;
+    float phi_hi, phi_lo;     // frame: longitude reduced mod 2 pi, latitude,
+    float dec_hi, dec_lo;     //   each the sum of two FP32 values
+    float versr;              // disc: 1 - cos(radius)
     float z0f, s0f;           // frame: sin and |cos| of the latitude
     float sps, cps;           // sin and cos of psi times a common factor (psi_phasor),
                               // negated with the frame's flip
     int ring_lo, ring_hi;     // rings on the edge formula
     int full_lo, full_hi;     // rings touched
-    int flags;                // kPlanBad: non-finite pointing; kPlanAllSky
+    int flags;                // kPlanBad: non-finite pointing; kPlanAllSky; kPlanExact
 };
 constexpr int kPlanBad = 1;
 constexpr int kPlanAllSky = 2;
+constexpr int kPlanExact = 4;  // the frame is not the disc's (an ulp from a pole): exact edges
 
 // Per-warp shared state: one ring batch, the samples in flight, the FP64
 // re-evaluation queue (sky pixel, slot) and the current sample's plan (read
@@ -221,6 +225,7 @@ struct Beam {
     int npix;
     double rho_max;
     double cosr;   // cos(rho_max), evaluated on the device
+    float versr;   // 1 - cos(rho_max)
     float rscale;  // sqrt(3) * nside
 };
 
@@ -232,6 +237,8 @@ __device__ __forceinline__ Beam make_beam(const F8* beam, int nside, int npix, d
     b.npix = npix;
     b.rho_max = rho_max;
     b.cosr = rho_max >= kPi ? 0.0 : cos(rho_max);
+    const double half = sin(0.5 * rho_max);
+    b.versr = (float)(2.0 * half * half);
     b.rscale = (float)(1.7320508075688772 * (double)nside);
     return b;
 }
@@ -424,17 +431,76 @@ __device__ __forceinline__ F8 load_beam_stencil(const F8* p)
 #endif
 }
 
+// sin(x) and 1 - cos(x): Taylor series for |x| <= 0.5 (truncation below
+// 3e-11 relative), CUDA sincosf beyond.
+__device__ __forceinline__ void sin_versin(float x, float& sn, float& h)
+{
+    if (fabsf(x) <= 0.5f) {
+        const float x2 = x * x;
+        sn = x * fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, 2.75573192e-6f, -1.98412698e-4f),
+                                        8.33333333e-3f), -1.66666667e-1f), 1.0f);
+        h = x2 * fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, 2.75573192e-7f, -2.48015873e-5f),
+                                        1.38888889e-3f), -4.16666667e-2f), 0.5f);
+    } else {
+        float cs;
+        sincosf(x, &sn, &cs);
+        h = (cs > 0.0f) ? (sn * sn) / (1.0f + cs) : 1.0f - cs;
+    }
+}
+
 // The disc's pixels on one ring, as ring indices lo .. lo + n - 1 (0 <= lo <
 // npix, wrapping at npix).
 struct RingRange {
     int lo, n;
 };
 
-// FP32 edge angle, FP64 positions, exact FP64 HEALPix formula (disc_ring)
-// whenever an edge decision is within the FP32 angle's error of a pixel
-// boundary.  Same pixels as disc_ring.
-__device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePlan& p, double cosr,
-                                                    int ring, const RingT& rt)
+// A ring's place under the sample: its latitude offset (sin Di and 1 - cos
+// K), and the boresight's longitude in ring pixels, phi npix / 2 pi = at + f +
+// e (at an integer, |f| <= 1/2, e what the FP32 product leaves out: f and e are
+// kept apart because the anchor's offset can cancel f).
+struct RingPlace {
+    float Di, K, f, e;
+    int at;
+};
+__device__ __forceinline__ RingPlace place_ring(const SamplePlan& p, const RingT& rt)
+{
+    RingPlace g;
+    // dec - dec0: the difference of the high parts and its exact rounding
+    // error, plus the low parts; then sin and 1 - cos at the FP32 value, with
+    // a first-order correction for what it leaves out
+    const float a = rt.dec_hi - p.dec_hi;
+    const float b = a - rt.dec_hi;
+    const float e = (rt.dec_hi - (a - b)) - (p.dec_hi + b);
+    const float t = e + (rt.dec_lo - p.dec_lo);
+    const float df = a + t;
+    const float de = t - (df - a);
+    float sD, hD;
+    sin_versin(df, sD, hD);
+    g.Di = fmaf(de, 1.0f - hD, sD);
+    g.K = fmaf(de, sD, hD);
+    // the product of the two pairs, its rounding error by a fused multiply-add
+    const float m = p.phi_hi * rt.fr_hi;
+    g.e = fmaf(p.phi_hi, rt.fr_lo, fmaf(p.phi_lo, rt.fr_hi, fmaf(p.phi_hi, rt.fr_hi, -m)));
+    const float n = (m + 12582912.0f) - 12582912.0f;  // rint(m), |m| < 2^22
+    g.f = __fsub_rn(m, n);  // (not contracted with m's product: e holds its error)
+    g.at = small_float_to_int(n);
+    return g;
+}
+
+// The disc's range on a ring: the edge longitude in FP32 from
+//   1 - cos D = (1 - cos radius - (1 - cos(dec - dec0))) / (s s0),
+// the exact FP64 HEALPix formula (disc_ring) whenever an edge lies within the
+// FP32 angle's error of a pixel boundary.  Same pixels as disc_ring.
+//
+// The error: with C = 1 - cos radius, H = C / (s s0) and D the edge angle,
+// the numerator is off by at most 3.6e-7 C (K to 3e-7, C and the difference
+// to half an ulp), 1 - cos D by 7.2e-7 H, D by 7.2e-7 H / sin D + 6e-7 D, and a
+// position of fr D pixels by 3e-7 fr D + 2e-7 more (products, sums and f); the
+// margin is 1e-6 fr (H / sin D + D) + 3e-7 pixels, at least 1.1 times that.  At
+// nside 1024 and 3 degrees it is 6e-5 pixels: two rings in ten thousand take
+// the exact formula.
+__device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePlan& p, int ring,
+                                                    const RingT& rt, const RingPlace& g)
 {
     RingRange s = {0, 0};
     const int npix = rt.npix2 >> 1;
@@ -442,22 +508,23 @@ __device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePl
         s.n = npix;
         return s;
     }
-    const double x = PD_MUL(PD_SUB(cosr, PD_MUL(rt.z, p.z0)), p.xa);
-    const double ysq = PD_SUB(rt.omz2, PD_MUL(x, x));
-    if (!(ysq > 0.0)) return s;  // no intersection (HEALPix: dphi = 0, ring skipped)
-    const float de = atan2f(sqrtf((float)ysq), (float)x);
-    const double shift = (rt.npix2 & 1) ? 0.5 : 0.0;
-    const double fr = rt.fr;
-    const double vlo = fr * (p.phi - (double)de) - shift;
-    const double vhi = fr * (p.phi + (double)de) - shift;
-    // |de - atan2(sqrt(ysq), x)| <= 3e-7 de (FP32 rounding of x, ysq and atan2f)
-    const double m = fr * (4e-7 * (double)de) + 1e-9;
-    const double flo = vlo - floor(vlo), fhi = vhi - floor(vhi);
-    if (!(de > 0.0f) || flo < m || flo > 1.0 - m || fhi < m || fhi > 1.0 - m) {
+    const float is = 1.0f / (rt.s * p.s0f);
+    const float x = (p.versr - g.K) * is;  // 1 - cos D
+    const float y = sqrtf(x * (2.0f - x));
+    const float D = atan2f(y, 1.0f - x);
+    const float shift = (rt.npix2 & 1) ? 0.5f : 0.0f;
+    const float w = rt.fr_hi * D;
+    const float at = (g.f - shift) + g.e;
+    const float vlo = at - w, vhi = at + w;
+    const float flo = floorf(vlo), fhi = floorf(vhi);
+    // y = 0 or a NaN (an edge outside [0, pi]) makes m infinite or a NaN
+    const float m = fmaf(1e-6f, rt.fr_hi * (p.versr * is / y + D), 3e-7f);
+    const float rlo = vlo - flo, rhi = vhi - fhi;
+    if (!(fminf(rlo, rhi) > m && fmaxf(rlo, rhi) < 1.0f - m) || (p.flags & kPlanExact)) {
         DiscPlan d;
         d.z0 = p.z0;
         d.xa = p.xa;
-        d.cosr = cosr;
+        d.cosr = p.cosr;
         d.phi = p.phi;
         d.ring_lo = p.ring_lo;
         d.ring_hi = p.ring_hi;
@@ -470,7 +537,7 @@ __device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePl
         if (s.n <= 0) s = RingRange{0, 0};
         return s;
     }
-    const int lo = (int)floor(vlo) + 1, hi = (int)floor(vhi);
+    const int lo = g.at + (int)flo + 1, hi = g.at + (int)fhi;
     if (lo > hi) return s;
     s.lo = lo < 0 ? lo + npix : (lo >= npix ? lo - npix : lo);
     s.n = hi - lo + 1;
@@ -772,23 +839,6 @@ __device__ __forceinline__ void flush(const Hpx& hs, WarpSmem& S, Queue& Q, int 
     if (Q.n > 0) drain<kBil>(hs, Q.n, S, Q, lane, err, act);
 }
 
-// sin(x) and 1 - cos(x): Taylor series for |x| <= 0.5 (truncation below
-// 3e-11 relative), CUDA sincosf beyond.
-__device__ __forceinline__ void sin_versin(float x, float& sn, float& h)
-{
-    if (fabsf(x) <= 0.5f) {
-        const float x2 = x * x;
-        sn = x * fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, 2.75573192e-6f, -1.98412698e-4f),
-                                        8.33333333e-3f), -1.66666667e-1f), 1.0f);
-        h = x2 * fmaf(x2, fmaf(x2, fmaf(x2, fmaf(x2, 2.75573192e-7f, -2.48015873e-5f),
-                                        1.38888889e-3f), -4.16666667e-2f), 0.5f);
-    } else {
-        float cs;
-        sincosf(x, &sn, &cs);
-        h = (cs > 0.0f) ? (sn * sn) / (1.0f + cs) : 1.0f - cs;
-    }
-}
-
 // The same for |x| <= kShortOffset, two terms fewer each (truncation below
 // 8e-10 relative, an eightieth of an FP32 ulp).
 __device__ __forceinline__ void short_sin_versin(float x, float& sn, float& h)
@@ -1017,16 +1067,16 @@ __device__ __forceinline__ void psi_phasor(double s, double c, float& sf, float&
 {
     const bool swap = fabs(s) > fabs(c);
     const double big = swap ? s : c, small = swap ? c : s;
+    // small / big as the sum of two FP32 values: the trials then run in FP32
     const double ratio = small / big;
+    const float rh = (float)ratio, rl = (float)(ratio - (double)rh);
     const float b0 = (float)big;
-    float bb = b0, bs = (float)(ratio * (double)b0);
-    float best = 1.0f;
+    float bb = b0, bs = rh * b0, best = 1.0f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         const float b = b0 * (1.0f - 0.03125f * (float)i);
-        const double p = ratio * (double)b;
-        const float r = (float)p;
-        const float e = fabsf((float)(p - (double)r)) / fabsf(b);
+        const float r = rh * b;
+        const float e = fabsf(fmaf(rl, b, fmaf(rh, b, -r)) * rcp_approx(b));
         if (e < best) {
             best = e;
             bb = b;
@@ -1061,20 +1111,25 @@ __device__ __forceinline__ SamplePlan make_plan(const Hpx& hs, const Beam& B, do
     // which decides the flip as in the reference chain; they can differ
     // only within an ulp of the poles, where the frame is rebuilt from dec.
     const bool flip = fabs(dec) < 1.5707963 ? false : cos(dec) < 0.0;
-    double z0d, s0d;
+    double z0d, s0d, phi_f, dec0;
     if (flip == P.flip) {
         z0d = P.z0;
         s0d = P.s0;
-        sp.phi_f = P.phi;
-        sp.dec0 = PD_SUB(kHalfPi, P.theta);
+        phi_f = P.phi;
+        dec0 = PD_SUB(kHalfPi, P.theta);
     } else {
         double sdec, cdec;
         sincos(dec, &sdec, &cdec);
         z0d = sdec;
         s0d = fabs(cdec);
-        sp.phi_f = fmodulo(flip ? ra + kPi : ra, kTwoPi);
-        sp.dec0 = atan2(z0d, s0d);
+        phi_f = fmodulo(flip ? ra + kPi : ra, kTwoPi);
+        dec0 = atan2(z0d, s0d);
     }
+    sp.phi_hi = (float)phi_f;
+    sp.phi_lo = (float)(phi_f - (double)sp.phi_hi);
+    sp.dec_hi = (float)dec0;
+    sp.dec_lo = (float)(dec0 - (double)sp.dec_hi);
+    sp.versr = B.versr;
     sp.z0f = (float)z0d;
     sp.s0f = (float)s0d;
     double spsi, cpsi;
@@ -1088,7 +1143,7 @@ __device__ __forceinline__ SamplePlan make_plan(const Hpx& hs, const Beam& B, do
     sp.ring_hi = (int)P.ring_hi;
     sp.full_lo = (int)P.full_lo;
     sp.full_hi = (int)P.full_hi;
-    sp.flags = P.all_sky ? kPlanAllSky : 0;
+    sp.flags = (P.all_sky ? kPlanAllSky : 0) | (flip == P.flip ? 0 : kPlanExact);
     return sp;
 }
 
@@ -1178,7 +1233,8 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
         RingC rc;
         if (ring <= PL.full_hi) {
             const RingT rt = rings[ring - 1];
-            RingRange sp = fast_disc_ring(hs, PL, PL.cosr, ring, rt);
+            const RingPlace g = place_ring(PL, rt);
+            RingRange sp = fast_disc_ring(hs, PL, ring, rt, g);
             const int nr = rt.npix2 >> 1;
             // every pixel of the ring's range must lie in the sky map:
             // checked here, once per ring, instead of once per pair
@@ -1189,33 +1245,26 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
             }
             cnt = sp.n;
             if (cnt) {
-                const double sh = (rt.npix2 & 1) ? 0.5 : 0.0;
-                const double phi_f = PL.phi_f;
-                const double jc = floor(phi_f * rt.fr - sh + 0.5);
-                rc.dc = (float)((jc + sh) * rt.dphi - phi_f);
-                rc.dphi = rt.dphif;
-                // sin and 1 - cos of the latitude offset D: FP32 series at the
-                // rounded offset, first-order correction by its rounding error
-                const double dd = rt.dec - PL.dec0;
-                const float df = (float)dd;
-                const float de = (float)(dd - (double)df);
-                float sD, hD;
-                sin_versin(df, sD, hD);
-                const float Di = fmaf(de, 1.0f - hD, sD);
-                rc.Ki = R2 * fmaf(de, sD, hD);
+                // the anchor: the pixel centre nearest to the boresight's longitude
+                const float sh = (rt.npix2 & 1) ? 0.5f : 0.0f;
+                const float near = floorf(g.f - sh + 0.5f);
+                const int jc = g.at + (int)near;
+                rc.dc = (((near + sh) - g.f) - g.e) * rt.dphi;
+                rc.dphi = rt.dphi;
+                rc.Ki = R2 * g.K;
                 rc.s = rt.s;
-                rc.Wz = F.s0 * rt.zf;
-                rc.Di = Di;
+                rc.Wz = F.s0 * rt.z;
+                rc.Di = g.Di;
                 rc.nr = nr;
                 rc.start = rt.start;
                 // offsets from the anchor, the range centred on it; a whole
                 // ring starts half a turn from it
                 if (cnt == nr) {
-                    int lo = (int)jc - (nr >> 1);
+                    int lo = jc - (nr >> 1);
                     lo += lo < 0 ? nr : 0;
                     sp.lo = lo >= nr ? lo - nr : lo;
                 }
-                int kk = sp.lo - (int)jc;
+                int kk = sp.lo - jc;
                 const int mid = kk + (cnt >> 1);
                 if (mid >= (nr >> 1) + 1) kk -= nr;
                 else if (mid < -(nr >> 1)) kk += nr;
@@ -1228,7 +1277,7 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 rc.j0 = kUnits ? sp.lo & ~1 : sp.lo;
                 items = kUnits ? (hi >> 1) - (sp.lo >> 1) + 1 : cnt;
                 const int far = max(-kk, kk + cnt);
-                wide = (float)far * rt.dphif > kShortOffset - rt.dphif;
+                wide = (float)far * rt.dphi > kShortOffset - rt.dphi;
             }
         }
         int incl = items;
