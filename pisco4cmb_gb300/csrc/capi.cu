@@ -634,6 +634,13 @@ pisco_status pisco_forward_device(pisco_ctx* c, pisco_form form, long begin, lon
     a.err = c->d_err;
     a.fallbacks = c->d_fallbacks;
     cudaError_t e;
+    const bool tuned = tuned_supported(c->nside_beam, (int)c->npix_beam, c->rho_max);
+    // PLAIN and FP64 with the nearest lookup walk the TUNED geometry's pairs
+    // (fwd_exact.cu); the bilinear lookup, and beams outside that geometry's
+    // domain (reaching beyond the polar cap of their grid), take the chain
+    const bool exact = tuned && c->interp == PISCO_BEAM_NEAREST;
+    void* plans = nullptr;
+    long long plan_cap = 0;
     if (form == PISCO_FORM_FP64) {
         const long long npix = 12LL * c->nside_sky * c->nside_sky;
         if (!c->sky64_valid) {
@@ -650,22 +657,25 @@ pisco_status pisco_forward_device(pisco_ctx* c, pisco_form form, long begin, lon
         }
         a.sky64 = c->sky64;
         a.beam64 = c->beam64;
-        e = launch_forward_plain(a, true, c->sm_count, s);
-    } else if (form == PISCO_FORM_TUNED &&
-               tuned_supported(c->nside_beam, (int)c->npix_beam, c->rho_max)) {
+        if (exact) {
+            c->plan_scratch(n, s, &plans, &plan_cap);
+            e = launch_forward_exact(a, true, c->sm_count, s, plans, plan_cap);
+        } else {
+            e = launch_forward_plain(a, true, c->sm_count, s);
+        }
+    } else if (form == PISCO_FORM_TUNED && tuned) {
         CK(cudaMemsetAsync(c->d_fallbacks, 0, sizeof(unsigned long long), s), "reset fallbacks");
-        void* plans = nullptr;
-        long long plan_cap = 0;
 #if PISCO_FWD_PLANS
         c->plan_scratch(n, s, &plans, &plan_cap);
 #endif
         e = launch_forward_tuned(a, c->sm_count, s, plans, plan_cap);
-        if (plans) c->plans_used(s);
+    } else if (exact) {
+        c->plan_scratch(n, s, &plans, &plan_cap);
+        e = launch_forward_exact(a, false, c->sm_count, s, plans, plan_cap);
     } else {
-        // PLAIN, and TUNED outside the tuned geometry's domain (a beam
-        // reaching beyond the polar cap of its grid).
         e = launch_forward_plain(a, false, c->sm_count, s);
     }
+    if (plans) c->plans_used(s);
     if (a.order) c->order_used(s);
     if (e != cudaSuccess) return cuda_fail(c, e, "forward launch");
     if (s != c->stream) {

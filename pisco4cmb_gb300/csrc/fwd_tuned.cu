@@ -143,6 +143,20 @@ __global__ void ring_table_kernel(int nside, RingT* rings)
     }
 }
 
+}  // namespace
+
+void launch_plans(const FwdArgs& a, tuned::SamplePlan* plans, long long pos0, long long pos1,
+                  cudaStream_t st)
+{
+    // small blocks, so that a short launch's plans spread over the SMs: a plan
+    // is a chain of some 300 FP64 instructions, and eight warps on one SM queue
+    // for its FP64 pipe
+    const long long b = (pos1 - pos0 + 63) / 64;
+    plan_kernel<<<(int)(b < 65536 ? b : 65536), 64, 0, st>>>(a, plans, pos0, pos1);
+}
+
+namespace {
+
 template <class K>
 int resident_blocks(K kernel, int threads)
 {
@@ -163,10 +177,7 @@ void launch_shape(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib,
     const long long step = kPlanned ? plan_cap : a.n;
     for (long long p0 = 0; p0 < a.n; p0 += step) {
         const long long p1 = p0 + step < a.n ? p0 + step : a.n;
-        if (kPlanned) {
-            const long long pb = (p1 - p0 + 255) / 256;
-            plan_kernel<<<(int)(pb < 65536 ? pb : 65536), 256, 0, st>>>(a, plans, p0, p1);
-        }
+        if (kPlanned) launch_plans(a, plans, p0, p1, st);
         const long long need = (p1 - p0 + kTW - 1) / kTW;
         tuned_kernel<kCalib, kBil, kTW, kPlanned>
             <<<(int)(resident < need ? resident : need), threads, 0, st>>>(a, calib, plans, p0, p1);

@@ -229,6 +229,13 @@ constexpr size_t kSamplePlanBytes = 96;
 cudaError_t launch_forward_tuned(const FwdArgs& a, int sm_count, cudaStream_t st,
                                  void* plans = nullptr, long long plan_cap = 0);
 bool tuned_supported(int nside_beam, int npix_beam, double rho_max);
+// The sample plans of positions [pos0, pos1) into plans[0 ...) (fwd_tuned.cu).
+void launch_plans(const FwdArgs& a, tuned::SamplePlan* plans, long long pos0, long long pos1,
+                  cudaStream_t st);
+// PLAIN and FP64 forms with the nearest lookup, for beams that tuned_supported
+// accepts (fwd_exact.cu); plans as launch_forward_tuned's.
+cudaError_t launch_forward_exact(const FwdArgs& a, bool f64, int sm_count, cudaStream_t st,
+                                 void* plans, long long plan_cap);
 // Same kernel with every FP32 decision also evaluated in FP64: writes the
 // worst |FP32 - FP64| / margin seen over the non-fallback pairs to *calib.
 cudaError_t launch_tuned_calibrate(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib);

@@ -95,6 +95,12 @@ template <class A, class = void>
 struct HasOutside : std::false_type {};
 template <class A>
 struct HasOutside<A, std::void_t<decltype(&A::outside)>> : std::true_type {};
+// Does the action take the pair's phasor in FP64 (the PLAIN and FP64 forms,
+// fwd_exact.cu)?
+template <class A, class = void>
+struct IsExact : std::false_type {};
+template <class A>
+struct IsExact<A, std::void_t<decltype(&A::pair64)>> : std::true_type {};
 // Does the action take two pixels per lane?
 template <class A, class = void>
 struct HasPair2 : std::false_type {};
@@ -183,13 +189,26 @@ constexpr int kPlanExact = 4;  // the frame is not the disc's (an ulp from a pol
 // Per-warp shared state: one ring batch, the samples in flight, the FP64
 // re-evaluation queue (sky pixel, slot) and the current sample's plan (read
 // from here where needed rather than held in registers across the pair loop).
-struct WarpSmem {
+template <class Real>
+struct WarpState {
     SamplePlan plan;
     RingC r[32];
     Pend p[kPend];
     int q[kQCap];
     unsigned char qs[kQCap];
-    float ta[32], tb[32];
+    Real ta[32], tb[32];  // re-evaluated pairs of a drain
+};
+using WarpSmem = WarpState<float>;
+
+// One disc ring of the current batch in FP64, and the sample's frame: what the
+// phasor of an IsExact action is formed from.
+struct RingD {
+    double dc, dphi;      // anchor offset, pixel spacing
+    double s, Zs, Wz, Di; // s, s z0, s0 z, sin(dec - dec0)
+};
+struct ExactSmem : WarpState<double> {
+    RingD rd[32];
+    double z0, s0, c2p, s2p;  // sin and |cos| of the latitude, cos and sin of 2 psi
 };
 
 // Warp-uniform queue state, in registers.
@@ -755,11 +774,11 @@ __device__ __forceinline__ bool stencil_f32(const Beam& B, int qd, float tp, flo
 // order, by the first lane of each run of one slot's entries), writes the TOD
 // of every sample left with nothing queued, and drops the m entries.  kBil:
 // the beam value is PLAIN's bilinear one instead of the nearest pixel's.
-template <bool kBil = false, class Action>
-__device__ __forceinline__ void drain(const Hpx& hs, int m, WarpSmem& S, Queue& Q, int lane,
+template <bool kBil = false, class Smem, class Action>
+__device__ __forceinline__ void drain(const Hpx& hs, int m, Smem& S, Queue& Q, int lane,
                                       unsigned int* err, Action& act)
 {
-    float ta = 0.0f, tb = 0.0f;
+    std::remove_reference_t<decltype(S.ta[0])> ta = 0, tb = 0;
     int slot = -1;
     if (lane < m) {
         slot = S.qs[lane];
@@ -783,8 +802,11 @@ __device__ __forceinline__ void drain(const Hpx& hs, int m, WarpSmem& S, Queue& 
         } else if (bp < 0) {
             record(err, kCheckBeamIndex);
         } else if (bp < P.npix_beam) {
-            act.deferred(P, pix, load_beam(P.beam + bp), (int)bp, (float)cos(2.0 * chi),
-                         (float)sin(2.0 * chi), ta, tb);
+            if constexpr (IsExact<Action>::value)
+                act.deferred64(pix, (int)bp, cos(2.0 * chi), sin(2.0 * chi), ta, tb);
+            else
+                act.deferred(P, pix, load_beam(P.beam + bp), (int)bp, (float)cos(2.0 * chi),
+                             (float)sin(2.0 * chi), ta, tb);
         } else if constexpr (HasOutside<Action>::value) {
             act.outside_deferred(P, pix, (int)bp);
         }
@@ -832,8 +854,8 @@ __device__ __forceinline__ void drain(const Hpx& hs, int m, WarpSmem& S, Queue& 
 // Redoes every queued pair (at a sample boundary, where fewer than 32 are
 // queued): all slots are free afterwards.  Called once more before a warp
 // leaves the kernel.
-template <bool kBil = false, class Action>
-__device__ __forceinline__ void flush(const Hpx& hs, WarpSmem& S, Queue& Q, int lane,
+template <bool kBil = false, class Smem, class Action>
+__device__ __forceinline__ void flush(const Hpx& hs, Smem& S, Queue& Q, int lane,
                                       unsigned int* err, Action& act)
 {
     if (Q.n > 0) drain<kBil>(hs, Q.n, S, Q, lane, err, act);
@@ -1049,6 +1071,67 @@ struct Unit {
     bool in0, in1;
 };
 
+// The FP64 ring constants of an IsExact action: ring jc the anchor's index.
+__device__ __forceinline__ RingD ring_exact(const Hpx& hs, int ring, int jc, const RingT& rt,
+                                            const SamplePlan& p, double z0, double s0)
+{
+    RingD r;
+    const int ns = (int)hs.nside;
+    const int north = ring > 2 * ns ? 4 * ns - ring : ring;
+    double z;
+    if (north < ns) {  // polar caps: z = 1 - t
+        const double t = (double)north * (double)north * hs.fact2;
+        z = ring == north ? 1.0 - t : t - 1.0;
+        r.s = sqrt(t * (2.0 - t));
+    } else {
+        z = (double)(2 * ns - ring) * hs.fact1;
+        r.s = sqrt((1.0 - z) * (1.0 + z));
+    }
+    const double phi = p.flags & kPlanExact ? (double)p.phi_hi + (double)p.phi_lo : p.phi;
+    r.dphi = kTwoPi / (double)(rt.npix2 >> 1);
+    r.dc = fma((double)jc + ((rt.npix2 & 1) ? 0.5 : 0.0), r.dphi, -phi);
+    r.Zs = r.s * z0;
+    r.Wz = s0 * z;
+    r.Di = z * s0 - r.s * z0;
+    return r;
+}
+
+// exp(2i chi) of a pair in FP64 without trigonometric functions of its
+// angles: sin D and 1 - cos D by their Taylor series (narrow: |D| <=
+// kShortOffset, truncated below 3e-17 relative), then phasor's w, turned by
+// psi.  About 45 FP64 instructions, against some 600 of the reference chain's
+// arccosines, arctangents, sines and cosines, on a GPU that issues one FP64
+// instruction in the time of 64 FP32 ones.
+__device__ __forceinline__ void phasor_exact(const RingD& R, double kf, bool narrow, double s0,
+                                             double c2p, double s2p, double& c2, double& s2)
+{
+    const double x = fma(kf, R.dphi, R.dc);
+    double sn, h;
+    if (narrow) {
+        const double x2 = x * x;
+        sn = fma(x2, 1.0 / 362880.0, -1.0 / 5040.0);
+        sn = fma(x2, sn, 1.0 / 120.0);
+        sn = fma(x2, sn, -1.0 / 6.0);
+        sn = fma(x * x2, sn, x);
+        h = fma(x2, 1.0 / 3628800.0, -1.0 / 40320.0);
+        h = fma(x2, h, 1.0 / 720.0);
+        h = fma(x2, h, -1.0 / 24.0);
+        h = x2 * fma(x2, h, 0.5);
+    } else {
+        double cs;
+        sincos(x, &sn, &cs);
+        h = cs > 0.0 ? sn * sn / (1.0 + cs) : 1.0 - cs;
+    }
+    const double u = R.s * sn, v = fma(R.Zs, h, R.Di);
+    const double nb = s0 * sn, db = fma(R.Wz, h, -R.Di);
+    const double wr = fma(db, v, -(nb * u)), wi = fma(db, u, nb * v);
+    const double rr = wr * wr;
+    const double iw = 1.0 / fma(wi, wi, rr);
+    const double er = fma(-wi, wi, rr) * iw, ei = wr * wi * (iw + iw);
+    c2 = fma(er, c2p, -(ei * s2p));
+    s2 = fma(ei, c2p, er * s2p);
+}
+
 // 1 << x, 0 for x outside [0, 32).
 __device__ __forceinline__ unsigned bit_or_0(int x)
 {
@@ -1153,11 +1236,11 @@ __device__ __forceinline__ SamplePlan make_plan(const Hpx& hs, const Beam& B, do
 // and npairs the disc pairs (lane 0 only); cmax (kCalib) is the worst FP32
 // decision error over the non-queued pairs, in units of the margin.  kBil:
 // bilinear beam lookup (bilinear_f32; only the degenerate pairs are queued).
-template <bool kCalib, bool kBil = false, class Action>
+template <bool kCalib, bool kBil = false, class Smem, class Action>
 __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& hs,
                                                const RingT* rings, const Hpx& hb, const Beam& B,
                                                double ra, double dec, double pa, const Out& o,
-                                               WarpSmem& S, Queue& Qs, int lane,
+                                               Smem& S, Queue& Qs, int lane,
                                                unsigned int* err, Action& act,
                                                unsigned long long& nfall, float& cmax,
                                                unsigned long long& npairs)
@@ -1201,6 +1284,20 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
     __syncwarp();
     if constexpr (Action::kSums) act.reset();
     const SamplePlan& PL = S.plan;
+    if constexpr (IsExact<Action>::value) {
+        // the frame in FP64: lanes 0 and 1 take sin and cos of dec and 2 psi in
+        // the same instructions
+        double sn, cs;
+        sincos(lane & 1 ? -2.0 * pa : dec, &sn, &cs);
+        if (lane == 0) {
+            S.z0 = sn;
+            S.s0 = fabs(cs);
+        } else if (lane == 1) {
+            S.c2p = cs;
+            S.s2p = sn;
+        }
+        __syncwarp();
+    }
     // what the pair loop reads on every pair, in registers
     const float R2 = B.rscale * B.rscale;
     const Frame F{PL.z0f, PL.s0f, R2 * PL.s0f, PL.sps, PL.cps};
@@ -1231,6 +1328,7 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
         int cnt = 0, items = 0;  // the ring's disc pixels; its lane slots
         bool wide = false;
         RingC rc;
+        [[maybe_unused]] RingD rd;
         if (ring <= PL.full_hi) {
             const RingT rt = rings[ring - 1];
             const RingPlace g = place_ring(PL, rt);
@@ -1269,6 +1367,8 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 if (mid >= (nr >> 1) + 1) kk -= nr;
                 else if (mid < -(nr >> 1)) kk += nr;
                 rc.kc = 0x4B400000 + kk - sp.lo;
+                if constexpr (IsExact<Action>::value)
+                    rd = ring_exact(hs, ring, jc, rt, PL, S.z0, S.s0);
                 const int hi = sp.lo + cnt - 1;  // below 2^16: rings hold at most 2^15 pixels
                 rc.ends = sp.lo | hi << 16;
                 // two pixels per lane: ring indices 2m and 2m + 1, which are
@@ -1302,6 +1402,7 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
         if (items > 0) {
             rc.j0 -= (kUnits ? 2 : 1) * first;
             W[__popc(some & lt_mask)] = rc;
+            if constexpr (IsExact<Action>::value) S.rd[__popc(some & lt_mask)] = rd;
         }
         const bool narrow = !__any_sync(kFull, wide);
         __syncwarp();
@@ -1390,7 +1491,13 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                         cmax = fmaxf(cmax, (float)fmax(fmax(e1, e2), e3) / kMarginRel);
                     }
                     if (!fb) {
-                        if ((unsigned)c.bp < (unsigned)B.npix) {  // 0 <= bp < npix
+                        if constexpr (IsExact<Action>::value) {
+                            if ((unsigned)c.bp < (unsigned)B.npix) {
+                                double c2, s2;
+                                phasor_exact(S.rd[k], (double)kf, narrow, S.s0, S.c2p, S.s2p, c2, s2);
+                                act.pair64(pix, c.bp, c2, s2);
+                            }
+                        } else if ((unsigned)c.bp < (unsigned)B.npix) {  // 0 <= bp < npix
                             float c2, s2;
                             phasor(p, F.s0, R1.x, R1.y, c2, s2);
                             act.pair(pix, act.fetch(pix), load_beam(B.beam + c.bp), c.bp, c2, s2);
@@ -1422,10 +1529,10 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
 }
 
 // Processes one sample, its plan built here by the warp.
-template <bool kCalib, bool kBil = false, class Action>
+template <bool kCalib, bool kBil = false, class Smem, class Action>
 __device__ __forceinline__ void sample(const Hpx& hs, const RingT* rings, const Hpx& hb,
                                        const Beam& B, double ra, double dec, double pa,
-                                       const Out& o, WarpSmem& S, Queue& Qs, int lane,
+                                       const Out& o, Smem& S, Queue& Qs, int lane,
                                        unsigned int* err, Action& act, unsigned long long& nfall,
                                        float& cmax, unsigned long long& npairs)
 {
