@@ -20,8 +20,15 @@
 // plus the detector's polarization angle.  BPoint's ephemeris part (SOFA and
 // the JPL tables, absent from the reference tree) is not on this path.
 //
-// One thread per (detector, sample), FP64 throughout (the pointing feeds the
-// FP64 per-sample frame of the convolver); outputs [det * nsamples + s].
+// FP64 throughout (the pointing feeds the convolver's FP64 per-sample frame);
+// outputs [det * nsamples + s].  What bounds it is the FP64 pipe (16 cycles per
+// warp instruction on an SM), so the kernel spends as few instructions per
+// output as it can: a thread takes one sample and up to 16 detectors, the
+// detectors' sines and cosines are formed once per block and the sample's once
+// per thread, g needs no angle (sin r cos g = sin dy cos rot + sin dx cos dy sin
+// rot, sin r sin g = sin dx cos dy cos rot - sin dy sin rot), and the three
+// inverse functions go through one table (atan2_table).  96 detectors x 30,011
+// samples: 1.59 ms with everything formed per output, 0.63 ms with this.
 #include <cuda_runtime.h>
 
 #include <string>
@@ -38,38 +45,90 @@ using namespace pisco;
 
 namespace {
 
-__global__ void focal_plane_kernel(int ndets, const double* __restrict__ det_dx,
-                                   const double* __restrict__ det_dy,
-                                   const double* __restrict__ det_pol, long long ns,
-                                   const double* __restrict__ x_ac, const double* __restrict__ y_ac,
-                                   const double* __restrict__ rot_ac, int flag,
-                                   double* __restrict__ x_det, double* __restrict__ y_det,
-                                   double* __restrict__ rot_det)
+constexpr int kThreads = 128;
+constexpr int kMostDets = 16;  // detectors of a block
+
+// atan2(y, x) to about an ulp in some 20 FP64 instructions: an FP32 arctangent
+// picks the nearest multiple k of pi/64, the vector is turned back by it (tab:
+// cos and sin of k pi/64), and the rest, at most 0.0246, comes from the
+// arctangent's series to the ninth power (truncated below 1e-17 relative).
+__device__ __forceinline__ double atan2_table(double y, double x, const double2* tab)
 {
-    const long long total = (long long)ndets * ns;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total;
-         k += (long long)gridDim.x * blockDim.x) {
-        const int d = (int)(k / ns);
-        const long long s = k - (long long)d * ns;
-        double sx, cx, sdy, cdy;
-        sincos(det_dx[d], &sx, &cx);
-        sincos(det_dy[d], &sdy, &cdy);
-        const double cr = cx * cdy;
-        const double sr = sqrt((1.0 - cr) * (1.0 + cr));
-        const double a = atan2(sdy, sx * cdy);
-        const double rot = rot_ac[s];
-        double sg, cg, sl, cl, se, ce;
-        sincos(kHalfPi - a - rot, &sg, &cg);
+    if (!(fabs(x) + fabs(y) > 1e-30)) return atan2(y, x);  // zeros, NaNs
+    const int k = __float2int_rn(atan2f((float)y, (float)x) * 20.371832715762604f);
+    const double2 t = tab[k & 127];
+    const double d = (y * t.x - x * t.y) / (x * t.x + y * t.y);
+    const double d2 = d * d;
+    const double p = d2 * fma(d2, fma(d2, fma(d2, 1.0 / 9.0, -1.0 / 7.0), 1.0 / 5.0), -1.0 / 3.0);
+    // pi/64 as the sum of two doubles
+    const double r = fma((double)k, 1.9135106236677394e-18, fma(d, p, d));
+    return fma((double)k, 0.04908738521234052, r);
+}
+
+// asin(v); a NaN for |v| > 1.
+__device__ __forceinline__ double asin_table(double v, const double2* tab)
+{
+    return atan2_table(v, sqrt((1.0 - v) * (1.0 + v)), tab);
+}
+
+struct DetTrig {
+    double sx, cx, sy, cy, a, cr, pol;  // sin, cos of dx and dy; sin dx cos dy; cos dx cos dy
+};
+
+// Blocks take (group of `group` detectors, kThreads samples) items in turn.
+__global__ void __launch_bounds__(kThreads)
+    focal_plane_kernel(int ndets, int group, const double* __restrict__ det_dx,
+                       const double* __restrict__ det_dy, const double* __restrict__ det_pol,
+                       long long ns, const double* __restrict__ x_ac,
+                       const double* __restrict__ y_ac, const double* __restrict__ rot_ac, int flag,
+                       double* __restrict__ x_det, double* __restrict__ y_det,
+                       double* __restrict__ rot_det)
+{
+    __shared__ double2 tab[128];
+    __shared__ DetTrig det[kMostDets];
+    {
+        double s, c;
+        sincospi((double)threadIdx.x / 64.0, &s, &c);
+        tab[threadIdx.x] = make_double2(c, s);
+    }
+    const long long parts = (ns + kThreads - 1) / kThreads;
+    const long long items = parts * ((ndets + group - 1) / group);
+    for (long long item = blockIdx.x; item < items; item += gridDim.x) {
+        const int d0 = (int)(item / parts) * group;
+        const int nd = min(group, ndets - d0);
+        __syncthreads();  // tab, and the last item's detectors
+        if (threadIdx.x < nd) {
+            const int d = d0 + threadIdx.x;
+            DetTrig t;
+            sincos(det_dx[d], &t.sx, &t.cx);
+            sincos(det_dy[d], &t.sy, &t.cy);
+            t.a = t.sx * t.cy;
+            t.cr = t.cx * t.cy;
+            t.pol = det_pol[d];
+            det[threadIdx.x] = t;
+        }
+        __syncthreads();
+        const long long s = (item % parts) * kThreads + threadIdx.x;
+        if (s >= ns) continue;
+        double sl, cl, se, ce;
+        const double x = x_ac[s];
         sincos(y_ac[s], &sl, &cl);
-        sincos(rot, &se, &ce);
-        y_det[k] = asin(cr * sl + sr * cl * cg);
-        const double pa = atan2(cl * se * cx - sl * sx, cl * ce * cdy - (sl * cx + cl * se * sx) * sdy);
-        rot_det[k] = pa + det_pol[d];
-        if (flag == 2) {
-            x_det[k] = -pa;
-        } else {
-            const double dl = atan2(sr * sg, cr * cl - sr * sl * cg);
-            x_det[k] = flag == 0 ? x_ac[s] + dl : x_ac[s] - dl;
+        sincos(rot_ac[s], &se, &ce);
+        const double cse = cl * se, cce = cl * ce;
+        for (int i = 0; i < nd; ++i) {
+            const DetTrig& t = det[i];
+            const long long k = (long long)(d0 + i) * ns + s;
+            const double gc = t.sy * ce + t.a * se;  // sin r cos g
+            y_det[k] = asin_table(t.cr * sl + cl * gc, tab);
+            const double pa = atan2_table(cse * t.cx - sl * t.sx,
+                                          cce * t.cy - (sl * t.cx + cse * t.sx) * t.sy, tab);
+            rot_det[k] = pa + t.pol;
+            if (flag == 2) {
+                x_det[k] = -pa;
+            } else {
+                const double dl = atan2_table(t.a * ce - t.sy * se, t.cr * cl - sl * gc, tab);
+                x_det[k] = flag == 0 ? x + dl : x - dl;
+            }
         }
     }
 }
@@ -95,11 +154,14 @@ cudaError_t launch(int ndets, const double* dx, const double* dy, const double* 
                    const double* x, const double* y, const double* rot, int flag, double* xo,
                    double* yo, double* ro, cudaStream_t st)
 {
-    const long long total = (long long)ndets * ns;
-    if (total <= 0) return cudaSuccess;
-    const long long b = (total + 255) / 256;
-    focal_plane_kernel<<<(int)(b < 8192 ? b : 8192), 256, 0, st>>>(ndets, dx, dy, pol, ns, x, y,
-                                                                    rot, flag, xo, yo, ro);
+    if (ndets <= 0 || ns <= 0) return cudaSuccess;
+    // as many detectors per thread as leave about 16 warps for each of 152 SMs
+    const long long parts = (ns + kThreads - 1) / kThreads;
+    long long group = parts * ndets / (152 * 16 * 32 / kThreads);
+    group = group < 1 ? 1 : (group > kMostDets ? kMostDets : group);
+    const long long items = parts * ((ndets + group - 1) / group);
+    focal_plane_kernel<<<(int)(items < 16384 ? items : 16384), kThreads, 0, st>>>(
+        ndets, (int)group, dx, dy, pol, ns, x, y, rot, flag, xo, yo, ro);
     return cudaGetLastError();
 }
 
