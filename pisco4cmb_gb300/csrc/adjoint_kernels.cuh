@@ -82,10 +82,13 @@ struct Scatter {
     __device__ __forceinline__ void scatter(float wa, float wb, int pix, const F8& B, float c2,
                                            float s2) const
     {
-        const float gI = wa * B.a.x + wb * B.b.x;
-        const float gQ = wa * (B.a.y * c2 - B.a.z * s2) + wb * (-B.b.y * c2 + B.b.z * s2);
-        const float gU = wa * (B.a.z * c2 + B.a.y * s2) + wb * (-B.b.z * c2 - B.b.y * s2);
-        const float gV = want_v ? wa * B.a.w + wb * B.b.w : 0.0f;
+        // wa a - wb b turned by 2 chi, fused one way whatever surrounds it: the
+        // sky gradient is the same bit for bit in every action
+        const float q = fmaf(wa, B.a.y, -(wb * B.b.y)), u = fmaf(wa, B.a.z, -(wb * B.b.z));
+        const float gI = fmaf(wa, B.a.x, wb * B.b.x);
+        const float gQ = fmaf(q, c2, -(u * s2));
+        const float gU = fmaf(u, c2, q * s2);
+        const float gV = want_v ? fmaf(wa, B.a.w, wb * B.b.w) : 0.0f;
         if (kFixed) {
             // one plane per Stokes component: the lanes of a warp, on
             // consecutive pixels of a ring, add to consecutive words
@@ -135,6 +138,76 @@ struct ScatterBeam {
                                          float s2) const
     {
         scatter(ga, gb, pix, S, B, bp, c2, s2);
+    }
+
+    // The pairs of a warp.  A scattered atomic costs the path from L1 to L2 a
+    // sector each, a cycle and more, whatever it adds there, so lanes share
+    // sectors: four lanes turn their 4 x 4 values around and add the four
+    // 64-bit words of one detector's half pixel (a sector) at a time, two
+    // lanes the two float4s of a pixel: 64 sectors for 32 pairs instead of 192.
+    // Forward and DETERMINISTIC sky and beam maps, nside 256, 4 degree beam,
+    // 200,000 samples: 9.14 -> 6.87 ms.
+    __device__ __forceinline__ void pair_all(int pix, int bp, float c2, float s2) const
+    {
+        const unsigned lane = threadIdx.x & 31;
+        const bool in = bp >= 0;
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (in) {
+            beam_grad(ga, gb, fetch(pix), c2, s2, v);
+            if (want_sky) {
+                const Scatter<kFixed> sc{ga,      gb,      gsky,  gsky_fx, nullptr,
+                                         nullptr, nullptr, ssky,  sbeam,   want_v, plane};
+                sc.scatter(ga, gb, pix, tuned::load_beam(beam_base + bp), c2, s2);
+            }
+        }
+        __syncwarp();
+        if constexpr (kFixed) {
+            quad_turn(v, lane);
+            quad_turn(v + 4, lane);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                const int b = __shfl_sync(tuned::kFull, bp, (lane & ~3u) | m);
+                if (b < 0) continue;
+                unsigned long long* p = gbeam_fx + 8 * (long long)b + (lane & 3);
+                const unsigned long long x = Scatter<kFixed>::fx(v[m], sbeam);
+                const unsigned long long y = Scatter<kFixed>::fx(v[4 + m], sbeam);
+                if (x) atomicAdd(p, x);  // adding 0 changes nothing
+                if (y) atomicAdd(p + 4, y);
+            }
+        } else {
+            // even lanes add detector a's four values, odd lanes b's: first of
+            // the even lane's pixel, then of the odd lane's
+            const bool odd = lane & 1;
+            float own[4], got[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                got[k] = __shfl_xor_sync(tuned::kFull, odd ? v[k] : v[4 + k], 1);
+                own[k] = odd ? v[4 + k] : v[k];
+            }
+            const int other = __shfl_xor_sync(tuned::kFull, bp, 1);
+            const float4 o4 = make_float4(own[0], own[1], own[2], own[3]);
+            const float4 g4 = make_float4(got[0], got[1], got[2], got[3]);
+            float4* p = reinterpret_cast<float4*>(gbeam) + (lane & 1);
+            const int b0 = odd ? other : bp, b1 = odd ? bp : other;
+            if (b0 >= 0) atomicAdd(p + 2 * (long long)b0, odd ? g4 : o4);
+            if (b1 >= 0) atomicAdd(p + 2 * (long long)b1, odd ? o4 : g4);
+        }
+    }
+    // lane q's value m becomes lane m's value q, in each group of four lanes
+    __device__ __forceinline__ static void quad_turn(float* v, unsigned lane)
+    {
+#pragma unroll
+        for (int k = 0; k < 4; k += 2) {
+            const float x = __shfl_xor_sync(tuned::kFull, lane & 1 ? v[k] : v[k + 1], 1);
+            if (lane & 1) v[k] = x;
+            else v[k + 1] = x;
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float x = __shfl_xor_sync(tuned::kFull, lane & 2 ? v[k] : v[k + 2], 2);
+            if (lane & 2) v[k] = x;
+            else v[k + 2] = x;
+        }
     }
 
     __device__ __forceinline__ void pair_stencil(int pix, const float4& S, const int px[4],
@@ -244,6 +317,7 @@ struct ScatterBeam {
 // sum_i w_i B[b_i], and each stencil pixel gets w_i of s.
 template <bool kFixed>
 struct ScatterParams {
+    static constexpr bool kL1 = false;  // load_beam
     static constexpr bool kSums = false;
     static constexpr bool kStencil = true;
     float ga, gb;
@@ -274,6 +348,26 @@ struct ScatterParams {
         tuned::two_sum(acc[3], cmp[3], sp * t.a.w);
         tuned::two_sum(acc[4], cmp[4], sp * t.b.x);
         tuned::two_sum(acc[5], cmp[5], sp * t.b.y);
+    }
+    // Two neighbouring pixels per lane, as the forward takes them: their sky
+    // values and their ring's constants are read once (sky and parameters,
+    // nside 256, 4 degree beam, 200,000 samples: 5.42 -> 5.07 ms).  The actions
+    // that only scatter do not gain: their lanes' atomics would lie two pixels
+    // apart (back-projection 2.34 -> 2.65 ms, DETERMINISTIC 3.86 -> 4.86 ms).
+    __device__ __forceinline__ void fetch2(int pix, float4& S0, float4& S1) const
+    {
+        tuned::load_sky2(sky + pix, S0, S1);
+    }
+    __device__ __forceinline__ void pair2(const tuned::Unit& U)
+    {
+        const float c0 = tuned::lo2(U.c), s0 = tuned::lo2(U.s);
+        const float c1 = tuned::hi2(U.c), s1 = tuned::hi2(U.s);
+        if (want_sky) {
+            if (U.in0) sc.scatter(ga, gb, U.pix, U.B0, c0, s0);
+            if (U.in1) sc.scatter(ga, gb, U.pix + 1, U.B1, c1, s1);
+        }
+        if (U.in0) add(ga, gb, U.S0, c0, s0, U.bp0, 1.0f);
+        if (U.in1) add(ga, gb, U.S1, c1, s1, U.bp1, 1.0f);
     }
     __device__ __forceinline__ void pair(int pix, const float4& S, const F8& B, int bp, float c2,
                                          float s2)
@@ -338,13 +432,15 @@ template <class A>
 struct HasFinish<A, std::void_t<decltype(&A::finish)>> : std::true_type {};
 
 // Warps per SM of an instance: the planned nearest lookup runs 32 (register
-// cap 64, its plan and descriptors in shared memory, as the forward does),
-// the others 16 (cap 128).  The DETERMINISTIC beam-map gradient stays at 16:
-// its action spills at 64 registers (c5: 95 ms against 87 ms).
+// cap 64, its plan and descriptors in shared memory), 24 with two pixels per
+// lane (cap 80; 16 at 128 took 5.41 against 5.07 ms), the others 16 (cap 128).
+// The DETERMINISTIC beam-map gradient stays at 16: its action spills at 64
+// registers.
 template <class Act, bool kBil, bool kPlanned>
 constexpr int adj_warps_per_sm()
 {
-    return kPlanned && !kBil && !std::is_same_v<Act, ScatterBeam<true>> ? 32 : 16;
+    if (!kPlanned || kBil || std::is_same_v<Act, ScatterBeam<true>>) return 16;
+    return tuned::HasPair2<Act>::value ? 24 : 32;
 }
 
 // kBil: the transpose of the TUNED forward with the bilinear beam lookup.
@@ -354,7 +450,7 @@ template <class Act, bool kBil, bool kPlanned>
 __global__ void __launch_bounds__(kAW * 32, adj_warps_per_sm<Act, kBil, kPlanned>() / kAW)
     adjoint_kernel(AdjArgs a, Act proto)
 {
-    constexpr bool kDescSmem = adj_warps_per_sm<Act, kBil, kPlanned>() == 32;
+    constexpr bool kDescSmem = kPlanned && !kBil;
     __shared__ tuned::WarpSmem sm[kAW];
     __shared__ Hpx s_hs, s_hb;
     __shared__ tuned::Beam s_B;

@@ -101,6 +101,12 @@ template <class A, class = void>
 struct IsExact : std::false_type {};
 template <class A>
 struct IsExact<A, std::void_t<decltype(&A::pair64)>> : std::true_type {};
+// Does the action take the pairs of a warp together (every lane calls
+// pair_all, with beam pixel -1 where it has no pair)?
+template <class A, class = void>
+struct HasPairAll : std::false_type {};
+template <class A>
+struct HasPairAll<A, std::void_t<decltype(&A::pair_all)>> : std::true_type {};
 // Does the action take two pixels per lane?
 template <class A, class = void>
 struct HasPair2 : std::false_type {};
@@ -422,6 +428,15 @@ __device__ __forceinline__ F8 load_beam(const F8* p)
               "=f"(r.b.z), "=f"(r.b.w)
             : "l"(p));
     return r;
+}
+
+// Two neighbouring sky pixels, 32-byte aligned.
+__device__ __forceinline__ void load_sky2(const float4* p, float4& S0, float4& S1)
+{
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(S0.x), "=f"(S0.y), "=f"(S0.z), "=f"(S0.w), "=f"(S1.x), "=f"(S1.y), "=f"(S1.z),
+          "=f"(S1.w)
+        : "l"(p));
 }
 
 // A beam pixel of the bilinear stencil: its four pixels are two pairs of
@@ -921,7 +936,7 @@ __device__ __forceinline__ Spot locate(float kf, const Frame& F, const float4& R
     const unsigned sgn = (__float_as_uint(p.X) ^ __float_as_uint(p.Y)) & 0x80000000u;
     p.qd = (int)(2u * (__float_as_uint(p.Y) >> 31) + (sgn >> 31));
     p.tp = quarter_turns(p.X, p.Y, sgn);
-    p.r = p.q * rsqrt_approx(p.q);
+    p.r = __fmul_rn(p.q, rsqrt_approx(p.q));
     return p;
 }
 
@@ -953,12 +968,12 @@ struct CapPixel {
 __device__ __forceinline__ CapPixel cap_pixel(const Spot& p)
 {
     CapPixel c;
-    c.av = p.tp * p.r;
-    c.bv = fmaf(-p.tp, p.r, p.r);
+    c.av = __fmul_rn(p.tp, p.r);
+    c.bv = __fsub_rn(p.r, c.av);
     float ha, fa, hb, fb, hc, fc;
     const int ja = split_half(c.av, ha, fa), jb = split_half(c.bv, hb, fb);
     const float irf = ha + hb;
-    c.cv = p.tp * irf;
+    c.cv = __fmul_rn(p.tp, irf);
     const int jc = split_half(c.cv, hc, fc);
     // 1/2 less kMarginRel (r + 2), and r + 1 >= ir
     const float edge = fmaf(-kMarginRel, p.r, 0.5f - 2.0f * kMarginRel);
@@ -970,7 +985,9 @@ __device__ __forceinline__ CapPixel cap_pixel(const Spot& p)
 }
 
 // Two pairs of one ring, side by side: locate, cap_pixel and phasor with
-// every operation that has no ring constant packed.
+// every operation that has no ring constant packed, each rounded as the scalar
+// form rounds it (whichever form an action takes, a pair's decisions and
+// phasor are the same bit for bit).
 struct Spot2 {
     float sn0, sn1, h0, h1, q0, q1;
     F32x2 X, Y, tp, r;
@@ -1026,18 +1043,22 @@ __device__ __forceinline__ Spot2 locate2(float kf, const Frame& F, const float4&
     a = fma2(a, t2, both((float)(q * -0.3333314528)));
     a = fma2(a, t2, both((float)q));
     p.tp = pack2(__saturatef(fmaf(lo2(t), lo2(a), 0.5f)), __saturatef(fmaf(hi2(t), hi2(a), 0.5f)));
-    p.r = mul2(pack2(p.q0, p.q1), pack2(rsqrt_approx(p.q0), rsqrt_approx(p.q1)));
+    p.r = pack2(__fmul_rn(p.q0, rsqrt_approx(p.q0)), __fmul_rn(p.q1, rsqrt_approx(p.q1)));
     return p;
 }
 __device__ __forceinline__ void cap_pixel2(const Spot2& p, int& bp0, int& bp1, bool& near0,
                                            bool& near1)
 {
     const F32x2 k23 = both(kTwo23), khalf = both(8388607.5f);
-    const F32x2 av = mul2(p.tp, p.r), bv = sub2(p.r, av);
+    // (products that sums take are scalar: ptxas fuses a packed product into
+    // a packed sum, which the scalar form does not)
+    const F32x2 av = pack2(__fmul_rn(lo2(p.tp), lo2(p.r)), __fmul_rn(hi2(p.tp), hi2(p.r)));
+    const F32x2 bv = sub2(p.r, av);
     const F32x2 ta = add2_rd(av, k23), tb = add2_rd(bv, k23);
     const F32x2 ha = sub2(ta, khalf), hb = sub2(tb, khalf);
     const F32x2 fa = sub2(av, ha), fb = sub2(bv, hb);
-    const F32x2 cv = mul2(p.tp, add2(ha, hb));
+    const F32x2 irf = add2(ha, hb);
+    const F32x2 cv = pack2(__fmul_rn(lo2(p.tp), lo2(irf)), __fmul_rn(hi2(p.tp), hi2(irf)));
     const F32x2 tc = add2_rd(cv, k23);
     const F32x2 fc = sub2(cv, sub2(tc, khalf));
     const F32x2 edge = fma2(p.r, both(-kMarginRel), both(0.5f - 2.0f * kMarginRel));
@@ -1056,10 +1077,9 @@ __device__ __forceinline__ void phasor2(const Spot2& p, float s0, float Wz, floa
     const F32x2 db = pack2(fmaf(-Wz, p.h0, Di), fmaf(-Wz, p.h1, Di));
     const F32x2 wr = fma2(db, p.X, mul2(mb, p.Y));
     const F32x2 wi = fma2(nb, p.X, mul2(db, p.Y));
-    const F32x2 rr = mul2(wr, wr), ii = mul2(wi, wi);
-    const F32x2 n = add2(rr, ii);
+    const F32x2 ww = mul2(wr, wr), n = fma2(wi, wi, ww);
     const F32x2 iw = pack2(rcp_approx(lo2(n)), rcp_approx(hi2(n)));
-    c2 = mul2(sub2(rr, ii), iw);
+    c2 = mul2(fma2(mul2(wi, both(-1.0f)), wi, ww), iw);
     s2 = mul2(mul2(wr, wi), mul2(iw, both(-2.0f)));
 }
 
@@ -1068,6 +1088,8 @@ struct Unit {
     F8 B0, B1;
     float4 S0, S1;
     F32x2 c, s;  // cos 2chi, sin 2chi
+    int pix;     // the first sky pixel
+    int bp0, bp1;
     bool in0, in1;
 };
 
@@ -1436,8 +1458,11 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 Unit U;
                 U.in0 = in0;
                 U.in1 = in1;
-                U.B0 = load_beam<Action::kL1>(beam + (in0 ? bp0 : 0));
-                U.B1 = load_beam<Action::kL1>(beam + (in1 ? bp1 : 0));
+                U.pix = pix;
+                U.bp0 = in0 ? bp0 : 0;
+                U.bp1 = in1 ? bp1 : 0;
+                U.B0 = load_beam<Action::kL1>(beam + U.bp0);
+                U.B1 = load_beam<Action::kL1>(beam + U.bp1);
                 act.fetch2(pix, U.S0, U.S1);
                 phasor2(p, F.s0, R1.x, R1.y, U.c, U.s);
                 act.pair2(U);
@@ -1448,6 +1473,8 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
             } else {
             bool fb = false;
             int pix = 0;
+            [[maybe_unused]] int bp = -1;
+            [[maybe_unused]] float cos2 = 0.0f, sin2 = 0.0f;
             if (t < total) {
                 const float4 R0 = *reinterpret_cast<const float4*>(&W[k].dc);
                 const float4 R1 = *reinterpret_cast<const float4*>(&W[k].Wz);
@@ -1500,13 +1527,20 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                         } else if ((unsigned)c.bp < (unsigned)B.npix) {  // 0 <= bp < npix
                             float c2, s2;
                             phasor(p, F.s0, R1.x, R1.y, c2, s2);
-                            act.pair(pix, act.fetch(pix), load_beam(B.beam + c.bp), c.bp, c2, s2);
+                            if constexpr (HasPairAll<Action>::value) {
+                                bp = c.bp;
+                                cos2 = c2;
+                                sin2 = s2;
+                            } else {
+                                act.pair(pix, act.fetch(pix), load_beam(B.beam + c.bp), c.bp, c2, s2);
+                            }
                         } else if constexpr (HasOutside<Action>::value) {
                             act.outside(pix, c.bp);
                         }
                     }
                 }
             }
+            if constexpr (HasPairAll<Action>::value && !kBil) act.pair_all(pix, bp, cos2, sin2);
             queue(fb, pix);
             }
         }
@@ -1572,10 +1606,7 @@ struct Gather {
     {
         const float4* p = sky + pix;
         if (wide) {
-            asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                : "=f"(S0.x), "=f"(S0.y), "=f"(S0.z), "=f"(S0.w), "=f"(S1.x), "=f"(S1.y),
-                  "=f"(S1.z), "=f"(S1.w)
-                : "l"(p));
+            load_sky2(p, S0, S1);
         } else {
             S0 = __ldg(p);
             S1 = __ldg(p + 1);
