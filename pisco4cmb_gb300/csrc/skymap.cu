@@ -62,10 +62,19 @@ namespace {
 
 enum Scratch { kKeys = 0, kKeys2, kPos, kPos2, kRec, kUniq, kCount, kOff, kRuns, kTmp };
 
-// (c, s, d) of one TOD value.
-struct alignas(8) MapRec {
-    double c, s, d;
+// (c, s, d) of one TOD value: a sector of its own, gathered by one 256-bit
+// load.
+struct alignas(32) MapRec {
+    double c, s, d, pad;
 };
+__device__ __forceinline__ MapRec load_rec(const MapRec* p)
+{
+    MapRec r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(r.c), "=d"(r.s), "=d"(r.d), "=d"(r.pad)
+        : "l"(p));
+    return r;
+}
 
 pisco_status map_fail(pisco_map* m, pisco_status s, const std::string& msg)
 {
@@ -98,6 +107,49 @@ pisco_status grow(pisco_map* m, int k, size_t bytes)
     return PISCO_OK;
 }
 
+// ang2pix(pi/2 - dec, ra) for a finite ra and |dec| <= pi/2, with FP32 for all
+// but the longitude's reduction: -1 where a decision lies within the FP32 error
+// of an integer (or |z| of 2/3), and ang2pix itself has to take it.  FP64 is
+// 64 times slower here, and ang2pix is a third of map_keys_kernel's FP64.
+//
+// The error: sin(dec) is good to 1.2e-7, the positions (at most nside in the
+// caps, 3/4 nside from the equator) to nside (0.75 x 1.2e-7 + 2^-24) or, in the
+// caps, nside (3e-7 + 2^-24); the margin is 5e-7 nside + 1e-6.
+__device__ __forceinline__ int quick_ang2pix(int ns, double ra, double dec)
+{
+    const double t = ra * kInvHalfPi;
+    const double tt = fma(-4.0, floor(0.25 * t), t);  // quarter turns, [0, 4]
+    const float m = fmaf((float)ns, 5e-7f, 1e-6f);
+    const float z = sinf((float)dec);
+    auto near = [&](float f) { return f < m || f > 1.0f - m; };
+    if (fabsf(fabsf(z) - 0.6666667f) < 1e-6f) return -1;
+    if (fabsf(z) < 0.6666667f) {
+        const double t1 = (double)ns * (0.5 + tt);
+        const double n1 = floor(t1);
+        const float f1 = (float)(t1 - n1), t2 = 0.75f * (float)ns * z;
+        const float a = f1 - t2, b = f1 + t2;
+        const float fa = floorf(a), fb = floorf(b);
+        if (near(a - fa) || near(b - fb)) return -1;
+        const int jp = (int)n1 + (int)fa, jm = (int)n1 + (int)fb;
+        const int ir = ns + 1 + jp - jm;
+        const int kshift = 1 - (ir & 1);
+        int ip = (jp + jm - ns + kshift + 1 + 8 * ns) >> 1;
+        while (ip >= 4 * ns) ip -= 4 * ns;
+        return 2 * ns * (ns - 1) + (ir - 1) * 4 * ns + ip;
+    }
+    const double q = floor(tt);
+    const float tp = (float)(tt - q);
+    // nside sqrt(3 (1 - |z|)) from the colatitude
+    const float r = (float)ns * 2.4494897f * sinf(0.5f * (float)(kHalfPi - fabs(dec)));
+    const float a = tp * r, b = r - a;
+    const float fa = floorf(a), fb = floorf(b);
+    const int ir = (int)fa + (int)fb + 1;
+    const float c = tp * (float)ir, fc = floorf(c);
+    if (q > 3.0 || near(a - fa) || near(b - fb) || near(c - fc)) return -1;
+    const int ip = (int)q * ir + (int)fc;
+    return z > 0.0f ? 2 * ir * (ir - 1) + ip : 12 * ns * ns - 2 * ir * (ir + 1) + ip;
+}
+
 template <class T>
 __global__ void map_keys_kernel(long long total, long long ns, int nside, const T* ra, const T* dec,
                                 const T* pa, const T* data, const float* pol, int* keys,
@@ -115,14 +167,17 @@ __global__ void map_keys_kernel(long long total, long long ns, int nside, const 
         sincos(twopsi, &s, &c);
         const double theta = PD_SUB(kHalfPi, dc);
         long long p = h.npix;  // sentinel: sorted last, never accumulated
-        if (isfinite(r) && isfinite(theta) && theta >= 0.0 && theta <= kPi) p = ang2pix(h, theta, r);
+        if (isfinite(r) && isfinite(theta) && theta >= 0.0 && theta <= kPi) {
+            p = fabs(r) < 1e4 ? quick_ang2pix(nside, r, dc) : -1;
+            if (p < 0) p = ang2pix(h, theta, r);
+        }
         if (p < 0 || p >= h.npix) {
             atomicOr(bad, 1u);  // non-finite pointing or |dec| > pi/2
             p = h.npix;
         }
         keys[e] = (int)p;
         pos[e] = (int)e;
-        rec[e] = MapRec{c, s, (double)data[e]};
+        rec[e] = MapRec{c, s, (double)data[e], 0.0};
     }
 }
 
@@ -140,8 +195,7 @@ __global__ void map_reduce_kernel(const int* runs, const int* uniq, const int* c
 #pragma unroll
         for (int k = 0; k < kAcc; ++k) t[k] = acc[k * npix + p];
         const int b = off[r], n = count[r];
-        for (int i = b; i < b + n; ++i) {
-            const MapRec v = rec[pos[i]];
+        auto add = [&](const MapRec& v) {
             t[kD] = PD_ADD(t[kD], PD_MUL(1.0, v.d));
             t[kCD] = PD_ADD(t[kCD], PD_MUL(v.c, v.d));
             t[kSD] = PD_ADD(t[kSD], PD_MUL(v.s, v.d));
@@ -151,7 +205,17 @@ __global__ void map_reduce_kernel(const int* runs, const int* uniq, const int* c
             t[kCC] = PD_ADD(t[kCC], PD_MUL(v.c, v.c));
             t[kCS] = PD_ADD(t[kCS], PD_MUL(v.c, v.s));
             t[kSS] = PD_ADD(t[kSS], PD_MUL(v.s, v.s));
+        };
+        // four records in flight, added in order
+        int i = b;
+        for (; i + 4 <= b + n; i += 4) {
+            MapRec v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = load_rec(rec + pos[i + k]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) add(v[k]);
         }
+        for (; i < b + n; ++i) add(load_rec(rec + pos[i]));
 #pragma unroll
         for (int k = 0; k < kAcc; ++k) acc[k * npix + p] = t[k];
     }
