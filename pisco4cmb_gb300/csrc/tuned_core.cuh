@@ -153,8 +153,9 @@ constexpr int kPend = 16;
 
 // A sample whose queued pairs may not all be re-evaluated yet.
 struct alignas(16) Pend {
-    Hpx hb;                  // beam grid
-    double ra, dec, psi;     // FP64 frame (psi = -pa)
+    double ra, dec, psi;     // as given (psi = -pa): the chain's
+    double z0, s0, phi;      // the frame in FP64, as the plan has it
+    double spsi, cpsi;
     double main_a, main_b;   // main-pass totals
     double fb_a, fb_b;       // re-evaluated pairs, summed in queue order
     const F8* beam;
@@ -162,10 +163,11 @@ struct alignas(16) Pend {
     void* out_b;
     long long idx;           // output index
     float ga, gb;            // adjoint weights
-    int npix_beam;
+    int nside_beam, npix_beam;
     int left;                // queued entries not yet re-evaluated
     int open;                // main pass still running
     int f64;                 // output type
+    int plain;               // the frame does not carry the chain's accuracy
 };
 
 // A sample's per-sample geometry: its disc (the rings it touches and the
@@ -175,15 +177,13 @@ struct alignas(16) Pend {
 // it is FP64 work (about three hundred FP64 instructions), which GB300 runs
 // at a small fraction of its FP32 rate.  96 bytes.
 struct alignas(16) SamplePlan {
-    // disc, for disc_ring's exact formula: cos(theta), 1 / sin(theta),
-    // cos(radius) (the beam's, as evaluated on the device), longitude
-    double z0, xa, cosr, phi;
+    // disc, for disc_ring's exact formula: cos(theta), 1 / sin(theta), longitude
+    double z0, xa, phi;
+    double spsi, cpsi;        // sin and cos of psi, negated with the frame's flip
     float phi_hi, phi_lo;     // frame: longitude reduced mod 2 pi, latitude,
     float dec_hi, dec_lo;     //   each the sum of two FP32 values
-    float versr;              // disc: 1 - cos(radius)
     float z0f, s0f;           // frame: sin and |cos| of the latitude
-    float sps, cps;           // sin and cos of psi times a common factor (psi_phasor),
-                              // negated with the frame's flip
+    float sps, cps;           // the same of psi times a common factor (psi_phasor)
     int ring_lo, ring_hi;     // rings on the edge formula
     int full_lo, full_hi;     // rings touched
     int flags;                // kPlanBad: non-finite pointing; kPlanAllSky; kPlanExact
@@ -533,7 +533,8 @@ __device__ __forceinline__ RingPlace place_ring(const SamplePlan& p, const RingT
 // margin is 1e-6 fr (H / sin D + D) + 3e-7 pixels, at least 1.1 times that.  At
 // nside 1024 and 3 degrees it is 6e-5 pixels: two rings in ten thousand take
 // the exact formula.
-__device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePlan& p, int ring,
+__device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePlan& p,
+                                                    double cosr, float versr, int ring,
                                                     const RingT& rt, const RingPlace& g)
 {
     RingRange s = {0, 0};
@@ -543,7 +544,7 @@ __device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePl
         return s;
     }
     const float is = 1.0f / (rt.s * p.s0f);
-    const float x = (p.versr - g.K) * is;  // 1 - cos D
+    const float x = (versr - g.K) * is;  // 1 - cos D
     const float y = sqrtf(x * (2.0f - x));
     const float D = atan2f(y, 1.0f - x);
     const float shift = (rt.npix2 & 1) ? 0.5f : 0.0f;
@@ -552,13 +553,13 @@ __device__ __forceinline__ RingRange fast_disc_ring(const Hpx& h, const SamplePl
     const float vlo = at - w, vhi = at + w;
     const float flo = floorf(vlo), fhi = floorf(vhi);
     // y = 0 or a NaN (an edge outside [0, pi]) makes m infinite or a NaN
-    const float m = fmaf(1e-6f, rt.fr_hi * (p.versr * is / y + D), 3e-7f);
+    const float m = fmaf(1e-6f, rt.fr_hi * (versr * is / y + D), 3e-7f);
     const float rlo = vlo - flo, rhi = vhi - fhi;
     if (!(fminf(rlo, rhi) > m && fmaxf(rlo, rhi) < 1.0f - m) || (p.flags & kPlanExact)) {
         DiscPlan d;
         d.z0 = p.z0;
         d.xa = p.xa;
-        d.cosr = p.cosr;
+        d.cosr = cosr;
         d.phi = p.phi;
         d.ring_lo = p.ring_lo;
         d.ring_hi = p.ring_hi;
@@ -784,6 +785,48 @@ __device__ __forceinline__ bool stencil_f32(const Beam& B, int qd, float tp, flo
     return true;
 }
 
+// The beam pixel and exp(2i chi) of a pair in FP64 without the chain's
+// arccosines and the sines and cosines of its angles: one sine and cosine (of
+// the longitude offset) and one arctangent, some 200 FP64 instructions against
+// 700.  false (nothing computed) where the chain itself has to decide: within
+// 1e-4 rad of the boresight (its own rounding shows there, and its degenerate
+// branch lies at 1e-6), a frame near a pole, or a decision within 1e-9 of an
+// integer.
+__device__ __forceinline__ bool quick_pair(const Hpx& hs, const Hpx& hb, const Pend& P, int pix,
+                                           long long& bp, double& c2, double& s2)
+{
+    if (P.plain) return false;
+    double z, phi, s;
+    bool have;
+    pix2loc(hs, pix, &z, &phi, &s, &have);
+    if (!have) s = sqrt((1.0 - z) * (1.0 + z));
+    double sd, cd;
+    sincos(phi - P.phi, &sd, &cd);
+    const double u = s * sd, v = z * P.s0 - s * P.z0 * cd;
+    const double nb = P.s0 * sd, db = s * P.z0 - z * P.s0 * cd;
+    const double sin2 = fma(u, u, v * v);
+    if (!(sin2 > 1e-8)) return false;
+    // r = nside sqrt(3 (1 - cos rho)), 1 - cos rho = sin^2 rho / (1 + cos rho)
+    const double r = (double)hb.nside * sqrt(3.0 * sin2 / (1.0 + z * P.z0 + s * P.s0 * cd));
+    const double X = u * P.spsi - v * P.cpsi, Y = u * P.cpsi + v * P.spsi;
+    const double t = atan2(Y, X) * kInvHalfPi;  // quarter turns, in [-2, 2]
+    const double tt = t < 0.0 ? t + 4.0 : t;
+    const double qd = floor(tt), tp = tt - qd;
+    const double av = tp * r, bv = r - av;
+    const double fa = floor(av), fb = floor(bv);
+    const double ir = fa + fb + 1.0, cv = tp * ir, fc = floor(cv);
+    const double m = 1e-9 * (r + 2.0);
+    const double ea = av - fa, eb = bv - fb, ec = cv - fc;
+    if (!(fmin(fmin(ea, eb), ec) > m && fmax(fmax(ea, eb), ec) < 1.0 - m)) return false;
+    bp = (long long)(2.0 * ir * (ir - 1.0) + qd * ir + fc);
+    // phasor's w, turned by psi
+    const double wr = fma(db, X, nb * Y), wi = fma(nb, X, -(db * Y));
+    const double rr = wr * wr, iw = 1.0 / fma(wi, wi, rr);
+    c2 = fma(-wi, wi, rr) * iw;
+    s2 = wr * wi * (iw + iw);
+    return true;
+}
+
 // Redoes the first m (<= 32, <= Q.n) queued pairs with the FP64 chain of the
 // PLAIN form, one per lane; credits each to its sample (serially, in queue
 // order, by the first lane of each run of one slot's entries), writes the TOD
@@ -799,29 +842,34 @@ __device__ __forceinline__ void drain(const Hpx& hs, int m, Smem& S, Queue& Q, i
         slot = S.qs[lane];
         const Pend& P = S.p[slot];
         const int pix = S.q[lane];
-        double rho, sig, chi;
-        const long long bp = pair_beam_pixel(hs, P.hb, pix, P.ra, P.dec, P.psi, &rho, &sig, &chi);
+        const Hpx hb = hpx_make(P.nside_beam);
+        double rho = 0.0, sig = 0.0, c2, s2;
+        long long bp = -1;
+        if (kBil || !quick_pair(hs, hb, P, pix, bp, c2, s2)) {
+            double chi;
+            bp = pair_beam_pixel(hs, hb, pix, P.ra, P.dec, P.psi, &rho, &sig, &chi);
+            sincos(2.0 * chi, &s2, &c2);
+        }
         if constexpr (kBil && Action::kStencil) {
             int px[4];
             float w[4];
-            if (stencil_f64(P.hb, P.npix_beam, rho, sig, px, w))
-                act.deferred_stencil(P, pix, px, w, (float)cos(2.0 * chi), (float)sin(2.0 * chi));
+            if (stencil_f64(hb, P.npix_beam, rho, sig, px, w))
+                act.deferred_stencil(P, pix, px, w, (float)c2, (float)s2);
             else if constexpr (HasOutside<Action>::value)
                 act.outside_deferred(P, pix, -1);
         } else if constexpr (kBil) {
             F8 Bv;
-            if (bilinear_f64(P.hb, P.npix_beam, rho, sig, P.beam, Bv))
-                act.deferred(P, pix, Bv, -1, (float)cos(2.0 * chi), (float)sin(2.0 * chi), ta, tb);
+            if (bilinear_f64(hb, P.npix_beam, rho, sig, P.beam, Bv))
+                act.deferred(P, pix, Bv, -1, (float)c2, (float)s2, ta, tb);
             else if constexpr (HasOutside<Action>::value)
                 act.outside_deferred(P, pix, -1);
         } else if (bp < 0) {
             record(err, kCheckBeamIndex);
         } else if (bp < P.npix_beam) {
             if constexpr (IsExact<Action>::value)
-                act.deferred64(pix, (int)bp, cos(2.0 * chi), sin(2.0 * chi), ta, tb);
+                act.deferred64(pix, (int)bp, c2, s2, ta, tb);
             else
-                act.deferred(P, pix, load_beam(P.beam + bp), (int)bp, (float)cos(2.0 * chi),
-                             (float)sin(2.0 * chi), ta, tb);
+                act.deferred(P, pix, load_beam(P.beam + bp), (int)bp, (float)c2, (float)s2, ta, tb);
         } else if constexpr (HasOutside<Action>::value) {
             act.outside_deferred(P, pix, (int)bp);
         }
@@ -1234,16 +1282,16 @@ __device__ __forceinline__ SamplePlan make_plan(const Hpx& hs, const Beam& B, do
     sp.phi_lo = (float)(phi_f - (double)sp.phi_hi);
     sp.dec_hi = (float)dec0;
     sp.dec_lo = (float)(dec0 - (double)sp.dec_hi);
-    sp.versr = B.versr;
     sp.z0f = (float)z0d;
     sp.s0f = (float)s0d;
     double spsi, cpsi;
     sincos(psi, &spsi, &cpsi);
-    psi_phasor(flip ? -spsi : spsi, flip ? -cpsi : cpsi, sp.sps, sp.cps);
+    sp.spsi = flip ? -spsi : spsi;
+    sp.cpsi = flip ? -cpsi : cpsi;
+    psi_phasor(sp.spsi, sp.cpsi, sp.sps, sp.cps);
     sp.z0 = P.z0;
     sp.xa = P.xa;
     sp.phi = P.phi;
-    sp.cosr = B.cosr;
     sp.ring_lo = (int)P.ring_lo;
     sp.ring_hi = (int)P.ring_hi;
     sp.full_lo = (int)P.full_lo;
@@ -1285,10 +1333,17 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
     if (S.p[slot].left > 0) flush<kBil>(hs, S, Qs, lane, err, act);
     if (lane == 0) {
         Pend& Ps = S.p[slot];
-        Ps.hb = hb;
         Ps.ra = ra;
         Ps.dec = dec;
         Ps.psi = -pa;
+        // a latitude near a pole loses digits in 1 / sin(theta)
+        Ps.z0 = SP.z0;
+        Ps.s0 = 1.0 / SP.xa;
+        Ps.phi = SP.phi;
+        Ps.spsi = SP.spsi;
+        Ps.cpsi = SP.cpsi;
+        Ps.plain = (SP.flags & kPlanExact) != 0 || SP.s0f < 0.01f;
+        Ps.nside_beam = (int)hb.nside;
         Ps.fb_a = Ps.fb_b = 0.0;
         Ps.beam = B.beam;
         Ps.out_a = o.a;
@@ -1307,16 +1362,17 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
     if constexpr (Action::kSums) act.reset();
     const SamplePlan& PL = S.plan;
     if constexpr (IsExact<Action>::value) {
-        // the frame in FP64: lanes 0 and 1 take sin and cos of dec and 2 psi in
-        // the same instructions
-        double sn, cs;
-        sincos(lane & 1 ? -2.0 * pa : dec, &sn, &cs);
+        // the frame in FP64; near a pole cos(dec) itself, not 1 / sin(theta)
+        double s0 = 1.0 / PL.xa, z0 = PL.z0;
+        if (PL.s0f < 0.5f || (PL.flags & kPlanExact)) {
+            sincos(dec, &z0, &s0);
+            s0 = fabs(s0);
+        }
         if (lane == 0) {
-            S.z0 = sn;
-            S.s0 = fabs(cs);
-        } else if (lane == 1) {
-            S.c2p = cs;
-            S.s2p = sn;
+            S.z0 = z0;
+            S.s0 = s0;
+            S.c2p = fma(PL.cpsi, PL.cpsi, -(PL.spsi * PL.spsi));
+            S.s2p = 2.0 * PL.spsi * PL.cpsi;
         }
         __syncwarp();
     }
@@ -1354,7 +1410,7 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
         if (ring <= PL.full_hi) {
             const RingT rt = rings[ring - 1];
             const RingPlace g = place_ring(PL, rt);
-            RingRange sp = fast_disc_ring(hs, PL, ring, rt, g);
+            RingRange sp = fast_disc_ring(hs, PL, B.cosr, B.versr, ring, rt, g);
             const int nr = rt.npix2 >> 1;
             // every pixel of the ring's range must lie in the sky map:
             // checked here, once per ring, instead of once per pair
