@@ -456,17 +456,14 @@ __global__ void __launch_bounds__(kAW * 32, adj_warps_per_sm<Act, kBil, kPlanned
     __shared__ tuned::Beam s_B;
     const int lane = threadIdx.x & 31;
     tuned::WarpSmem& S = sm[threadIdx.x >> 5];
-    const Hpx rhs = hpx_make(a.nside_sky);
-    const Hpx rhb = hpx_make(a.nside_beam);
-    const tuned::Beam rB = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
-    if constexpr (kDescSmem) {
-        if (threadIdx.x == 0) {
-            s_hs = rhs;
-            s_hb = rhb;
-            s_B = rB;
-        }
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        s_hs = hpx_make(a.nside_sky);
+        s_hb = hpx_make(a.nside_beam);
+        s_B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
     }
+    __syncthreads();
+    const Hpx rhs = s_hs, rhb = s_hb;
+    const tuned::Beam rB = s_B;
     const Hpx& hs = kDescSmem ? s_hs : rhs;
     const Hpx& hb = kDescSmem ? s_hb : rhb;
     const tuned::Beam& B = kDescSmem ? s_B : rB;
@@ -493,7 +490,7 @@ __global__ void __launch_bounds__(kAW * 32, adj_warps_per_sm<Act, kBil, kPlanned
             tuned::sample<false, kBil>(hs, a.rings, hb, B, a.ra[s], a.dec[s], a.pa[s], none, S, Q,
                                        lane, a.err, act, nfall, cmax, npairs);
     }
-    tuned::flush<kBil>(hs, S, Q, lane, a.err, act);
+    tuned::flush_block<kBil>(hs, sm, kAW, Q, lane, a.err, act);
     if (lane == 0 && nfall && a.fallbacks) atomicAdd(a.fallbacks, nfall);
     if constexpr (HasFinish<Act>::value) act.finish(lane, gw);
 }

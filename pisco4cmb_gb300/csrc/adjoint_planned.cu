@@ -16,8 +16,13 @@ namespace {
 // Positions [0, a.n): plans[i] is the plan of sample a.begin + order(i).
 __global__ void adjoint_plan_kernel(AdjArgs a)
 {
-    const Hpx hs = hpx_make(a.nside_sky);
-    const tuned::Beam B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
+    __shared__ Hpx hs;
+    __shared__ tuned::Beam B;
+    if (threadIdx.x == 0) {
+        hs = hpx_make(a.nside_sky);
+        B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
+    }
+    __syncthreads();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.n;
          i += (long long)gridDim.x * blockDim.x) {
         const long long j = a.order ? (long long)a.order[i] : i;
@@ -32,8 +37,8 @@ cudaError_t launch_adjoint_planned(const AdjArgs& a, int sm_count, cudaStream_t 
 {
     if (nwarps) *nwarps = 0;
     if (a.n <= 0) return cudaSuccess;
-    const long long b = (a.n + 255) / 256;
-    adjoint_plan_kernel<<<(int)(b < 65536 ? b : 65536), 256, 0, st>>>(a);
+    const long long b = (a.n + 127) / 128;
+    adjoint_plan_kernel<<<(int)(b < 65536 ? b : 65536), 128, 0, st>>>(a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return launch_adjoint_impl<true>(a, sm_count, st, nwarps);

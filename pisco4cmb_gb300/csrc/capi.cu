@@ -173,10 +173,6 @@ void pisco_ctx::order_used(cudaStream_t s)
     if (ord_event) cudaEventRecord(ord_event, s);
 }
 
-// Sample plans built by the plan kernel (1) or by each warp (0).
-#ifndef PISCO_FWD_PLANS
-#define PISCO_FWD_PLANS 1
-#endif
 // At most max_plans sample plans (4M: 384 MB of scratch, for the forward's
 // chunks); fewer when maxMemUsage leaves less room (the forward then runs in
 // more chunks), none below kMinPlans.
@@ -665,9 +661,7 @@ pisco_status pisco_forward_device(pisco_ctx* c, pisco_form form, long begin, lon
         }
     } else if (form == PISCO_FORM_TUNED && tuned) {
         CK(cudaMemsetAsync(c->d_fallbacks, 0, sizeof(unsigned long long), s), "reset fallbacks");
-#if PISCO_FWD_PLANS
-        c->plan_scratch(n, s, &plans, &plan_cap);
-#endif
+        if (!tuned_plans_itself(n, c->sm_count)) c->plan_scratch(n, s, &plans, &plan_cap);
         e = launch_forward_tuned(a, c->sm_count, s, plans, plan_cap);
     } else if (exact) {
         c->plan_scratch(n, s, &plans, &plan_cap);

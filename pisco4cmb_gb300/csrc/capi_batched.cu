@@ -253,6 +253,7 @@ pisco_status pisco_forward_batched(pisco_ctx* c, const pisco_det_desc* dets, int
             CK(cudaMemcpyAsync(c->d_items, items.data(), sizeof(BatchItem) * items.size(),
                                cudaMemcpyHostToDevice, c->stream),
                "items H2D");
+        CK(launch_batch_trig(c->d_dets, ndet, c->stream), "batch trig");
         CK(cudaStreamSynchronize(c->stream), "batch upload");
         BatchArgs a;
         a.nside_sky = c->nside_sky;

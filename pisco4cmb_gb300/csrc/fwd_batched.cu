@@ -55,6 +55,13 @@ struct ItemState {
     int state;  // 0: queue empty, 1: run, 2: bad item (skipped)
 };
 
+// The FP64 trig of every detector's beam (BatchDet::cosr, versr).
+__global__ void batch_trig_kernel(BatchDet* dets, int ndet)
+{
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d < ndet) tuned::beam_trig(dets[d].rho_max, dets[d].cosr, dets[d].versr);
+}
+
 // Every detector's sample plans (position p of detector d at
 // plans[plan_base + p]; the bases ascend with d and end at a.nplans), one
 // thread per sample over all detectors at once: the FP64 per-sample geometry
@@ -76,7 +83,7 @@ __global__ void batched_plan_kernel(BatchArgs a)
             tuned::record(a.err, kCheckQueue);
             continue;
         }
-        const tuned::Beam B = tuned::make_beam(det.beam, det.nside_beam, det.npix_beam, det.rho_max);
+        const tuned::Beam B = tuned::det_beam(det);
         const long long s = det.order ? (long long)det.order[p] : p;
         a.plans[g] = tuned::make_plan(hs, B, det.ra[s], det.dec[s], det.pa[s]);
     }
@@ -131,7 +138,7 @@ __global__ void __launch_bounds__(kW * 32, warps_per_sm<kBil, kPlanned, kW>() / 
                 } else {
                     const BatchDet& d = a.dets[it.det];
                     T.hb = hpx_make(d.nside_beam);
-                    T.B = tuned::make_beam(d.beam, d.nside_beam, d.npix_beam, d.rho_max);
+                    T.B = tuned::det_beam(d);
                     T.ra = d.ra;
                     T.dec = d.dec;
                     T.pa = d.pa;
@@ -161,7 +168,7 @@ __global__ void __launch_bounds__(kW * 32, warps_per_sm<kBil, kPlanned, kW>() / 
                                            S, Q, lane, a.err, g, nfall, cmax, npairs);
         }
     }
-    tuned::flush<kBil>(hs, S, Q, lane, a.err, g);
+    tuned::flush_block<kBil>(hs, sm, kBW, Q, lane, a.err, g);
     if (lane == 0 && nfall && a.fallbacks) atomicAdd(a.fallbacks, nfall);
 }
 
@@ -202,6 +209,12 @@ void launch_shape(const BatchArgs& a, int sm_count, cudaStream_t st)
 }
 
 }  // namespace
+
+cudaError_t launch_batch_trig(BatchDet* dets, int ndet, cudaStream_t st)
+{
+    batch_trig_kernel<<<(ndet + 63) / 64, 64, 0, st>>>(dets, ndet);
+    return cudaGetLastError();
+}
 
 bool batched_warps_valid(int warps) { return warps == 4 || warps == 8 || warps == 16; }
 

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kEW * 32, 2)
             tuned::sample<false>(s_hs, a.rings, s_hb, s_B, ra, dec, pa, o, S, Q, lane, a.err, g,
                                  nfall, cmax, npairs);
     }
-    tuned::flush(s_hs, S, Q, lane, a.err, g);
+    tuned::flush_block(s_hs, sm, kEW, Q, lane, a.err, g);
 }
 
 template <bool F64, bool kPlanned>

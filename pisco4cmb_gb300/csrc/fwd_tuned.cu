@@ -30,20 +30,25 @@ namespace {
 #define PISCO_BIL_WARPS 8
 #endif
 
+// Where a launch's sample plans come from: each warp builds its own, an array
+// built beforehand by plan_kernel, or the block's first warp, one plan per lane
+// (a short launch: at most 32 samples per block).
+enum Plans { kOwnPlans, kArrayPlans, kBlockPlans };
+
 // kBil: bilinear beam lookup (the PLAIN form's get_interpol stencil in FP32).
 // kTW: warps per block (fwd_warps_per_sm / kTW blocks per SM).
-// Positions [pos0, pos1) of the launch.  kPlanned: plans holds their sample
-// plans (index position - pos0); otherwise each warp builds its own.
+// Positions [pos0, pos1) of the launch; plans (kArrayPlans): theirs, index
+// position - pos0.
 // Warps per SM: 20 for the planned nearest lookup (register cap 96), 16 for
 // the others (cap 128).
-template <bool kCalib, bool kBil, bool kPlanned>
+template <bool kCalib, bool kBil, Plans kPlans>
 constexpr int fwd_warps_per_sm()
 {
-    return kPlanned && !kBil && !kCalib ? PISCO_FWD_WARPS : 16;
+    return kPlans != kOwnPlans && !kBil && !kCalib ? PISCO_FWD_WARPS : 16;
 }
 
-template <bool kCalib, bool kBil, int kTW, bool kPlanned>
-__global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlanned>() / kTW)
+template <bool kCalib, bool kBil, int kTW, Plans kPlans>
+__global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlans>() / kTW)
     tuned_kernel(FwdArgs a, float* calib, const tuned::SamplePlan* __restrict__ plans,
                  long long pos0, long long pos1)
 {
@@ -58,17 +63,14 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
     constexpr bool kDescSmem = !kBil;
     __shared__ Hpx s_hs, s_hb;
     __shared__ tuned::Beam s_B;
-    const Hpx rhs = hpx_make(a.nside_sky);
-    const Hpx rhb = hpx_make(a.nside_beam);
-    const tuned::Beam rB = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
-    if constexpr (kDescSmem) {
-        if (threadIdx.x == 0) {
-            s_hs = rhs;
-            s_hb = rhb;
-            s_B = rB;
-        }
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        s_hs = hpx_make(a.nside_sky);
+        s_hb = hpx_make(a.nside_beam);
+        s_B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
     }
+    __syncthreads();
+    const Hpx rhs = s_hs, rhb = s_hb;
+    const tuned::Beam rB = s_B;
     const Hpx& hs = kDescSmem ? s_hs : rhs;
     const Hpx& hb = kDescSmem ? s_hb : rhb;
     const tuned::Beam& B = kDescSmem ? s_B : rB;
@@ -80,19 +82,33 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
     g.sky = a.sky32;
     g.wide = (reinterpret_cast<size_t>(a.sky32) & 31) == 0;
     tuned::Queue Q{0, 0};
-    for (long long i = pos0 + gw; i < pos1; i += nw) {
+    __shared__ tuned::SamplePlan s_plans[kPlans == kBlockPlans ? 32 : 1];
+    if constexpr (kPlans == kBlockPlans) {
+        if (threadIdx.x < 32) {
+            // lane l: the plan of warp l % kTW's sample number l / kTW
+            const long long i = pos0 + (long long)blockIdx.x * kTW + lane % kTW + lane / kTW * nw;
+            if (lane < 32 / kTW * kTW && i < pos1) {
+                const long long s = a.begin + (a.order ? (long long)a.order[i] : i);
+                s_plans[lane] = tuned::make_plan(hs, B, a.ra[s], a.dec[s], a.pa[s]);
+            }
+        }
+        __syncthreads();
+    }
+    int mine = threadIdx.x >> 5;  // kBlockPlans: this sample's plan
+    for (long long i = pos0 + gw; i < pos1; i += nw, mine += kTW) {
         const long long j = a.order ? (long long)a.order[i] : i;  // sample of position i
         const long long s = a.begin + j;
         const tuned::Out o{a.out_a, a.out_b, j, a.out_f64};
         const double ra = a.ra[s], dec = a.dec[s], pa = a.pa[s];
-        if constexpr (kPlanned)
-            tuned::sample_planned<kCalib, kBil>(plans[i - pos0], hs, a.rings, hb, B, ra, dec, pa, o,
+        if constexpr (kPlans != kOwnPlans)
+            tuned::sample_planned<kCalib, kBil>(kPlans == kBlockPlans ? s_plans[mine] : plans[i - pos0],
+                                                hs, a.rings, hb, B, ra, dec, pa, o,
                                                 S, Q, lane, a.err, g, nfall, cmax, npairs);
         else
             tuned::sample<kCalib, kBil>(hs, a.rings, hb, B, ra, dec, pa, o, S, Q, lane, a.err, g,
                                         nfall, cmax, npairs);
     }
-    tuned::flush<kBil>(hs, S, Q, lane, a.err, g);
+    tuned::flush_block<kBil>(hs, sm, kTW, Q, lane, a.err, g);
     if (lane == 0 && nfall && a.fallbacks) atomicAdd(a.fallbacks, nfall);
     if (kCalib && calib) {
 #pragma unroll
@@ -108,8 +124,13 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
 __global__ void plan_kernel(FwdArgs a, tuned::SamplePlan* __restrict__ plans, long long pos0,
                             long long pos1)
 {
-    const Hpx hs = hpx_make(a.nside_sky);
-    const tuned::Beam B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
+    __shared__ Hpx hs;
+    __shared__ tuned::Beam B;
+    if (threadIdx.x == 0) {
+        hs = hpx_make(a.nside_sky);
+        B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
+    }
+    __syncthreads();
     for (long long i = pos0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < pos1;
          i += (long long)gridDim.x * blockDim.x) {
         const long long j = a.order ? (long long)a.order[i] : i;
@@ -143,16 +164,23 @@ __global__ void ring_table_kernel(int nside, RingT* rings)
     }
 }
 
+constexpr int kShortWarps = 8, kShortBlocks = 2;  // a short launch's blocks, and theirs per SM
+
 }  // namespace
+
+bool tuned_plans_itself(long long n, int sm_count)
+{
+    return n <= 32LL * kShortBlocks * sm_count;
+}
 
 void launch_plans(const FwdArgs& a, tuned::SamplePlan* plans, long long pos0, long long pos1,
                   cudaStream_t st)
 {
     // small blocks, so that a short launch's plans spread over the SMs: a plan
-    // is a chain of some 300 FP64 instructions, and eight warps on one SM queue
-    // for its FP64 pipe
-    const long long b = (pos1 - pos0 + 63) / 64;
-    plan_kernel<<<(int)(b < 65536 ? b : 65536), 64, 0, st>>>(a, plans, pos0, pos1);
+    // is a chain of some 200 FP64 instructions, and the warps of an SM queue for
+    // its FP64 pipe
+    const long long b = (pos1 - pos0 + 127) / 128;
+    plan_kernel<<<(int)(b < 65536 ? b : 65536), 128, 0, st>>>(a, plans, pos0, pos1);
 }
 
 namespace {
@@ -167,42 +195,43 @@ int resident_blocks(K kernel, int threads)
     return nb;
 }
 
-template <bool kCalib, bool kBil, int kTW, bool kPlanned>
+template <bool kCalib, bool kBil, int kTW, Plans kPlans>
 void launch_shape(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib,
                   tuned::SamplePlan* plans, long long plan_cap)
 {
     const int threads = kTW * 32;
     const long long resident =
-        (long long)sm_count * resident_blocks(tuned_kernel<kCalib, kBil, kTW, kPlanned>, threads);
-    const long long step = kPlanned ? plan_cap : a.n;
+        (long long)sm_count * resident_blocks(tuned_kernel<kCalib, kBil, kTW, kPlans>, threads);
+    const long long step = kPlans == kArrayPlans ? plan_cap : a.n;
     for (long long p0 = 0; p0 < a.n; p0 += step) {
         const long long p1 = p0 + step < a.n ? p0 + step : a.n;
-        if (kPlanned) launch_plans(a, plans, p0, p1, st);
-        const long long need = (p1 - p0 + kTW - 1) / kTW;
-        tuned_kernel<kCalib, kBil, kTW, kPlanned>
-            <<<(int)(resident < need ? resident : need), threads, 0, st>>>(a, calib, plans, p0, p1);
+        if (kPlans == kArrayPlans) launch_plans(a, plans, p0, p1, st);
+        long long blocks = (p1 - p0 + kTW - 1) / kTW;
+        if (kPlans != kBlockPlans && resident < blocks) blocks = resident;
+        // kBlockPlans: every warp's samples have a plan among the block's 32
+        else if (kPlans == kBlockPlans && blocks > kShortBlocks * sm_count) blocks = kShortBlocks * sm_count;
+        tuned_kernel<kCalib, kBil, kTW, kPlans>
+            <<<(int)blocks, threads, 0, st>>>(a, calib, plans, p0, p1);
     }
 }
 
-// kTW: the planned launch's block; without plans the warps build their own
-// (FP64 disc plan in the loop's registers), and that launch keeps 16 warps per
-// SM.  A planned launch of fewer than four samples per resident warp uses
-// blocks of 8 warps (2 per SM), so that its samples spread over every SM
-// (20-warp blocks would fill n / 20 SMs).
+// kTW: the planned launch's block.  A short launch (tuned_plans_itself: at most
+// four samples per warp of two blocks of 8 per SM) uses blocks of 8 warps, so
+// that its samples spread over every SM (20-warp blocks would fill n / 20 SMs),
+// and plans in the block: 2,003 samples spent 11 us of 178 in plan_kernel and
+// 3 between the launches.  Without plans the warps build their own (FP64 disc
+// plan in the loop's registers).
 template <bool kBil, int kTW>
 void launch_lookup(const FwdArgs& a, int sm_count, cudaStream_t st, tuned::SamplePlan* plans,
                    long long plan_cap)
 {
     constexpr int kUnplanned = kTW > 16 ? 16 : kTW;
-    if (plans && plan_cap > 0) {
-        const long long chunk = plan_cap < a.n ? plan_cap : a.n;
-        if (kTW > 8 && chunk < 4LL * sm_count * kTW)
-            launch_shape<false, kBil, (kTW > 8 ? 8 : kTW), true>(a, sm_count, st, nullptr, plans, plan_cap);
-        else
-            launch_shape<false, kBil, kTW, true>(a, sm_count, st, nullptr, plans, plan_cap);
-    } else {
-        launch_shape<false, kBil, kUnplanned, false>(a, sm_count, st, nullptr, nullptr, 0);
-    }
+    if (tuned_plans_itself(a.n, sm_count))
+        launch_shape<false, kBil, kShortWarps, kBlockPlans>(a, sm_count, st, nullptr, nullptr, 0);
+    else if (plans && plan_cap > 0)
+        launch_shape<false, kBil, kTW, kArrayPlans>(a, sm_count, st, nullptr, plans, plan_cap);
+    else
+        launch_shape<false, kBil, kUnplanned, kOwnPlans>(a, sm_count, st, nullptr, nullptr, 0);
 }
 
 cudaError_t launch_tuned_impl(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib,
@@ -210,7 +239,7 @@ cudaError_t launch_tuned_impl(const FwdArgs& a, int sm_count, cudaStream_t st, f
 {
     if (a.n <= 0) return cudaSuccess;
     // calibration measures the nearest-pixel decisions, whatever the lookup
-    if (calib) launch_shape<true, false, 16, false>(a, sm_count, st, calib, nullptr, 0);
+    if (calib) launch_shape<true, false, 16, kOwnPlans>(a, sm_count, st, calib, nullptr, 0);
     else if (a.interp == 1) launch_lookup<true, PISCO_BIL_WARPS>(a, sm_count, st, plans, plan_cap);
     else launch_lookup<false, PISCO_FWD_WARPS>(a, sm_count, st, plans, plan_cap);
     return cudaGetLastError();

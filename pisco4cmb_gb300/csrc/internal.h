@@ -98,6 +98,8 @@ struct BatchDet {
     void* out_b;
     const int* order;  // position -> sample (sky order) or null
     long long plan_base;  // planned launch: its plans start at BatchArgs::plans[plan_base]
+    double cosr;          // cos and 1 - cos of rho_max as evaluated on the device
+    float versr;          //   (launch_batch_trig)
 };
 
 // One unit of the work queue: samples [begin, begin + count) of detector det.
@@ -228,6 +230,8 @@ constexpr size_t kSamplePlanBytes = 96;
 // without it each warp builds its own (the same values either way).
 cudaError_t launch_forward_tuned(const FwdArgs& a, int sm_count, cudaStream_t st,
                                  void* plans = nullptr, long long plan_cap = 0);
+// Does a TUNED launch of n samples take no plan scratch (its blocks plan)?
+bool tuned_plans_itself(long long n, int sm_count);
 bool tuned_supported(int nside_beam, int npix_beam, double rho_max);
 // The sample plans of positions [pos0, pos1) into plans[0 ...) (fwd_tuned.cu).
 void launch_plans(const FwdArgs& a, tuned::SamplePlan* plans, long long pos0, long long pos1,
@@ -252,6 +256,8 @@ cudaError_t launch_ring_table(int nside, RingT* rings, cudaStream_t st);
 // warps: warps per block, 4, 8 or 16 (32 warps per SM for the planned nearest
 // lookup, 16 otherwise, in every shape).
 bool batched_warps_valid(int warps);
+// Fills cosr and versr of the device descriptors.
+cudaError_t launch_batch_trig(BatchDet* dets, int ndet, cudaStream_t st);
 // The persistent grid is the instance's resident blocks on sm_count SMs.
 cudaError_t launch_batched(const BatchArgs& a, int sm_count, cudaStream_t st, int warps = 8);
 // Per-sample disc sizes (pairs) for the roofline byte model.

@@ -198,6 +198,7 @@ extern "C" pisco_status pisco_forward_batched_noalloc(int device, int nside_sky,
     }
     cudaStream_t st = (cudaStream_t)stream;
     noalloc_setup_kernel<<<1, 256, 0, st>>>(p, scratch);
+    launch_batch_trig(scratch->dets, ndet, st);
     cudaError_t e0 = cudaGetLastError();
     if (e0 == cudaSuccess) e0 = launch_ring_table(nside_sky, scratch->rings, st);
     BatchArgs a;

@@ -254,6 +254,15 @@ struct Beam {
     float rscale;  // sqrt(3) * nside
 };
 
+// cos(rho_max) as the disc takes it, and 1 - cos(rho_max): about 100 FP64
+// instructions, formed once per block or per detector.
+__device__ __forceinline__ void beam_trig(double rho_max, double& cosr, float& versr)
+{
+    cosr = rho_max >= kPi ? 0.0 : cos(rho_max);
+    const double half = sin(0.5 * rho_max);
+    versr = (float)(2.0 * half * half);
+}
+
 __device__ __forceinline__ Beam make_beam(const F8* beam, int nside, int npix, double rho_max)
 {
     Beam b;
@@ -261,11 +270,16 @@ __device__ __forceinline__ Beam make_beam(const F8* beam, int nside, int npix, d
     b.nside = nside;
     b.npix = npix;
     b.rho_max = rho_max;
-    b.cosr = rho_max >= kPi ? 0.0 : cos(rho_max);
-    const double half = sin(0.5 * rho_max);
-    b.versr = (float)(2.0 * half * half);
+    beam_trig(rho_max, b.cosr, b.versr);
     b.rscale = (float)(1.7320508075688772 * (double)nside);
     return b;
+}
+
+// The beam of a batched launch's detector (its trig formed beforehand).
+__device__ __forceinline__ Beam det_beam(const BatchDet& d)
+{
+    return Beam{d.beam, d.nside_beam, d.npix_beam, d.rho_max, d.cosr, d.versr,
+                (float)(1.7320508075688772 * (double)d.nside_beam)};
 }
 
 __device__ __forceinline__ void record(unsigned int* err, unsigned int code)
@@ -827,58 +841,55 @@ __device__ __forceinline__ bool quick_pair(const Hpx& hs, const Hpx& hb, const P
     return true;
 }
 
-// Redoes the first m (<= 32, <= Q.n) queued pairs with the FP64 chain of the
-// PLAIN form, one per lane; credits each to its sample (serially, in queue
-// order, by the first lane of each run of one slot's entries), writes the TOD
-// of every sample left with nothing queued, and drops the m entries.  kBil:
-// the beam value is PLAIN's bilinear one instead of the nearest pixel's.
-template <bool kBil = false, class Smem, class Action>
-__device__ __forceinline__ void drain(const Hpx& hs, int m, Smem& S, Queue& Q, int lane,
-                                      unsigned int* err, Action& act)
+// Redoes queued pair e of the warp whose state S is, in FP64: the beam pixel
+// and phasor of quick_pair or of the PLAIN form's chain.  kBil: the beam value
+// is PLAIN's bilinear one instead of the nearest pixel's.
+template <bool kBil, class Smem, class Action, class Real>
+__device__ __forceinline__ void redo(const Hpx& hs, const Smem& S, int e, unsigned int* err,
+                                     Action& act, Real& ta, Real& tb)
 {
-    std::remove_reference_t<decltype(S.ta[0])> ta = 0, tb = 0;
-    int slot = -1;
-    if (lane < m) {
-        slot = S.qs[lane];
-        const Pend& P = S.p[slot];
-        const int pix = S.q[lane];
-        const Hpx hb = hpx_make(P.nside_beam);
-        double rho = 0.0, sig = 0.0, c2, s2;
-        long long bp = -1;
-        if (kBil || !quick_pair(hs, hb, P, pix, bp, c2, s2)) {
-            double chi;
-            bp = pair_beam_pixel(hs, hb, pix, P.ra, P.dec, P.psi, &rho, &sig, &chi);
-            sincos(2.0 * chi, &s2, &c2);
-        }
-        if constexpr (kBil && Action::kStencil) {
-            int px[4];
-            float w[4];
-            if (stencil_f64(hb, P.npix_beam, rho, sig, px, w))
-                act.deferred_stencil(P, pix, px, w, (float)c2, (float)s2);
-            else if constexpr (HasOutside<Action>::value)
-                act.outside_deferred(P, pix, -1);
-        } else if constexpr (kBil) {
-            F8 Bv;
-            if (bilinear_f64(hb, P.npix_beam, rho, sig, P.beam, Bv))
-                act.deferred(P, pix, Bv, -1, (float)c2, (float)s2, ta, tb);
-            else if constexpr (HasOutside<Action>::value)
-                act.outside_deferred(P, pix, -1);
-        } else if (bp < 0) {
-            record(err, kCheckBeamIndex);
-        } else if (bp < P.npix_beam) {
-            if constexpr (IsExact<Action>::value)
-                act.deferred64(pix, (int)bp, c2, s2, ta, tb);
-            else
-                act.deferred(P, pix, load_beam(P.beam + bp), (int)bp, (float)c2, (float)s2, ta, tb);
-        } else if constexpr (HasOutside<Action>::value) {
-            act.outside_deferred(P, pix, (int)bp);
-        }
+    const Pend& P = S.p[S.qs[e]];
+    const int pix = S.q[e];
+    const Hpx hb = hpx_make(P.nside_beam);
+    double rho = 0.0, sig = 0.0, c2, s2;
+    long long bp = -1;
+    if (kBil || !quick_pair(hs, hb, P, pix, bp, c2, s2)) {
+        double chi;
+        bp = pair_beam_pixel(hs, hb, pix, P.ra, P.dec, P.psi, &rho, &sig, &chi);
+        sincos(2.0 * chi, &s2, &c2);
     }
-    if (Action::kSums) {
-        S.ta[lane] = ta;
-        S.tb[lane] = tb;
+    if constexpr (kBil && Action::kStencil) {
+        int px[4];
+        float w[4];
+        if (stencil_f64(hb, P.npix_beam, rho, sig, px, w))
+            act.deferred_stencil(P, pix, px, w, (float)c2, (float)s2);
+        else if constexpr (HasOutside<Action>::value)
+            act.outside_deferred(P, pix, -1);
+    } else if constexpr (kBil) {
+        F8 Bv;
+        if (bilinear_f64(hb, P.npix_beam, rho, sig, P.beam, Bv))
+            act.deferred(P, pix, Bv, -1, (float)c2, (float)s2, ta, tb);
+        else if constexpr (HasOutside<Action>::value)
+            act.outside_deferred(P, pix, -1);
+    } else if (bp < 0) {
+        record(err, kCheckBeamIndex);
+    } else if (bp < P.npix_beam) {
+        if constexpr (IsExact<Action>::value)
+            act.deferred64(pix, (int)bp, c2, s2, ta, tb);
+        else
+            act.deferred(P, pix, load_beam(P.beam + bp), (int)bp, (float)c2, (float)s2, ta, tb);
+    } else if constexpr (HasOutside<Action>::value) {
+        act.outside_deferred(P, pix, (int)bp);
     }
-    __syncwarp();
+}
+
+// Credits the first m redone pairs (S.ta, S.tb) to their samples: serially, in
+// queue order, by the first lane of each run of one slot's entries; writes the
+// TOD of every sample left with nothing queued.
+template <class Action, class Smem>
+__device__ __forceinline__ void credit(Smem& S, int m, int lane)
+{
+    const int slot = lane < m ? S.qs[lane] : -1;
     if (lane < m && (lane == 0 || S.qs[lane - 1] != slot)) {
         Pend& P = S.p[slot];
         int k = lane;
@@ -898,6 +909,22 @@ __device__ __forceinline__ void drain(const Hpx& hs, int m, Smem& S, Queue& Q, i
         P.left -= k - lane;
         if (Action::kSums && P.left == 0 && !P.open) finalize(P);
     }
+}
+
+// Redoes the first m (<= 32, <= Q.n) queued pairs, one per lane, credits them
+// and drops the m entries.
+template <bool kBil = false, class Smem, class Action>
+__device__ __forceinline__ void drain(const Hpx& hs, int m, Smem& S, Queue& Q, int lane,
+                                      unsigned int* err, Action& act)
+{
+    std::remove_reference_t<decltype(S.ta[0])> ta = 0, tb = 0;
+    if (lane < m) redo<kBil>(hs, S, lane, err, act, ta, tb);
+    if (Action::kSums) {
+        S.ta[lane] = ta;
+        S.tb[lane] = tb;
+    }
+    __syncwarp();
+    credit<Action>(S, m, lane);
     // move the rest (<= 32 entries: the queue holds < 64) to the front
     const int rest = Q.n - m;
     int vq = 0, vs = 0;
@@ -922,6 +949,34 @@ __device__ __forceinline__ void flush(const Hpx& hs, Smem& S, Queue& Q, int lane
                                       unsigned int* err, Action& act)
 {
     if (Q.n > 0) drain<kBil>(hs, Q.n, S, Q, lane, err, act);
+}
+
+// The same for all the warps of a block, when they leave the kernel (every
+// thread calls it): their left-over entries are redone together, 32 at a time
+// from whichever warp, instead of a long FP64 chain per warp with a few lanes
+// active -- what a launch of a few samples per warp spends a tenth of its time
+// on.  sm: the block's states; warps: their number.
+template <bool kBil = false, class Smem, class Action>
+__device__ __forceinline__ void flush_block(const Hpx& hs, Smem* sm, int warps, Queue& Q, int lane,
+                                            unsigned int* err, Action& act)
+{
+    __shared__ int counts[32];
+    const int warp = threadIdx.x >> 5;
+    if (lane == 0) counts[warp] = Q.n;
+    __syncthreads();
+    int e = threadIdx.x, w = 0;
+    while (w < warps && e >= counts[w]) e -= counts[w++];
+    if (w < warps) {
+        std::remove_reference_t<decltype(sm->ta[0])> ta = 0, tb = 0;
+        redo<kBil>(hs, sm[w], e, err, act, ta, tb);
+        if (Action::kSums) {
+            sm[w].ta[e] = ta;
+            sm[w].tb[e] = tb;
+        }
+    }
+    __syncthreads();
+    credit<Action>(sm[warp], Q.n, lane);
+    Q.n = 0;
 }
 
 // The same for |x| <= kShortOffset, two terms fewer each (truncation below
