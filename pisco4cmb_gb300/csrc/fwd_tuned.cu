@@ -155,9 +155,16 @@ __global__ void ring_table_kernel(int nside, RingT* rings)
         t.dec_lo = (float)(dec - (double)t.dec_hi);
         t.fr_hi = (float)fr;
         t.fr_lo = (float)(fr - (double)t.fr_hi);
+        // near a pole sin(theta) from i^2 / (3 nside^2): 1 - z has lost digits
+        const double i = (double)(r <= 2 * h.nside ? r : 4 * h.nside - r), t2 = i * i * h.fact2;
+        const double sx = i < (double)h.nside ? sqrt(t2 * (2.0 - t2)) : s;
+        const double dphi = PD_DIV(kTwoPi, (double)ri.npix);
         t.s = (float)s;
-        t.dphi = (float)PD_DIV(kTwoPi, (double)ri.npix);
+        t.s_lo = (float)(sx - (double)t.s);
+        t.dphi = (float)dphi;
+        t.dphi_lo = (float)(dphi - (double)t.dphi);
         t.z = (float)z;
+        t.z_lo = (float)(z - (double)t.z);
         t.start = (int)ri.start;
         t.npix2 = (int)(2 * ri.npix + (ri.shifted ? 1 : 0));
         rings[r - 1] = t;

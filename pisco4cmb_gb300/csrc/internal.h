@@ -38,12 +38,11 @@ struct alignas(64) D8 {
 struct alignas(16) RingT {
     float dec_hi, dec_lo;  // latitude atan2(z, sqrt((1 - z)(1 + z)))
     float fr_hi, fr_lo;    // npix / (2 pi)
-    float s;               // sqrt(1 - z^2)
-    float dphi;            // 2 pi / npix
-    float z;
+    float s, s_lo;         // sqrt(1 - z^2)
+    float dphi, dphi_lo;   // 2 pi / npix
+    float z, z_lo;
     int start;             // first pixel
     int npix2;             // 2 npix + (1 if the ring is shifted by half a pixel)
-    int pad[3];
 };
 constexpr int kMaxRings = 4 * 8192 - 1;
 

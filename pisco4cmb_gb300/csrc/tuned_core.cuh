@@ -101,6 +101,12 @@ template <class A, class = void>
 struct IsExact : std::false_type {};
 template <class A>
 struct IsExact<A, std::void_t<decltype(&A::pair64)>> : std::true_type {};
+// ... in two-float arithmetic (the PLAIN form, whose products take it rounded
+// to FP32)?
+template <class A, class = void>
+struct IsTwoFloat : std::false_type {};
+template <class A>
+struct IsTwoFloat<A, std::void_t<decltype(&A::kTwoFloat)>> : std::true_type {};
 // Does the action take the pairs of a warp together (every lane calls
 // pair_all, with beam pixel -1 where it has no pair)?
 template <class A, class = void>
@@ -216,6 +222,58 @@ struct ExactSmem : WarpState<double> {
     RingD rd[32];
     double z0, s0, c2p, s2p;  // sin and |cos| of the latitude, cos and sin of 2 psi
 };
+
+// A value as the unevaluated sum of two FP32 values, h the sum rounded (2^-48
+// relative), by Dekker's and Knuth's exact sums and products (T. J. Dekker,
+// Numer. Math. 18, 224 (1971)).  A product takes 7 FP32 instructions, a sum 8
+// to 11, where one FP64 instruction takes as long as 64 FP32 ones.
+struct FF {
+    float h, l;
+};
+__device__ __forceinline__ FF ff(double d)
+{
+    const float h = (float)d;
+    return FF{h, (float)(d - (double)h)};
+}
+__device__ __forceinline__ FF ff_quick(float a, float b)  // a + b, |a| >= |b|
+{
+    const float h = __fadd_rn(a, b);
+    return FF{h, __fsub_rn(b, __fsub_rn(h, a))};
+}
+__device__ __forceinline__ FF ff_sum(float a, float b)  // a + b, exactly
+{
+    const float h = __fadd_rn(a, b), t = __fsub_rn(h, a);
+    return FF{h, __fadd_rn(__fsub_rn(a, __fsub_rn(h, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ FF operator+(FF a, FF b)
+{
+    const FF s = ff_sum(a.h, b.h), t = ff_sum(a.l, b.l);
+    const FF u = ff_quick(s.h, __fadd_rn(s.l, t.h));
+    return ff_quick(u.h, __fadd_rn(u.l, t.l));
+}
+__device__ __forceinline__ FF operator-(FF a) { return FF{-a.h, -a.l}; }
+__device__ __forceinline__ FF operator-(FF a, FF b) { return a + (-b); }
+__device__ __forceinline__ FF operator*(FF a, FF b)
+{
+    const float p = __fmul_rn(a.h, b.h);
+    return ff_quick(p, fmaf(a.h, b.l, fmaf(a.l, b.h, fmaf(a.h, b.h, -p))));
+}
+__device__ __forceinline__ FF operator*(float a, FF b)
+{
+    const float p = __fmul_rn(a, b.h);
+    return ff_quick(p, fmaf(a, b.l, fmaf(a, b.h, -p)));
+}
+
+// The same of a PLAIN sample: ring constants and frame.
+struct RingF {
+    FF dc, dphi, s, Zs, Wz, Di;
+};
+struct PlainSmem : WarpState<double> {
+    RingF rd[32];
+    FF z0, s0, c2p, s2p;
+};
+__device__ __forceinline__ void put(double& x, double v) { x = v; }
+__device__ __forceinline__ void put(FF& x, double v) { x = ff(v); }
 
 // Warp-uniform queue state, in registers.
 struct Queue {
@@ -1257,6 +1315,62 @@ __device__ __forceinline__ void phasor_exact(const RingD& R, double kf, bool nar
     s2 = fma(ei, c2p, er * s2p);
 }
 
+// ring_exact and phasor_exact in two-float arithmetic.  The anchor's offset is
+// near - f - e pixels (RingPlace).
+__device__ __forceinline__ RingF ring_two_float(float near, float f, float e, const RingT& rt,
+                                                FF z0, FF s0)
+{
+    RingF r;
+    r.dphi = FF{rt.dphi, rt.dphi_lo};
+    r.dc = (ff_sum(near, -f) + FF{-e, 0.0f}) * r.dphi;
+    r.s = FF{rt.s, rt.s_lo};
+    const FF z = FF{rt.z, rt.z_lo};
+    r.Zs = r.s * z0;
+    r.Wz = s0 * z;
+    r.Di = z * s0 - r.Zs;
+    return r;
+}
+
+// exp(2i chi) rounded to FP32: its error before that rounding, some 1e-12 at
+// rho of a degree, is far below what moves the rounded value.  About 260 FP32
+// instructions, the time of four FP64 ones; the 45 FP64 instructions of
+// phasor_exact took two thirds of a PLAIN launch.  narrow: |x| <= 1/2, where the
+// series' FP32 terms leave 2e-10 of sin x (8e-12 at 1/8).
+__device__ __forceinline__ void phasor_two_float(const RingF& R, float kf, bool narrow, FF s0,
+                                                 FF c2p, FF s2p, float& c2, float& s2)
+{
+    const FF x = kf * R.dphi + R.dc;
+    FF sn, h;
+    if (narrow) {
+        const FF x2 = x * x;
+        // sin x = x + x (x2 (-1/6 + x2 p)), 1 - cos x = x2 (1/2 + x2 (-1/24 + x2 q))
+        const float p = fmaf(x2.h, fmaf(x2.h, fmaf(x2.h, -2.50521084e-8f, 2.75573192e-6f),
+                                        -1.98412698e-4f), 8.33333333e-3f);
+        const float q = fmaf(x2.h, fmaf(x2.h, fmaf(x2.h, -2.08767570e-9f, 2.75573192e-7f),
+                                        -2.48015873e-5f), 1.38888889e-3f);
+        const FF a = ff_quick(-0.16666667f, fmaf(x2.h, p, 4.9670537e-9f));
+        const FF b = ff_quick(-0.041666668f, fmaf(x2.h, q, 1.2417634e-9f));
+        sn = x + x * (x2 * a);
+        h = x2 * (FF{0.5f, 0.0f} + x2 * b);
+    } else {
+        double s, c;
+        sincos((double)x.h + (double)x.l, &s, &c);
+        sn = ff(s);
+        h = ff(c > 0.0 ? s * s / (1.0 + c) : 1.0 - c);
+    }
+    const FF u = R.s * sn, v = R.Zs * h + R.Di;
+    const FF nb = s0 * sn, db = R.Wz * h - R.Di;
+    const FF wr = db * v - nb * u, wi = db * u + nb * v;
+    const FF rr = wr * wr, ii = wi * wi, n = rr + ii;
+    // 1 / n: the reciprocal approximation and one Newton step
+    const float y = rcp_approx(n.h);
+    const float e = fmaf(-n.l, y, fmaf(-n.h, y, 1.0f));
+    const FF iw = ff_quick(y, fmaf(e, e * y, e * y));
+    const FF er = (rr - ii) * iw, ei = 2.0f * (wr * wi * iw);
+    c2 = (er * c2p - ei * s2p).h;
+    s2 = (ei * c2p + er * s2p).h;
+}
+
 // 1 << x, 0 for x outside [0, 32).
 __device__ __forceinline__ unsigned bit_or_0(int x)
 {
@@ -1418,16 +1532,16 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
     const SamplePlan& PL = S.plan;
     if constexpr (IsExact<Action>::value) {
         // the frame in FP64; near a pole cos(dec) itself, not 1 / sin(theta)
-        double s0 = 1.0 / PL.xa, z0 = PL.z0;
+        double s0 = S.p[slot].s0, z0 = PL.z0;
         if (PL.s0f < 0.5f || (PL.flags & kPlanExact)) {
             sincos(dec, &z0, &s0);
             s0 = fabs(s0);
         }
         if (lane == 0) {
-            S.z0 = z0;
-            S.s0 = s0;
-            S.c2p = fma(PL.cpsi, PL.cpsi, -(PL.spsi * PL.spsi));
-            S.s2p = 2.0 * PL.spsi * PL.cpsi;
+            put(S.z0, z0);
+            put(S.s0, s0);
+            put(S.c2p, fma(PL.cpsi, PL.cpsi, -(PL.spsi * PL.spsi)));
+            put(S.s2p, 2.0 * PL.spsi * PL.cpsi);
         }
         __syncwarp();
     }
@@ -1461,7 +1575,7 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
         int cnt = 0, items = 0;  // the ring's disc pixels; its lane slots
         bool wide = false;
         RingC rc;
-        [[maybe_unused]] RingD rd;
+        [[maybe_unused]] std::conditional_t<IsTwoFloat<Action>::value, RingF, RingD> rd;
         if (ring <= PL.full_hi) {
             const RingT rt = rings[ring - 1];
             const RingPlace g = place_ring(PL, rt);
@@ -1500,7 +1614,9 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 if (mid >= (nr >> 1) + 1) kk -= nr;
                 else if (mid < -(nr >> 1)) kk += nr;
                 rc.kc = 0x4B400000 + kk - sp.lo;
-                if constexpr (IsExact<Action>::value)
+                if constexpr (IsTwoFloat<Action>::value)
+                    rd = ring_two_float(near + sh, g.f, g.e, rt, S.z0, S.s0);
+                else if constexpr (IsExact<Action>::value)
                     rd = ring_exact(hs, ring, jc, rt, PL, S.z0, S.s0);
                 const int hi = sp.lo + cnt - 1;  // below 2^16: rings hold at most 2^15 pixels
                 rc.ends = sp.lo | hi << 16;
@@ -1509,8 +1625,10 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 // pixel are multiples of 4)
                 rc.j0 = kUnits ? sp.lo & ~1 : sp.lo;
                 items = kUnits ? (hi >> 1) - (sp.lo >> 1) + 1 : cnt;
-                const int far = max(-kk, kk + cnt);
-                wide = (float)far * rt.dphi > kShortOffset - rt.dphi;
+                // (the anchor is within half a pixel of the boresight's longitude)
+                const float far = ((float)max(-kk, kk + cnt - 1) + 0.5f) * rt.dphi;
+                wide = far > kShortOffset;
+                if constexpr (IsTwoFloat<Action>::value) wide = far > 0.5f;
             }
         }
         int incl = items;
@@ -1631,9 +1749,15 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                     if (!fb) {
                         if constexpr (IsExact<Action>::value) {
                             if ((unsigned)c.bp < (unsigned)B.npix) {
-                                double c2, s2;
-                                phasor_exact(S.rd[k], (double)kf, narrow, S.s0, S.c2p, S.s2p, c2, s2);
-                                act.pair64(pix, c.bp, c2, s2);
+                                if constexpr (IsTwoFloat<Action>::value) {
+                                    float c2, s2;
+                                    phasor_two_float(S.rd[k], kf, narrow, S.s0, S.c2p, S.s2p, c2, s2);
+                                    act.pair64(pix, c.bp, c2, s2);
+                                } else {
+                                    double c2, s2;
+                                    phasor_exact(S.rd[k], (double)kf, narrow, S.s0, S.c2p, S.s2p, c2, s2);
+                                    act.pair64(pix, c.bp, c2, s2);
+                                }
                             }
                         } else if ((unsigned)c.bp < (unsigned)B.npix) {  // 0 <= bp < npix
                             float c2, s2;
