@@ -9,13 +9,14 @@
 // at least 3 hits (skymap.cpp:134-231).
 //
 // GB300 layout of the work.  Per call: one thread per TOD value computes its
-// pixel (the FP64 HEALPix ang2pix of hpx.cuh) and (c, s, d) in FP64; a stable
-// radix sort by pixel (CUB) groups the values of a pixel while keeping them
+// pixel (in FP32 and two-float arithmetic, with the FP64 HEALPix ang2pix of
+// hpx.cuh for values near a pixel's edge: the same pixels) and (c, s, d) in
+// FP64 (a table of sin and cos with a short series); a stable radix sort by pixel (CUB) groups the values of a pixel while keeping them
 // in the reference's (detector, sample) order; one thread per occupied pixel
 // then adds them sequentially, in FP64 without contraction, onto the
 // pixel's running totals.  Each total therefore receives exactly the
 // reference's additions in the reference's order (bit-identical up to the
-// last-ulp differences of CUDA's and the host's cos/sin), with no atomics
+// last-ulp differences of the device's and the host's cos/sin), with no atomics
 // and run-to-run determinism.  The solve restates the reference LAPACK
 // dgesv (dgetf2 + dgetrs) per pixel in non-contracted FP64.
 //
@@ -107,69 +108,123 @@ pisco_status grow(pisco_map* m, int k, size_t bytes)
     return PISCO_OK;
 }
 
-// ang2pix(pi/2 - dec, ra) for a finite ra and |dec| <= pi/2, with FP32 for all
-// but the longitude's reduction: -1 where a decision lies within the FP32 error
-// of an integer (or |z| of 2/3), and ang2pix itself has to take it.  FP64 is
-// 64 times slower here, and ang2pix is a third of map_keys_kernel's FP64.
+// x as the sum of two FP32 values.
+__device__ __forceinline__ void split(float x, float& h, float& l)
+{
+    h = x;
+    l = 0.0f;
+}
+__device__ __forceinline__ void split(double x, float& h, float& l)
+{
+    h = (float)x;
+    l = (float)(x - (double)h);
+}
+
+// ang2pix(pi/2 - dec, ra) for |ra| < 1e4 and |dec| <= pi/2 in FP32 (the
+// longitude in two-float arithmetic): -1 where a decision lies within the FP32
+// error of an integer (or |z| of 2/3), and ang2pix itself has to take it.  FP64
+// is 64 times slower here.
 //
 // The error: sin(dec) is good to 1.2e-7, the positions (at most nside in the
 // caps, 3/4 nside from the equator) to nside (0.75 x 1.2e-7 + 2^-24) or, in the
 // caps, nside (3e-7 + 2^-24); the margin is 5e-7 nside + 1e-6.
-__device__ __forceinline__ int quick_ang2pix(int ns, double ra, double dec)
+template <class T>
+__device__ __forceinline__ int quick_ang2pix(int ns, T ra, T dec)
 {
-    const double t = ra * kInvHalfPi;
-    const double tt = fma(-4.0, floor(0.25 * t), t);  // quarter turns, [0, 4]
-    const float m = fmaf((float)ns, 5e-7f, 1e-6f);
-    const float z = sinf((float)dec);
+    float rh, rl, dh, dl;
+    split(ra, rh, rl);
+    split(dec, dh, dl);
+    // quarter turns mod 4, tt + tl: ra 2 / pi with the product's rounding error
+    const float th = __fmul_rn(rh, 0.63661975f);
+    const float tl = fmaf(rl, 0.63661975f, fmaf(rh, 2.5682e-8f, fmaf(rh, 0.63661975f, -th)));
+    const float tt = fmaf(-4.0f, floorf(0.25f * th), th);
+    const float n = (float)ns, m = fmaf(n, 5e-7f, 1e-6f);
+    const float z = sinf(dh);
     auto near = [&](float f) { return f < m || f > 1.0f - m; };
     if (fabsf(fabsf(z) - 0.6666667f) < 1e-6f) return -1;
     if (fabsf(z) < 0.6666667f) {
-        const double t1 = (double)ns * (0.5 + tt);
-        const double n1 = floor(t1);
-        const float f1 = (float)(t1 - n1), t2 = 0.75f * (float)ns * z;
+        // nside (1/2 + turns) = n1 + f1, and 3/4 nside z
+        const float p = __fmul_rn(n, tt), n1 = floorf(p), half = 0.5f * n, h1 = floorf(half);
+        const float f1 = __fsub_rn(p, n1) + (fmaf(n, tl, fmaf(n, tt, -p)) + (half - h1));
+        const float t2 = 0.75f * n * z;
         const float a = f1 - t2, b = f1 + t2;
         const float fa = floorf(a), fb = floorf(b);
         if (near(a - fa) || near(b - fb)) return -1;
-        const int jp = (int)n1 + (int)fa, jm = (int)n1 + (int)fb;
+        const int base = (int)n1 + (int)h1;
+        const int jp = base + (int)fa, jm = base + (int)fb;
         const int ir = ns + 1 + jp - jm;
         const int kshift = 1 - (ir & 1);
         int ip = (jp + jm - ns + kshift + 1 + 8 * ns) >> 1;
         while (ip >= 4 * ns) ip -= 4 * ns;
         return 2 * ns * (ns - 1) + (ir - 1) * 4 * ns + ip;
     }
-    const double q = floor(tt);
-    const float tp = (float)(tt - q);
-    // nside sqrt(3 (1 - |z|)) from the colatitude
-    const float r = (float)ns * 2.4494897f * sinf(0.5f * (float)(kHalfPi - fabs(dec)));
+    const float q = floorf(tt), tp = (tt - q) + tl;
+    if (!(tp > 0.0f && tp < 1.0f)) return -1;
+    // nside sqrt(3 (1 - |z|)) from the colatitude, pi/2 as a pair
+    const float colat = (1.5707964f - fabsf(dh)) + (dh < 0.0f ? dl : -dl) - 4.3711388e-8f;
+    const float r = n * 2.4494897f * sinf(0.5f * colat);
     const float a = tp * r, b = r - a;
     const float fa = floorf(a), fb = floorf(b);
     const int ir = (int)fa + (int)fb + 1;
     const float c = tp * (float)ir, fc = floorf(c);
-    if (q > 3.0 || near(a - fa) || near(b - fb) || near(c - fc)) return -1;
+    if (q > 3.0f || near(a - fa) || near(b - fb) || near(c - fc)) return -1;
     const int ip = (int)q * ir + (int)fc;
     return z > 0.0f ? 2 * ir * (ir - 1) + ip : 12 * ns * ns - 2 * ir * (ir + 1) + ip;
 }
 
+// sin and cos of x to about an ulp in 17 FP64 instructions (CUDA's takes some
+// 45): the nearest multiple k of pi/64 from a table (tab: cos and sin), the
+// rest, at most 0.0246, by the Taylor series (truncated below 4e-18).
+__device__ __forceinline__ void sincos_table(double x, const double2* tab, double* s, double* c)
+{
+    if (!(fabs(x) < 1e5)) {
+        sincos(x, s, c);
+        return;
+    }
+    const double t = fma(x, 20.371832715762604, 6755399441055744.0);  // + 1.5 2^52: rounds
+    const double k = t - 6755399441055744.0;
+    const double2 v = tab[__double2loint(t) & 127];
+    // pi/64 as the sum of two doubles
+    const double r = fma(-k, 1.9135106236677394e-18, fma(-k, 0.04908738521234052, x));
+    const double r2 = r * r;
+    const double sr = fma(r * r2, fma(r2, fma(r2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), r);
+    const double cr = r2 * fma(r2, fma(r2, -1.0 / 720.0, 1.0 / 24.0), -0.5);  // cos r - 1
+    *s = fma(v.x, sr, fma(v.y, cr, v.y));
+    *c = fma(-v.y, sr, fma(v.x, cr, v.x));
+}
+
+constexpr int kKeyThreads = 256;
+
 template <class T>
-__global__ void map_keys_kernel(long long total, long long ns, int nside, const T* ra, const T* dec,
+__global__ void __launch_bounds__(kKeyThreads) map_keys_kernel(long long total, long long ns, int nside, const T* ra, const T* dec,
                                 const T* pa, const T* data, const float* pol, int* keys,
                                 int* pos, MapRec* rec, unsigned int* bad)
 {
-    const Hpx h = hpx_make(nside);
+    __shared__ Hpx h;
+    __shared__ double2 tab[128];
+    if (threadIdx.x < 128) {
+        double s, c;
+        sincospi((double)threadIdx.x / 64.0, &s, &c);
+        tab[threadIdx.x] = make_double2(c, s);
+    } else if (threadIdx.x == 128) {
+        h = hpx_make(nside);
+    }
+    __syncthreads();
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
-        const int det = (int)(e / ns);
+        const int det = (int)((unsigned)e / (unsigned)ns);  // total < 2^31
         const double r = (double)ra[e], dc = (double)dec[e];
         // the reference's arithmetic (skymap.cpp:85-101), FP64, no contraction
         const double psi = -PD_ADD((double)pol[det], (double)pa[e]);
         const double twopsi = PD_MUL(2.0, psi);
         double s, c;
-        sincos(twopsi, &s, &c);
-        const double theta = PD_SUB(kHalfPi, dc);
-        long long p = h.npix;  // sentinel: sorted last, never accumulated
-        if (isfinite(r) && isfinite(theta) && theta >= 0.0 && theta <= kPi) {
-            p = fabs(r) < 1e4 ? quick_ang2pix(nside, r, dc) : -1;
-            if (p < 0) p = ang2pix(h, theta, r);
+        sincos_table(twopsi, tab, &s, &c);
+        long long p = -1;
+        if (fabs(dc) <= kHalfPi && fabs((float)ra[e]) < 1e4f) p = quick_ang2pix(nside, ra[e], dec[e]);
+        if (p < 0) {
+            const double theta = PD_SUB(kHalfPi, dc);
+            p = h.npix;  // sentinel: sorted last, never accumulated
+            if (isfinite(r) && isfinite(theta) && theta >= 0.0 && theta <= kPi) p = ang2pix(h, theta, r);
         }
         if (p < 0 || p >= h.npix) {
             atomicOr(bad, 1u);  // non-finite pointing or |dec| > pi/2
@@ -196,10 +251,9 @@ __global__ void map_reduce_kernel(const int* runs, const int* uniq, const int* c
         for (int k = 0; k < kAcc; ++k) t[k] = acc[k * npix + p];
         const int b = off[r], n = count[r];
         auto add = [&](const MapRec& v) {
-            t[kD] = PD_ADD(t[kD], PD_MUL(1.0, v.d));
+            t[kD] = PD_ADD(t[kD], v.d);
             t[kCD] = PD_ADD(t[kCD], PD_MUL(v.c, v.d));
             t[kSD] = PD_ADD(t[kSD], PD_MUL(v.s, v.d));
-            t[kN] = PD_ADD(t[kN], 1.0);
             t[kC] = PD_ADD(t[kC], v.c);
             t[kS] = PD_ADD(t[kS], v.s);
             t[kCC] = PD_ADD(t[kCC], PD_MUL(v.c, v.c));
@@ -216,6 +270,7 @@ __global__ void map_reduce_kernel(const int* runs, const int* uniq, const int* c
             for (int k = 0; k < 4; ++k) add(v[k]);
         }
         for (; i < b + n; ++i) add(load_rec(rec + pos[i]));
+        t[kN] = PD_ADD(t[kN], (double)n);  // n ones added one by one: exact as well
 #pragma unroll
         for (int k = 0; k < kAcc; ++k) acc[k * npix + p] = t[k];
     }
@@ -360,9 +415,10 @@ pisco_status accumulate(pisco_map* m, long long ns, int ndet, const T* ra, const
     void* tmp = m->buf[kTmp];
     MCK(cudaMemcpyAsync(pol, h_pol, sizeof(float) * ndet, cudaMemcpyHostToDevice, st), "pol H2D");
     MCK(cudaMemsetAsync(bad, 0, sizeof(unsigned int), st), "reset check");
+    // a persistent grid: a block's table takes as long as some of its values
     const long long blocks = std::min<long long>((total + 255) / 256, 8192);
-    map_keys_kernel<T><<<(int)blocks, 256, 0, st>>>(total, ns, m->nside, ra, dec, pa, data, pol,
-                                                   keys, pos, rec, bad);
+    map_keys_kernel<T><<<(int)std::min<long long>(blocks, 1216), kKeyThreads, 0, st>>>(
+        total, ns, m->nside, ra, dec, pa, data, pol, keys, pos, rec, bad);
     MCK(cudaGetLastError(), "map keys");
     size_t tb = m->cap[kTmp];
     MCK(cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys2, pos, pos2, n, 0, bits, st), "sort");
