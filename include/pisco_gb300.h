@@ -39,8 +39,9 @@ typedef enum pisco_status {
 
 typedef enum pisco_dtype { PISCO_FLOAT32 = 0, PISCO_FLOAT64 = 1 } pisco_dtype;
 
-/* PLAIN: the reference's per-pair chain on the GPU (FP64 geometry, FP32
- *        sky x beam products, FP64 accumulation).
+/* PLAIN: the reference's per-pair chain on the GPU (its FP64 pixel decisions
+ *        and chi rounded to FP32, FP32 sky x beam products, FP64
+ *        accumulation).
  * TUNED: FP64 per-sample frame, FP32 per-pair geometry with an FP64
  *        re-evaluation of every decision that lies near a pixel edge, FP32
  *        products with compensated (two-sum) accumulation.  With the
@@ -143,11 +144,13 @@ pisco_status pisco_forward_device(pisco_ctx* ctx, pisco_form form, long begin, l
 pisco_status pisco_sync(pisco_ctx* ctx);
 /* Device bytes the context holds, the figure RunConfig.maxMemUsage bounds
  * (the reference checks its fixed buffers against it once,
- * gpuconvolver.cu:58-70; here every buffer counts as it grows).  The TUNED
- * forward keeps up to 4M sample plans of 96 bytes as scratch: fewer (the
- * forward runs in chunks) when maxMemUsage leaves less room, none when it
- * leaves room for fewer than 1024 (each warp then plans its own samples);
- * the TOD is the same bit for bit in every case. */
+ * gpuconvolver.cu:58-70; here every buffer counts as it grows).  A forward
+ * (TUNED, and PLAIN or FP64 with the nearest lookup) keeps up to 4M sample
+ * plans of 96 bytes as scratch: fewer (the forward runs in chunks) when
+ * maxMemUsage leaves less room, none when it leaves room for fewer than 1024
+ * (each warp then plans its own samples) and none for a TUNED range of at most
+ * 64 samples per SM (each block plans its own); the TOD is the same bit for
+ * bit in every case. */
 pisco_status pisco_memory_used(const pisco_ctx* ctx, size_t* bytes);
 
 /* ---- statistics of the last forward (for the roofline) ---------------- */
@@ -189,8 +192,9 @@ typedef struct pisco_pair_dump {
 #define PISCO_PAIR_REDONE 1       /* TUNED: re-evaluated with the FP64 chain */
 #define PISCO_PAIR_OUTSIDE_BEAM 2 /* beam pixel (every stencil pixel) beyond the
                                      stored map: the pair adds nothing */
-/* Runs the per-sample body of `form` (with the context's beam lookup) over
- * samples [begin, begin+n) of the current scan and records every (sample,
+/* Runs the per-sample body of `form` (with the context's beam lookup; PLAIN
+ * and FP64: the reference's chain) over samples [begin, begin+n) of the
+ * current scan and records every (sample,
  * disc pixel) pair it visits: each sample's pairs appear together, in no
  * particular order within the sample.  *npairs = the number of disc pairs of
  * the range (HEALPix query_disc).  out == NULL only sizes the record;

@@ -462,9 +462,9 @@ __global__ void __launch_bounds__(kAW * 32, adj_warps_per_sm<Act, kBil, kPlanned
         s_B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
     }
     __syncthreads();
-    const Hpx rhs = s_hs, rhb = s_hb;
-    const tuned::Beam rB = s_B;
-    const Hpx& hs = kDescSmem ? s_hs : rhs;
+    const Hpx rhb = hpx_make(a.nside_beam);
+    const tuned::Beam rB{a.beam32, a.nside_beam, a.npix_beam, a.rho_max, s_B.cosr, s_B.versr, s_B.rscale};
+    const Hpx& hs = s_hs;
     const Hpx& hb = kDescSmem ? s_hb : rhb;
     const tuned::Beam& B = kDescSmem ? s_B : rB;
     const long long gw = (long long)blockIdx.x * kAW + (threadIdx.x >> 5);

@@ -68,7 +68,7 @@ struct GatherF64 : GatherSums {
 
 struct GatherPlain : GatherSums {
     using Smem = tuned::PlainSmem;
-    [[maybe_unused]] static constexpr bool kTwoFloat = true;
+    using TwoFloat = void;
     const float4* sky;
     const F8* beam;
     __device__ __forceinline__ explicit GatherPlain(const FwdArgs& a) : sky(a.sky32), beam(a.beam32) {}

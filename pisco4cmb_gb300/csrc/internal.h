@@ -252,8 +252,8 @@ cudaError_t sky_order(long long n, const double* ra, const double* dec, unsigned
 // Fills the sky ring table (4 nside - 1 entries) for nside <= 8192.
 cudaError_t launch_ring_table(int nside, RingT* rings, cudaStream_t st);
 // Batched TUNED forward (fwd_batched.cu).
-// warps: warps per block, 4, 8 or 16 (32 warps per SM for the planned nearest
-// lookup, 16 otherwise, in every shape).
+// warps: warps per block, 4, 8 or 16 (for the planned nearest lookup 20, 24 and
+// 16 warps per SM, otherwise 16).
 bool batched_warps_valid(int warps);
 // Fills cosr and versr of the device descriptors.
 cudaError_t launch_batch_trig(BatchDet* dets, int ndet, cudaStream_t st);

@@ -1,38 +1,49 @@
 // tuned_core.cuh -- per-sample body of the TUNED geometry, shared by the
 // single-detector forward (fwd_tuned.cu), the batched multi-detector forward
-// (fwd_batched.cu) and the adjoint (adjoint_kernels.cuh).
+// (fwd_batched.cu), the adjoint (adjoint_kernels.cuh) and the nearest-lookup
+// PLAIN and FP64 forms (fwd_exact.cu), which take the pairs from it and the
+// phasor exp(2i chi) to their own precision.
 //
 // A sample's FP64 set-up -- its disc plan, boresight frame and psi phasors
 // (SamplePlan, make_plan) -- is built beforehand by a plan kernel with one
-// thread per sample, or by the warp itself; the warp keeps it in its shared
-// memory (WarpSmem::plan), so the pair loop's registers hold only the pair
-// geometry (the kernels run 32 warps per SM at 64 registers).
+// thread per sample, by one lane per sample of the block's first warp (short
+// launches), or by the warp itself; the warp keeps it in its shared memory
+// (WarpSmem::plan), so the pair loop's registers hold only the pair geometry.
 //
 // For one sample, a warp evaluates the HEALPix query_disc rings, one ring per
-// lane, rounds per-ring small-offset constants to FP32 once, and strides the
-// disc pairs across lanes.  Per pair, FP32 only: longitude offset from a
-// per-ring anchor pixel, cancellation-free boresight-frame components, the
-// beam grid's polar-cap indices and exp(2i chi) as a product of unit
-// phasors.  Any of the three floor decisions lying within the margin of an
-// integer, and any pair within 2e-6 rad of the boresight, is queued and redone
-// with the FP64 chain of the PLAIN form (hpx.cuh pair_beam_pixel), so every
-// pair lands on the same beam pixel as in PLAIN.
+// lane (place_ring), rounds per-ring small-offset constants to FP32 once
+// (RingC, 48 B in shared memory), and strides the disc pairs across lanes; the
+// forward takes two neighbouring pixels of a ring per lane and iteration, with
+// the geometry of both in packed FP32 instructions, which halves the issue
+// slots and the reads of the ring constants (100,000 samples of nside 1024 and
+// 3 degrees: 5.2 -> 4.3 ms).  Per pair, FP32 only:
+// longitude offset from a per-ring anchor pixel, cancellation-free
+// boresight-frame components, the beam grid's polar-cap indices and
+// exp(2i chi) as a product of unit phasors.  Any of the three floor decisions
+// lying within the margin of an integer, and any pair within 2e-6 rad of the
+// boresight, is queued and decided in FP64: by the small-offset form in FP64
+// with Newton steps instead of transcendental functions (quick_pair), or,
+// where that too is close to an edge, with the FP64 chain of the PLAIN form
+// (hpx.cuh pair_beam_pixel), so every pair lands on the same beam pixel as in
+// PLAIN.
 //
 // The queue outlives the sample: each entry names a per-warp slot holding its
 // sample's FP64 frame and output, and the warp redoes 32 entries at a time,
-// whichever samples they came from (a sample queues about four pairs in a
-// thousand, so a per-sample drain would run the long FP64 chain with a few
-// lanes active).  The re-evaluated contributions of a sample are added in
+// whichever samples they came from (a sample queues about four pairs in ten
+// thousand, so a per-sample drain would run the FP64 code with a few lanes
+// active); what the warps of a block have left at the end the block redoes
+// together (flush_block).  The re-evaluated contributions of a sample are added in
 // queue order, one lane per sample, into an FP64 sum, and its TOD is written
 // (main-pass total + that sum) when its last entry is done: the result does
 // not depend on where the drains cut the queue, hence not on the other
 // samples of the warp.
 //
-// Disc edge: per ring, x and ysq of the HEALPix edge formula are formed in
-// FP64 with exactly HEALPix's rounding, the edge angle atan2(sqrt(ysq), x) is
-// taken in FP32, and the two floor decisions use FP64 positions; an edge
-// within the FP32 angle's error bound of a pixel boundary is recomputed with
-// the FP64 formula (disc_ring), so the disc is HEALPix query_disc's exactly.
+// Disc edge: per ring, the half width of the disc and the anchor are formed
+// in FP32 from split constants (two floats where one loses digits); an edge
+// within the error bound of a pixel boundary, and any ring near a pole or a
+// full circle, is recomputed with HEALPix's FP64 formula (disc_ring), so the
+// disc is HEALPix query_disc's exactly.  With the ring set-up in FP64 it took
+// a third of the time at 960 pairs per sample.
 //
 // Geometry, with the pixel at ring height z (s = sqrt(1 - z^2)), longitude
 // offset D from the boresight (z0, s0) and h = 1 - cos D:
@@ -49,6 +60,11 @@
 //   void reset(), total(a, b) main-pass sums (kSums)
 //   P fetch(int pix)          per-pixel data the action needs (Gather: the sky)
 //   void pair(int pix, P fetched, const F8& beam, int bp, float c2, float s2)
+//   void pair2(...)           optional: two neighbouring pixels at once
+//   void pair_all(...)        optional: every lane calls, with or without a
+//                             pair of its own (lanes share the atomics' sectors)
+//   void pair64(...)          optional: the phasor in FP64 or, with a member
+//                             type TwoFloat, in two-float arithmetic
 //   void stash(Pend&)         per-sample data a queued pair needs later
 //   void deferred(const Pend&, int pix, const F8& beam, int bp, float c2, float s2,
 //                 float& ta, float& tb)      a re-evaluated pair
@@ -106,7 +122,7 @@ struct IsExact<A, std::void_t<decltype(&A::pair64)>> : std::true_type {};
 template <class A, class = void>
 struct IsTwoFloat : std::false_type {};
 template <class A>
-struct IsTwoFloat<A, std::void_t<decltype(&A::kTwoFloat)>> : std::true_type {};
+struct IsTwoFloat<A, std::void_t<typename A::TwoFloat>> : std::true_type {};
 // Does the action take the pairs of a warp together (every lane calls
 // pair_all, with beam pixel -1 where it has no pair)?
 template <class A, class = void>
@@ -483,7 +499,7 @@ __device__ __forceinline__ float rsqrt_approx(float x)
 // hits, so a kernel whose shared memory leaves L1 150 KB or more keeps beam
 // pixels there (20 warps with two pixels per lane: 4.31 ms against 4.93 ms for
 // 100,000 samples of a 1.1 MB beam); one that leaves less gives L1 to the
-// sky, which neighbouring samples re-read (back-projection, 32 warps: 2.36 ms
+// sky, which neighbouring samples re-read (back-projection at 32 warps per SM: 2.36 ms
 // without allocation, 2.47 ms with).
 template <bool kL1 = false>
 __device__ __forceinline__ F8 load_beam(const F8* p)
@@ -1013,13 +1029,16 @@ __device__ __forceinline__ void flush(const Hpx& hs, Smem& S, Queue& Q, int lane
 // thread calls it): their left-over entries are redone together, 32 at a time
 // from whichever warp, instead of a long FP64 chain per warp with a few lanes
 // active -- what a launch of a few samples per warp spends a tenth of its time
-// on.  sm: the block's states; warps: their number.
+// on.  sm: the block's states; warps: their number.  The bilinear lookup queues
+// next to nothing (pairs at the boresight): its warps flush by themselves (2 %
+// of its time).
 template <bool kBil = false, class Smem, class Action>
 __device__ __forceinline__ void flush_block(const Hpx& hs, Smem* sm, int warps, Queue& Q, int lane,
                                             unsigned int* err, Action& act)
 {
-    __shared__ int counts[32];
     const int warp = threadIdx.x >> 5;
+    if constexpr (kBil) return flush<kBil>(hs, sm[warp], Q, lane, err, act);
+    __shared__ int counts[32];
     if (lane == 0) counts[warp] = Q.n;
     __syncthreads();
     int e = threadIdx.x, w = 0;
