@@ -13,9 +13,9 @@
 // hpx.cuh for values near a pixel's edge: the same pixels) and (c, s, d) in
 // FP64 (a table of sin and cos with a short series); a stable radix sort by
 // pixel (CUB) groups the values of a pixel while keeping them in the reference's
-// (detector, sample) order; eight lanes per occupied pixel, one per total, then
-// add them sequentially, in FP64 without contraction, onto the pixel's running
-// totals.  Each total therefore receives exactly the
+// (detector, sample) order; one thread per occupied pixel, or eight lanes with a
+// total each, then add them sequentially, in FP64 without contraction, onto the
+// pixel's running totals.  Each total therefore receives exactly the
 // reference's additions in the reference's order (bit-identical up to the
 // last-ulp differences of the device's and the host's cos/sin), with no atomics
 // and run-to-run determinism.  The solve restates the reference LAPACK
@@ -68,6 +68,14 @@ enum Scratch { kKeys = 0, kKeys2, kPos, kPos2, kRec, kUniq, kCount, kOff, kRuns,
 struct alignas(32) MapRec {
     double c, s, d, one;
 };
+__device__ __forceinline__ MapRec load_rec(const MapRec* p)
+{
+    MapRec r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(r.c), "=d"(r.s), "=d"(r.d), "=d"(r.one)
+        : "l"(p));
+    return r;
+}
 
 pisco_status map_fail(pisco_map* m, pisco_status s, const std::string& msg)
 {
@@ -228,22 +236,62 @@ __global__ void __launch_bounds__(kKeyThreads) map_keys_kernel(long long total, 
     }
 }
 
-// Eight lanes per occupied pixel, one for each of its totals but the number of
-// values: lane k adds x y of the pixel's values in sorted (= reference) order,
-// one by one, x and y two of the record's four members (FP64, not contracted;
-// a product with 1 is exact).  Adding one value to nine totals in one thread
-// took 13 FP64 instructions, and a warp as long as the longest of 32 pixels:
-// 80 us for 1,000,028 values at nside 512; here the FP64 pipe (16 cycles per
-// warp instruction) gets 2 for every 4 pixels' values: 54 us.
+// The values of each occupied pixel in sorted (= reference) order, added one by
+// one onto its totals (FP64, not contracted), eight lanes per pixel or one.
+// Eight lanes: lane k has one of the totals but the number of values, and adds x
+// y of each value, x and y two of the record's four members (a product with 1
+// is exact).  One thread takes 13 FP64 instructions per value, and a warp as
+// long as the longest of 32 pixels; eight lanes give the FP64 pipe (16 cycles
+// per warp instruction) 2 for every 4 pixels' values: 80 -> 54 us for 1,000,028
+// values at nside 512 (16 per pixel), reset to solve 0.61 -> 0.37 ms at 223 per
+// pixel, 0.43 -> 0.42 at 16, 1.73 -> 1.70 at 5.  With fewer values the eight
+// lanes' reads of the run and the totals weigh more: 0.71 -> 0.77 ms for 4M
+// values, 4.2 per pixel; so the line lies at 4.5 (0.72 ms there with both forms
+// in the kernel).
 __global__ void map_reduce_kernel(const int* runs, const int* uniq, const int* count,
                                   const int* off, const int* pos, const MapRec* rec, double* acc,
-                                  long long npix)
+                                  long long npix, int total)
 {
+    const int nr = *runs;
+    if (2LL * total < 9LL * nr) {
+        for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < nr;
+             r += (long long)gridDim.x * blockDim.x) {
+            const long long p = uniq[r];
+            if (p < 0 || p >= npix) continue;  // the sentinel run of rejected values
+            double t[kAcc];
+#pragma unroll
+            for (int k = 0; k < kAcc; ++k) t[k] = acc[k * npix + p];
+            const int b = off[r], n = count[r];
+            auto add = [&](const MapRec& v) {
+                t[kD] = PD_ADD(t[kD], v.d);
+                t[kCD] = PD_ADD(t[kCD], PD_MUL(v.c, v.d));
+                t[kSD] = PD_ADD(t[kSD], PD_MUL(v.s, v.d));
+                t[kC] = PD_ADD(t[kC], v.c);
+                t[kS] = PD_ADD(t[kS], v.s);
+                t[kCC] = PD_ADD(t[kCC], PD_MUL(v.c, v.c));
+                t[kCS] = PD_ADD(t[kCS], PD_MUL(v.c, v.s));
+                t[kSS] = PD_ADD(t[kSS], PD_MUL(v.s, v.s));
+            };
+            // four records in flight, added in order
+            int i = b;
+            for (; b + n - i >= 4; i += 4) {
+                MapRec v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = load_rec(rec + pos[i + k]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) add(v[k]);
+            }
+            for (; i < b + n; ++i) add(load_rec(rec + pos[i]));
+            t[kN] = PD_ADD(t[kN], (double)n);  // n ones added one by one: exact as well
+#pragma unroll
+            for (int k = 0; k < kAcc; ++k) acc[k * npix + p] = t[k];
+        }
+        return;
+    }
     const int k = threadIdx.x & 7;
     // the members x and y of totals kC + k: (c 1) (s 1) (c c) (c s) (s s) (d 1) (c d) (s d)
     const double* x = (const double*)rec + (0x10210010u >> 4 * k & 3u);
     const double* y = (const double*)rec + (0x22311033u >> 4 * k & 3u);
-    const int nr = *runs;
     for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3; r < nr;
          r += (long long)gridDim.x * blockDim.x >> 3) {
         const long long p = uniq[r];
@@ -253,7 +301,7 @@ __global__ void map_reduce_kernel(const int* runs, const int* uniq, const int* c
         double t = *to;
         // four values in flight, added in order
         int i = b;
-        for (; i + 4 <= e; i += 4) {
+        for (; e - i >= 4; i += 4) {
             double v[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
@@ -424,7 +472,7 @@ pisco_status accumulate(pisco_map* m, long long ns, int ndet, const T* ra, const
     tb = m->cap[kTmp];
     MCK(cub::DeviceScan::ExclusiveSum(tmp, tb, count, off, n, st), "scan");
     map_reduce_kernel<<<(int)blocks, 256, 0, st>>>(runs, uniq, count, off, pos2, rec, m->acc,
-                                                  m->npix);
+                                                  m->npix, n);
     MCK(cudaGetLastError(), "map reduce");
     unsigned int hb = 0;
     MCK(cudaMemcpyAsync(&hb, bad, sizeof(hb), cudaMemcpyDeviceToHost, st), "check D2H");

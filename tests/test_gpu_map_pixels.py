@@ -51,3 +51,35 @@ def test_hits_equal_the_oracle(gpu, oracle_mod, nside, dtype):
     assert np.array_equal(np.flatnonzero(hits), pix)
     assert np.array_equal(hits[pix], count)
     m.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("longest", [1, 7, 200])
+def test_totals_do_not_depend_on_how_pixels_are_reduced(gpu, dtype, longest):
+    """A pixel's totals are its values added one by one in order, whether one thread adds them (few
+    values per occupied pixel) or eight lanes do (many): the same bits with and without other pixels
+    of one value each in the call."""
+    from pisco4cmb_gb300 import SkyMap, pix2ang
+
+    nside = 64
+    rng = np.random.default_rng(longest)
+    few = rng.permutation(np.repeat(np.arange(100, 140), rng.integers(longest, longest + 5, 40)))
+    many = np.arange(4000, 4000 + 2 * len(few) + 300)
+
+    def normal(pix, pa, data):
+        theta, phi = pix2ang(nside, pix)
+        m = SkyMap(nside)
+        n = len(pix)
+        m.accumulate_data(n, *[v.astype(dtype)[None] for v in (phi, np.pi / 2 - theta, pa)], 1,
+                          np.array([0.3], np.float32), data.astype(dtype)[None])
+        got = [v.reshape(12 * nside * nside, -1)[100:140] for v in m.get_normal()]
+        m.close()
+        return got
+
+    pa, data = rng.uniform(0, np.pi, len(few)), rng.normal(size=len(few))
+    pa2, data2 = rng.uniform(0, np.pi, len(many)), rng.normal(size=len(many))
+    alone = normal(few, pa, data)
+    mixed = normal(np.concatenate([few, many]), np.concatenate([pa, pa2]),
+                   np.concatenate([data, data2]))
+    for x, y in zip(alone, mixed):
+        assert x.any(axis=1).all() and np.array_equal(x, y)
