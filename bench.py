@@ -417,14 +417,15 @@ def run_gpu_arm(args, rank, world, local):
     alg_bytes = pairs * BYTES_PER_PAIR + n * BYTES_PER_SAMPLE
     achieved = alg_bytes / (t_total / args.steps) / 1e9
     traffic = ncu_traffic_per_launch()
-    # what actually limits the kernel: one dependent L2 gather (the beam) per
-    # pair; L2 bytes per pair from ncu, the rate from this run's time
+    # what actually limits the kernel: the L1 data pipe, which the gather of one
+    # beam pixel per pair takes most of; L2 bytes per pair from ncu, the rate from this run's time
     l2_pp = ncu_l2_bytes_per_pair()
     l2_line = None if l2_pp is None else {
         "bytes_per_pair": l2_pp, "achieved_gbs": pairs * l2_pp / (t_total / args.steps) / 1e9,
-        "l1_serves": "the sky reads (all hits)", "l2_serves": "the beam gather (all L1 misses)",
+        "l1_serves": "the sky reads, a sixth of the beam gather", "l2_serves": "the rest of the beam gather",
         "source": "profiles/tuned_forward_c2_ncu.md"}
 
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
     line = None
     if rank == 0:
         cpu = None
@@ -449,7 +450,8 @@ def run_gpu_arm(args, rank, world, local):
             "e2e": {"value": e2e_value, "unit": "samples/s", "h2d_bytes_per_step": n * 24,
                     "d2h_bytes_per_step": n * 8},
             # per step: the plan kernel and the pair kernel, per 4M-sample chunk
-            "gpu_launches": args.steps * 2 * (-(-n // PLAN_CHUNK)),
+            # (a step of at most 64 samples per SM: the pair kernel, which plans itself)
+            "gpu_launches": args.steps * (1 if n <= 64 * sms else 2 * (-(-n // PLAN_CHUNK))),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": peak_kind,
                          "kernel": "the forward step: plan_kernel + tuned_kernel",

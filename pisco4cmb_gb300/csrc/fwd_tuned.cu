@@ -16,13 +16,13 @@ namespace {
 
 // Launch shape: the nearest lookup runs one block of 20 warps per SM (register
 // cap 96, no spills), two pixels per lane: its pair loop is bound by the L1
-// pipe (94 % busy at 1.1 MB of beam: the beam gather, the sky and the rings'
+// pipe (87 % busy at 1.1 MB of beam: the beam gather, the sky and the rings'
 // constants), and 20 warps leave L1 156 KB.  100,000 samples of nside 1024 and
 // a 3 degree beam: 16 warps 4.53 ms, 20 warps 4.31 ms, 24 warps (80 registers,
 // spilling) 4.47 ms; one pixel per lane at 32 warps of 64 registers took 5.2
 // ms.  The warps of a block work on consecutive samples, whose discs overlap,
 // so their sky reads share L1.  The bilinear lookup, which needs more
-// registers per pair, runs 8 x 2 with its descriptors in registers.
+// registers per pair, runs 8 x 2.
 #ifndef PISCO_FWD_WARPS
 #define PISCO_FWD_WARPS 20
 #endif
