@@ -75,8 +75,17 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
     const Hpx& hs = s_hs;
     const Hpx& hb = kDescSmem ? s_hb : rhb;
     const tuned::Beam& B = kDescSmem ? s_B : rB;
-    const long long gw = (long long)blockIdx.x * kTW + (threadIdx.x >> 5);
-    const long long nw = (long long)gridDim.x * kTW;
+    // the warp's positions: first, first + step, ...; a short launch gives each
+    // block a contiguous share
+    long long first = pos0 + (long long)blockIdx.x * kTW + (threadIdx.x >> 5);
+    long long step = (long long)gridDim.x * kTW, end = pos1, lo = 0;
+    if constexpr (kPlans == kBlockPlans) {
+        const int n = (int)(pos1 - pos0), g = gridDim.x, b = blockIdx.x;
+        lo = pos0 + n / g * b + min(b, n % g);
+        end = lo + n / g + (b < n % g ? 1 : 0);
+        first = lo + (threadIdx.x >> 5);
+        step = kTW;
+    }
     unsigned long long nfall = 0, npairs = 0;
     float cmax = 0.0f;
     tuned::Gather<true> g;
@@ -86,23 +95,21 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
     __shared__ tuned::SamplePlan s_plans[kPlans == kBlockPlans ? 32 : 1];
     if constexpr (kPlans == kBlockPlans) {
         if (threadIdx.x < 32) {
-            // lane l: the plan of warp l % kTW's sample number l / kTW
-            const long long i = pos0 + (long long)blockIdx.x * kTW + lane % kTW + lane / kTW * nw;
-            if (lane < 32 / kTW * kTW && i < pos1) {
+            const long long i = lo + lane;
+            if (i < end) {
                 const long long s = a.begin + (a.order ? (long long)a.order[i] : i);
                 s_plans[lane] = tuned::make_plan(hs, B, a.ra[s], a.dec[s], a.pa[s]);
             }
         }
         __syncthreads();
     }
-    int mine = threadIdx.x >> 5;  // kBlockPlans: this sample's plan
-    for (long long i = pos0 + gw; i < pos1; i += nw, mine += kTW) {
+    for (long long i = first; i < end; i += step) {
         const long long j = a.order ? (long long)a.order[i] : i;  // sample of position i
         const long long s = a.begin + j;
         const tuned::Out o{a.out_a, a.out_b, j, a.out_f64};
         const double ra = a.ra[s], dec = a.dec[s], pa = a.pa[s];
         if constexpr (kPlans != kOwnPlans)
-            tuned::sample_planned<kCalib, kBil>(kPlans == kBlockPlans ? s_plans[mine] : plans[i - pos0],
+            tuned::sample_planned<kCalib, kBil>(kPlans == kBlockPlans ? s_plans[i - lo] : plans[i - pos0],
                                                 hs, a.rings, hb, B, ra, dec, pa, o,
                                                 S, Q, lane, a.err, g, nfall, cmax, npairs);
         else
@@ -172,7 +179,10 @@ __global__ void ring_table_kernel(int nside, RingT* rings)
     }
 }
 
-constexpr int kShortWarps = 8, kShortBlocks = 2;  // a short launch's blocks, and theirs per SM
+// A short launch's warps per block, and its blocks per SM.
+template <bool kBil>
+constexpr int kShortWarps = kBil ? PISCO_BIL_WARPS : PISCO_FWD_WARPS / 2;
+constexpr int kShortBlocks = 2;
 
 }  // namespace
 
@@ -215,19 +225,23 @@ void launch_shape(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib,
         const long long p1 = p0 + step < a.n ? p0 + step : a.n;
         if (kPlans == kArrayPlans) launch_plans(a, plans, p0, p1, st);
         long long blocks = (p1 - p0 + kTW - 1) / kTW;
-        if (kPlans != kBlockPlans && resident < blocks) blocks = resident;
-        // kBlockPlans: every warp's samples have a plan among the block's 32
-        else if (kPlans == kBlockPlans && blocks > kShortBlocks * sm_count) blocks = kShortBlocks * sm_count;
+        if (kPlans == kBlockPlans)  // at most 32 samples to a block
+            blocks = a.n < kShortBlocks * sm_count ? a.n : kShortBlocks * sm_count;
+        else if (resident < blocks)
+            blocks = resident;
         tuned_kernel<kCalib, kBil, kTW, kPlans>
             <<<(int)blocks, threads, 0, st>>>(a, calib, plans, p0, p1);
     }
 }
 
 // kTW: the planned launch's block.  A short launch (tuned_plans_itself: at most
-// four samples per warp of two blocks of 8 per SM) uses blocks of 8 warps, so
-// that its samples spread over every SM (20-warp blocks would fill n / 20 SMs),
-// and plans in the block: 2,003 samples spent 11 us of 178 in plan_kernel and
-// 3 between the launches.  Without plans the warps build their own (FP64 disc
+// 64 samples per SM, 32 to a block) gives two blocks per SM an equal share of
+// the samples each, and plans in the block.  2,003 samples of nside 1024 and 3
+// degrees: 184 us in full 20-warp blocks with plan_kernel before them, 155 in
+// full blocks of 8 that plan themselves, which leave a third of the SMs with
+// half the work of the others, 151 with equal shares of 10 warps (20 per SM);
+// 3,040 samples 184, 229 and 181 us; 4,000 samples 314, 257 and 261; 6,000
+// samples 317, 350 and 309; 7,000 samples 445, 362 and 387.  Without plans the warps build their own (FP64 disc
 // plan in the loop's registers).
 template <bool kBil, int kTW>
 void launch_lookup(const FwdArgs& a, int sm_count, cudaStream_t st, tuned::SamplePlan* plans,
@@ -235,7 +249,7 @@ void launch_lookup(const FwdArgs& a, int sm_count, cudaStream_t st, tuned::Sampl
 {
     constexpr int kUnplanned = kTW > 16 ? 16 : kTW;
     if (tuned_plans_itself(a.n, sm_count))
-        launch_shape<false, kBil, kShortWarps, kBlockPlans>(a, sm_count, st, nullptr, nullptr, 0);
+        launch_shape<false, kBil, kShortWarps<kBil>, kBlockPlans>(a, sm_count, st, nullptr, nullptr, 0);
     else if (plans && plan_cap > 0)
         launch_shape<false, kBil, kTW, kArrayPlans>(a, sm_count, st, nullptr, plans, plan_cap);
     else
