@@ -166,6 +166,19 @@ pisco_status pisco_last_fallbacks(pisco_ctx* ctx, long long* fallbacks);
  * pisco_count_pairs over the same samples).  Outputs are discarded. */
 pisco_status pisco_tuned_calibrate(pisco_ctx* ctx, long begin, long n, double* worst_fraction,
                                    long long* tuned_pairs);
+/* The same for any form's nearest-lookup kernel (the beam must lie in the
+ * TUNED domain), pair by pair against the reference's FP64 chain. */
+typedef struct pisco_decision_check {
+    double worst_fp32;    /* worst error of an FP32 decision, in units of the
+                             margin within which it is redone in FP64 */
+    double worst_fp64;    /* worst difference between the FP64 re-evaluation and
+                             the chain, in units of the margin within which the
+                             chain itself decides */
+    long long pairs;      /* disc pairs visited */
+    long long differing;  /* pairs whose beam pixel is not the chain's */
+} pisco_decision_check;
+pisco_status pisco_debug_decisions(pisco_ctx* ctx, pisco_form form, long begin, long n,
+                                   pisco_decision_check* out);
 
 /* ---- per-pair record of a form's decisions (diagnostic; no reference
  *      counterpart as an entry point -- the reference checks the same

@@ -90,6 +90,13 @@ class PairDump(ctypes.Structure):
                 ("stencil_w", ctypes.c_void_p)]
 
 
+class DecisionCheck(ctypes.Structure):
+    """pisco_decision_check: a form's decisions against the reference's chain."""
+
+    _fields_ = [("worst_fp32", ctypes.c_double), ("worst_fp64", ctypes.c_double),
+                ("pairs", ctypes.c_longlong), ("differing", ctypes.c_longlong)]
+
+
 PAIR_REDONE = 1
 PAIR_OUTSIDE_BEAM = 2
 
@@ -125,6 +132,7 @@ SIGNATURES = [
     ("pisco_last_fallbacks", _S, [_P, ctypes.POINTER(ctypes.c_longlong)]),
     ("pisco_tuned_calibrate", _S, [_P, _L, _L, ctypes.POINTER(ctypes.c_double),
                                    ctypes.POINTER(ctypes.c_longlong)]),
+    ("pisco_debug_decisions", _S, [_P, _I, _L, _L, ctypes.POINTER(DecisionCheck)]),
     ("pisco_debug_pairs", _S, [_P, _I, _L, _L, ctypes.POINTER(PairDump),
                                ctypes.POINTER(ctypes.c_longlong)]),
     ("pisco_hpx_pix2ang_device", _S, [_I, ctypes.c_longlong, _P, _P, _P, _P]),

@@ -500,6 +500,15 @@ class GPUConvolver:
               self.ctx, "tuned_calibrate")
         return (float(v.value), int(p.value)) if with_pairs else float(v.value)
 
+    def debug_decisions(self, form: str | None = None, begin: int = 0, n: int | None = None):
+        """Every pair's decisions of ``form``'s nearest lookup against the reference's chain
+        (pisco_debug_decisions): worst_fp32, worst_fp64, pairs, differing."""
+        n = self._n - begin if n is None else n
+        out = _lib.DecisionCheck()
+        check(load().pisco_debug_decisions(self.ctx, FORMS[form or self.form], begin, n,
+                                           ctypes.byref(out)), self.ctx, "debug_decisions")
+        return out
+
     def debug_pairs(self, form: str | None = None, begin: int = 0, n: int | None = None) -> dict:
         """Every (sample, disc pixel) pair the kernels of ``form`` visit over
         samples [begin, begin+n), with their decisions (pisco_debug_pairs):

@@ -469,8 +469,8 @@ __global__ void __launch_bounds__(kAW * 32, adj_warps_per_sm<Act, kBil, kPlanned
     const tuned::Beam& B = kDescSmem ? s_B : rB;
     const long long gw = (long long)blockIdx.x * kAW + (threadIdx.x >> 5);
     const long long nw = (long long)gridDim.x * kAW;
-    unsigned long long nfall = 0, npairs = 0;
-    float cmax = 0.0f;
+    unsigned long long nfall = 0;
+    tuned::Check ck;
     Act act = proto;
     tuned::Queue Q{0, 0};
     const tuned::Out none{nullptr, nullptr, 0, 0};
@@ -484,11 +484,10 @@ __global__ void __launch_bounds__(kAW * 32, adj_warps_per_sm<Act, kBil, kPlanned
         act.gb = (float)gb;
         if constexpr (kPlanned)
             tuned::sample_planned<false, kBil>(a.plans[i], hs, a.rings, hb, B, a.ra[s], a.dec[s],
-                                               a.pa[s], none, S, Q, lane, a.err, act, nfall, cmax,
-                                               npairs);
+                                               a.pa[s], none, S, Q, lane, a.err, act, nfall, ck);
         else
             tuned::sample<false, kBil>(hs, a.rings, hb, B, a.ra[s], a.dec[s], a.pa[s], none, S, Q,
-                                       lane, a.err, act, nfall, cmax, npairs);
+                                       lane, a.err, act, nfall, ck);
     }
     tuned::flush_block<kBil>(hs, sm, kAW, Q, lane, a.err, act);
     if (lane == 0 && nfall && a.fallbacks) atomicAdd(a.fallbacks, nfall);

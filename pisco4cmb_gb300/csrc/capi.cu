@@ -46,6 +46,27 @@ pisco_status cuda_fail(pisco_ctx* c, cudaError_t e, const char* what)
         if (e_ != cudaSuccess) return cuda_fail(c, e_, what); \
     } while (0)
 
+// The FP64 form's maps: as given in FP64, or widened from the FP32 ones.
+pisco_status wide_maps(pisco_ctx* c, cudaStream_t s, FwdArgs& a)
+{
+    const long long npix = 12LL * c->nside_sky * c->nside_sky;
+    if (!c->sky64_valid) {
+        const pisco_status st = c->ensure((void**)&c->sky64, &c->sky64_cap, sizeof(D4) * npix, "sky64 buffer");
+        if (st != PISCO_OK) return st;
+        CK(launch_widen_sky(c->sky32, c->sky64, npix, s), "widen sky");
+        c->sky64_valid = true;
+    }
+    if (!c->beam64_valid) {
+        const pisco_status st = c->ensure((void**)&c->beam64, &c->beam64_cap, sizeof(D8) * c->npix_beam, "beam64 buffer");
+        if (st != PISCO_OK) return st;
+        CK(launch_widen_beam(c->beam32, c->beam64, c->npix_beam, s), "widen beam");
+        c->beam64_valid = true;
+    }
+    a.sky64 = c->sky64;
+    a.beam64 = c->beam64;
+    return PISCO_OK;
+}
+
 }  // namespace
 
 namespace pisco {
@@ -638,21 +659,8 @@ pisco_status pisco_forward_device(pisco_ctx* c, pisco_form form, long begin, lon
     void* plans = nullptr;
     long long plan_cap = 0;
     if (form == PISCO_FORM_FP64) {
-        const long long npix = 12LL * c->nside_sky * c->nside_sky;
-        if (!c->sky64_valid) {
-            st = c->ensure((void**)&c->sky64, &c->sky64_cap, sizeof(D4) * npix, "sky64 buffer");
-            if (st != PISCO_OK) return st;
-            CK(launch_widen_sky(c->sky32, c->sky64, npix, s), "widen sky");
-            c->sky64_valid = true;
-        }
-        if (!c->beam64_valid) {
-            st = c->ensure((void**)&c->beam64, &c->beam64_cap, sizeof(D8) * c->npix_beam, "beam64 buffer");
-            if (st != PISCO_OK) return st;
-            CK(launch_widen_beam(c->beam32, c->beam64, c->npix_beam, s), "widen beam");
-            c->beam64_valid = true;
-        }
-        a.sky64 = c->sky64;
-        a.beam64 = c->beam64;
+        st = wide_maps(c, s, a);
+        if (st != PISCO_OK) return st;
         if (exact) {
             c->plan_scratch(n, s, &plans, &plan_cap);
             e = launch_forward_exact(a, true, c->sm_count, s, plans, plan_cap);
@@ -766,10 +774,12 @@ pisco_status pisco_last_fallbacks(pisco_ctx* c, long long* fallbacks)
     return PISCO_OK;
 }
 
-pisco_status pisco_tuned_calibrate(pisco_ctx* c, long begin, long n, double* worst,
-                                   long long* tuned_pairs)
+pisco_status pisco_debug_decisions(pisco_ctx* c, pisco_form form, long begin, long n,
+                                   pisco_decision_check* out)
 {
-    if (!c || !worst) return PISCO_ERR_INVALID_ARGUMENT;
+    if (!c || !out) return PISCO_ERR_INVALID_ARGUMENT;
+    if (form != PISCO_FORM_PLAIN && form != PISCO_FORM_TUNED && form != PISCO_FORM_FP64)
+        return fail(c, PISCO_ERR_INVALID_ARGUMENT, "bad form");
     if (!c->sky32 || !c->nside_sky || !c->beam32)
         return fail(c, PISCO_ERR_NOT_READY, "sky and beam required");
     if (begin < 0 || n < 0 || begin + n > c->nsamples)
@@ -778,9 +788,6 @@ pisco_status pisco_tuned_calibrate(pisco_ctx* c, long begin, long n, double* wor
         return fail(c, PISCO_ERR_UNSUPPORTED, "beam outside the tuned form's domain");
     pisco_status st = c->activate();
     if (st != PISCO_OK) return st;
-    float* d = nullptr;  // {worst fraction, pad, u64 disc pairs of the TUNED disc}
-    CK(cudaMalloc(&d, 16), "calib buffer");
-    cudaMemsetAsync(d, 0, 16, c->stream);
     FwdArgs a{};
     a.nside_sky = c->nside_sky;
     a.sky32 = c->sky32;
@@ -796,17 +803,41 @@ pisco_status pisco_tuned_calibrate(pisco_ctx* c, long begin, long n, double* wor
     a.pa = c->pa;
     a.err = c->d_err;
     a.fallbacks = c->d_fallbacks;
-    cudaError_t e = launch_tuned_calibrate(a, c->sm_count, c->stream, d);
-    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(v, d, 16, cudaMemcpyDeviceToHost, c->stream);
+    if (form == PISCO_FORM_FP64) {
+        st = wide_maps(c, c->stream, a);
+        if (st != PISCO_OK) return st;
+    }
+    CheckOut* d = nullptr;
+    CK(cudaMalloc(&d, sizeof(CheckOut)), "check buffer");
+    CheckOut v{};
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(v), c->stream);
+    if (e == cudaSuccess)
+        e = form == PISCO_FORM_TUNED
+                ? launch_tuned_check(a, c->sm_count, c->stream, d)
+                : launch_exact_check(a, form == PISCO_FORM_FP64, c->sm_count, c->stream, d);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&v, d, sizeof(v), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     cudaFree(d);
-    if (e != cudaSuccess) return cuda_fail(c, e, "calibration");
-    *worst = v[0];
-    unsigned long long pairs = 0;
-    std::memcpy(&pairs, &v[2], sizeof(pairs));
-    if (tuned_pairs) *tuned_pairs = (long long)pairs;
+    if (e != cudaSuccess) return cuda_fail(c, e, "decision check");
+    float f[2];
+    std::memcpy(f, &v, sizeof(f));
+    out->worst_fp32 = f[0];
+    out->worst_fp64 = f[1];
+    out->pairs = (long long)v.pairs;
+    out->differing = (long long)v.differ;
     return c->check_device();
+}
+
+pisco_status pisco_tuned_calibrate(pisco_ctx* c, long begin, long n, double* worst,
+                                   long long* tuned_pairs)
+{
+    if (!c || !worst) return PISCO_ERR_INVALID_ARGUMENT;
+    pisco_decision_check check;
+    const pisco_status st = pisco_debug_decisions(c, PISCO_FORM_TUNED, begin, n, &check);
+    if (st != PISCO_OK) return st;
+    *worst = check.worst_fp32;
+    if (tuned_pairs) *tuned_pairs = check.pairs;
+    return PISCO_OK;
 }
 
 }  // extern "C"

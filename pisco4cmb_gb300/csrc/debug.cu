@@ -6,8 +6,10 @@
 // (sample, disc pixel) pair: the disc itself, the beam pixel of the nearest
 // lookup or the four-pixel stencil of the bilinear one, and the polarization
 // angle.  The TUNED record runs the TUNED per-sample body itself
-// (tuned::sample with a recording action in place of the sky gather); the
-// PLAIN record runs the PLAIN form's disc walk and per-pair functions.  The
+// (tuned::sample with a recording action in place of the sky gather, with the
+// nearest lookup two pixels per lane as the forward); the PLAIN record runs the
+// reference chain's disc walk and per-pair functions (fwd_plain.cu), which the
+// decisions of every form are held against (pisco_debug_decisions).  The
 // reference checks the same decisions with its own device tests
 // (tests/cudaConvolution/test_sky_to_beam_matching_kernel.cu:188-216,
 // tests/cudaHealpix/test_pix2ang.cu:80-114, test_interpol.cu).
@@ -54,6 +56,7 @@ pisco_status cuda_fail(pisco_ctx* c, cudaError_t e, const char* what)
 // Action of tuned::sample that writes each pair's decisions instead of
 // gathering the sky.
 struct Record {
+    static constexpr bool kL1 = false;  // load_beam
     static constexpr bool kSums = false;
     static constexpr bool kStencil = true;
     PairDump d;
@@ -83,10 +86,11 @@ struct Record {
             d.st_w[4 * k + i] = px ? (double)w[i] : 0.0;
         }
     }
-    __device__ __forceinline__ void pair(int pix, const float4&, const F8&, int bp, float c2,
-                                         float s2) const
+    __device__ __forceinline__ void fetch2(int, float4&, float4&) const {}
+    __device__ __forceinline__ void pair2(const tuned::Unit& U) const
     {
-        put(cur, pix, bp, c2, s2, 0, nullptr, nullptr);
+        if (U.in0) put(cur, U.pix, U.bp0, tuned::lo2(U.c), tuned::lo2(U.s), 0, nullptr, nullptr);
+        if (U.in1) put(cur, U.pix + 1, U.bp1, tuned::hi2(U.c), tuned::hi2(U.s), 0, nullptr, nullptr);
     }
     __device__ __forceinline__ void deferred(const tuned::Pend& P, int pix, const F8&, int bp,
                                             float c2, float s2, float&, float&) const
@@ -124,8 +128,8 @@ __global__ void __launch_bounds__(kTW * 32, PISCO_TUNED_MINB) tuned_dump_kernel(
     const tuned::Beam B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
     const long long gw = (long long)blockIdx.x * kTW + (threadIdx.x >> 5);
     const long long nw = (long long)gridDim.x * kTW;
-    unsigned long long nfall = 0, npairs = 0;
-    float cmax = 0.0f;
+    unsigned long long nfall = 0;
+    tuned::Check ck;
     Record rec{d, a.err, 0};
     tuned::Queue Q{0, 0};
     for (long long j = gw; j < a.n; j += nw) {
@@ -133,7 +137,7 @@ __global__ void __launch_bounds__(kTW * 32, PISCO_TUNED_MINB) tuned_dump_kernel(
         rec.cur = j;
         const tuned::Out o{nullptr, nullptr, j, 0};
         tuned::sample<false, kBil>(hs, a.rings, hb, B, a.ra[s], a.dec[s], a.pa[s], o, S, Q, lane,
-                                   a.err, rec, nfall, cmax, npairs);
+                                   a.err, rec, nfall, ck);
     }
     tuned::flush<kBil>(hs, S, Q, lane, a.err, rec);
 }

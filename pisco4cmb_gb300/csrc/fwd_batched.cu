@@ -117,8 +117,8 @@ __global__ void __launch_bounds__(kW * 32, warps_per_sm<kBil, kPlanned, kW>() / 
     if (threadIdx.x == 0) s_hs = hpx_make(a.nside_sky);
     __syncthreads();
     const Hpx& hs = s_hs;
-    unsigned long long nfall = 0, npairs = 0;
-    float cmax = 0.0f;
+    unsigned long long nfall = 0;
+    tuned::Check ck;
     tuned::Gather<(warps_per_sm<kBil, kPlanned, kW>() <= 20)> g;
     g.sky = a.sky32;
     g.wide = (reinterpret_cast<size_t>(a.sky32) & 31) == 0;
@@ -162,10 +162,10 @@ __global__ void __launch_bounds__(kW * 32, warps_per_sm<kBil, kPlanned, kW>() / 
             if constexpr (kPlanned)
                 tuned::sample_planned<false, kBil>(a.plans[T.plan_base + p], hs, a.rings, T.hb, T.B,
                                                    T.ra[s], T.dec[s], T.pa[s], o, S, Q, lane, a.err,
-                                                   g, nfall, cmax, npairs);
+                                                   g, nfall, ck);
             else
                 tuned::sample<false, kBil>(hs, a.rings, T.hb, T.B, T.ra[s], T.dec[s], T.pa[s], o,
-                                           S, Q, lane, a.err, g, nfall, cmax, npairs);
+                                           S, Q, lane, a.err, g, nfall, ck);
         }
     }
     tuned::flush_block<kBil>(hs, sm, kBW, Q, lane, a.err, g);

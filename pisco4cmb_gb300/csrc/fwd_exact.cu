@@ -103,9 +103,10 @@ struct GatherPlain : GatherSums {
 
 // kPlanned: plans holds the plans of positions [pos0, pos1); otherwise each
 // warp builds its own (the same values).
-template <class Act, bool kPlanned>
+// kCheck: the pairs' decisions are compared with the chain's (*check).
+template <class Act, bool kPlanned, bool kCheck>
 __global__ void __launch_bounds__(kEW * 32, 2)
-    exact_kernel(FwdArgs a, const tuned::SamplePlan* __restrict__ plans, long long pos0,
+    exact_kernel(FwdArgs a, CheckOut* check, const tuned::SamplePlan* __restrict__ plans, long long pos0,
                  long long pos1)
 {
     __shared__ typename Act::Smem sm[kEW];
@@ -119,8 +120,8 @@ __global__ void __launch_bounds__(kEW * 32, 2)
         s_B = tuned::make_beam(a.beam32, a.nside_beam, a.npix_beam, a.rho_max);
     }
     __syncthreads();
-    unsigned long long nfall = 0, npairs = 0;
-    float cmax = 0.0f;
+    unsigned long long nfall = 0;
+    tuned::Check ck;
     Act g(a);
     tuned::Queue Q{0, 0};
     const long long gw = (long long)blockIdx.x * kEW + (threadIdx.x >> 5);
@@ -131,26 +132,27 @@ __global__ void __launch_bounds__(kEW * 32, 2)
         const tuned::Out o{a.out_a, a.out_b, j, a.out_f64};
         const double ra = a.ra[s], dec = a.dec[s], pa = a.pa[s];
         if constexpr (kPlanned)
-            tuned::sample_planned<false>(plans[i - pos0], s_hs, a.rings, s_hb, s_B, ra, dec, pa, o,
-                                         S, Q, lane, a.err, g, nfall, cmax, npairs);
+            tuned::sample_planned<kCheck>(plans[i - pos0], s_hs, a.rings, s_hb, s_B, ra, dec, pa, o,
+                                         S, Q, lane, a.err, g, nfall, ck);
         else
-            tuned::sample<false>(s_hs, a.rings, s_hb, s_B, ra, dec, pa, o, S, Q, lane, a.err, g,
-                                 nfall, cmax, npairs);
+            tuned::sample<kCheck>(s_hs, a.rings, s_hb, s_B, ra, dec, pa, o, S, Q, lane, a.err, g,
+                                 nfall, ck);
     }
     tuned::flush_block(s_hs, sm, kEW, Q, lane, a.err, g);
+    if constexpr (kCheck) tuned::report(ck, check);
 }
 
-template <class Act, bool kPlanned>
+template <class Act, bool kPlanned, bool kCheck = false>
 void launch_form(const FwdArgs& a, int sm_count, cudaStream_t st, tuned::SamplePlan* plans,
-                 long long plan_cap)
+                 long long plan_cap, CheckOut* check = nullptr)
 {
     const long long step = kPlanned ? plan_cap : a.n;
     for (long long p0 = 0; p0 < a.n; p0 += step) {
         const long long p1 = p0 + step < a.n ? p0 + step : a.n;
         if (kPlanned) launch_plans(a, plans, p0, p1, st);
         const long long need = (p1 - p0 + kEW - 1) / kEW, most = 2LL * sm_count;
-        exact_kernel<Act, kPlanned>
-            <<<(int)(most < need ? most : need), kEW * 32, 0, st>>>(a, plans, p0, p1);
+        exact_kernel<Act, kPlanned, kCheck>
+            <<<(int)(most < need ? most : need), kEW * 32, 0, st>>>(a, check, plans, p0, p1);
     }
 }
 
@@ -168,6 +170,15 @@ cudaError_t launch_forward_exact(const FwdArgs& a, bool f64, int sm_count, cudaS
         if (f64) launch_form<GatherF64, false>(a, sm_count, st, nullptr, 0);
         else launch_form<GatherPlain, false>(a, sm_count, st, nullptr, 0);
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_exact_check(const FwdArgs& a, bool f64, int sm_count, cudaStream_t st,
+                               CheckOut* check)
+{
+    if (a.n <= 0) return cudaSuccess;
+    if (f64) launch_form<GatherF64, false, true>(a, sm_count, st, nullptr, 0, check);
+    else launch_form<GatherPlain, false, true>(a, sm_count, st, nullptr, 0, check);
     return cudaGetLastError();
 }
 

@@ -41,15 +41,15 @@ enum Plans { kOwnPlans, kArrayPlans, kBlockPlans };
 // position - pos0.
 // Warps per SM: 20 for the planned nearest lookup (register cap 96), 16 for
 // the others (cap 128).
-template <bool kCalib, bool kBil, Plans kPlans>
+template <bool kBil, Plans kPlans>
 constexpr int fwd_warps_per_sm()
 {
-    return kPlans != kOwnPlans && !kBil && !kCalib ? PISCO_FWD_WARPS : 16;
+    return kPlans != kOwnPlans && !kBil ? PISCO_FWD_WARPS : 16;
 }
 
-template <bool kCalib, bool kBil, int kTW, Plans kPlans>
-__global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlans>() / kTW)
-    tuned_kernel(FwdArgs a, float* calib, const tuned::SamplePlan* __restrict__ plans,
+template <bool kCheck, bool kBil, int kTW, Plans kPlans>
+__global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kBil, kPlans>() / kTW)
+    tuned_kernel(FwdArgs a, CheckOut* check, const tuned::SamplePlan* __restrict__ plans,
                  long long pos0, long long pos1)
 {
     __shared__ tuned::WarpSmem sm[kTW];
@@ -86,8 +86,8 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
         first = lo + (threadIdx.x >> 5);
         step = kTW;
     }
-    unsigned long long nfall = 0, npairs = 0;
-    float cmax = 0.0f;
+    unsigned long long nfall = 0;
+    tuned::Check ck;
     tuned::Gather<true> g;
     g.sky = a.sky32;
     g.wide = (reinterpret_cast<size_t>(a.sky32) & 31) == 0;
@@ -109,23 +109,16 @@ __global__ void __launch_bounds__(kTW * 32, fwd_warps_per_sm<kCalib, kBil, kPlan
         const tuned::Out o{a.out_a, a.out_b, j, a.out_f64};
         const double ra = a.ra[s], dec = a.dec[s], pa = a.pa[s];
         if constexpr (kPlans != kOwnPlans)
-            tuned::sample_planned<kCalib, kBil>(kPlans == kBlockPlans ? s_plans[i - lo] : plans[i - pos0],
+            tuned::sample_planned<kCheck, kBil>(kPlans == kBlockPlans ? s_plans[i - lo] : plans[i - pos0],
                                                 hs, a.rings, hb, B, ra, dec, pa, o,
-                                                S, Q, lane, a.err, g, nfall, cmax, npairs);
+                                                S, Q, lane, a.err, g, nfall, ck);
         else
-            tuned::sample<kCalib, kBil>(hs, a.rings, hb, B, ra, dec, pa, o, S, Q, lane, a.err, g,
-                                        nfall, cmax, npairs);
+            tuned::sample<kCheck, kBil>(hs, a.rings, hb, B, ra, dec, pa, o, S, Q, lane, a.err, g,
+                                        nfall, ck);
     }
     tuned::flush_block<kBil>(hs, sm, kTW, Q, lane, a.err, g);
     if (lane == 0 && nfall && a.fallbacks) atomicAdd(a.fallbacks, nfall);
-    if (kCalib && calib) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cmax = fmaxf(cmax, __shfl_xor_sync(tuned::kFull, cmax, o));
-        if (lane == 0) {
-            atomicMax((int*)calib, __float_as_int(cmax));
-            atomicAdd(reinterpret_cast<unsigned long long*>(calib + 2), npairs);
-        }
-    }
+    if constexpr (kCheck) tuned::report(ck, check);
 }
 
 // The sample plans of positions [pos0, pos1), one thread per sample.
@@ -213,13 +206,13 @@ int resident_blocks(K kernel, int threads)
     return nb;
 }
 
-template <bool kCalib, bool kBil, int kTW, Plans kPlans>
-void launch_shape(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib,
+template <bool kCheck, bool kBil, int kTW, Plans kPlans>
+void launch_shape(const FwdArgs& a, int sm_count, cudaStream_t st, CheckOut* check,
                   tuned::SamplePlan* plans, long long plan_cap)
 {
     const int threads = kTW * 32;
     const long long resident =
-        (long long)sm_count * resident_blocks(tuned_kernel<kCalib, kBil, kTW, kPlans>, threads);
+        (long long)sm_count * resident_blocks(tuned_kernel<kCheck, kBil, kTW, kPlans>, threads);
     const long long step = kPlans == kArrayPlans ? plan_cap : a.n;
     for (long long p0 = 0; p0 < a.n; p0 += step) {
         const long long p1 = p0 + step < a.n ? p0 + step : a.n;
@@ -229,8 +222,8 @@ void launch_shape(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib,
             blocks = a.n < kShortBlocks * sm_count ? a.n : kShortBlocks * sm_count;
         else if (resident < blocks)
             blocks = resident;
-        tuned_kernel<kCalib, kBil, kTW, kPlans>
-            <<<(int)blocks, threads, 0, st>>>(a, calib, plans, p0, p1);
+        tuned_kernel<kCheck, kBil, kTW, kPlans>
+            <<<(int)blocks, threads, 0, st>>>(a, check, plans, p0, p1);
     }
 }
 
@@ -254,17 +247,6 @@ void launch_lookup(const FwdArgs& a, int sm_count, cudaStream_t st, tuned::Sampl
         launch_shape<false, kBil, kTW, kArrayPlans>(a, sm_count, st, nullptr, plans, plan_cap);
     else
         launch_shape<false, kBil, kUnplanned, kOwnPlans>(a, sm_count, st, nullptr, nullptr, 0);
-}
-
-cudaError_t launch_tuned_impl(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib,
-                              tuned::SamplePlan* plans, long long plan_cap)
-{
-    if (a.n <= 0) return cudaSuccess;
-    // calibration measures the nearest-pixel decisions, whatever the lookup
-    if (calib) launch_shape<true, false, 16, kOwnPlans>(a, sm_count, st, calib, nullptr, 0);
-    else if (a.interp == 1) launch_lookup<true, PISCO_BIL_WARPS>(a, sm_count, st, plans, plan_cap);
-    else launch_lookup<false, PISCO_FWD_WARPS>(a, sm_count, st, plans, plan_cap);
-    return cudaGetLastError();
 }
 
 }  // namespace
@@ -291,13 +273,18 @@ cudaError_t launch_ring_table(int nside, RingT* rings, cudaStream_t st)
 cudaError_t launch_forward_tuned(const FwdArgs& a, int sm_count, cudaStream_t st, void* plans,
                                  long long plan_cap)
 {
-    return launch_tuned_impl(a, sm_count, st, nullptr, static_cast<tuned::SamplePlan*>(plans),
-                             plan_cap);
+    if (a.n <= 0) return cudaSuccess;
+    tuned::SamplePlan* p = static_cast<tuned::SamplePlan*>(plans);
+    if (a.interp == 1) launch_lookup<true, PISCO_BIL_WARPS>(a, sm_count, st, p, plan_cap);
+    else launch_lookup<false, PISCO_FWD_WARPS>(a, sm_count, st, p, plan_cap);
+    return cudaGetLastError();
 }
 
-cudaError_t launch_tuned_calibrate(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib)
+cudaError_t launch_tuned_check(const FwdArgs& a, int sm_count, cudaStream_t st, CheckOut* check)
 {
-    return launch_tuned_impl(a, sm_count, st, calib, nullptr, 0);
+    if (a.n <= 0) return cudaSuccess;
+    launch_shape<true, false, 16, kOwnPlans>(a, sm_count, st, check, nullptr, 0);
+    return cudaGetLastError();
 }
 
 }  // namespace pisco

@@ -239,9 +239,18 @@ void launch_plans(const FwdArgs& a, tuned::SamplePlan* plans, long long pos0, lo
 // accepts (fwd_exact.cu); plans as launch_forward_tuned's.
 cudaError_t launch_forward_exact(const FwdArgs& a, bool f64, int sm_count, cudaStream_t st,
                                  void* plans, long long plan_cap);
-// Same kernel with every FP32 decision also evaluated in FP64: writes the
-// worst |FP32 - FP64| / margin seen over the non-fallback pairs to *calib.
-cudaError_t launch_tuned_calibrate(const FwdArgs& a, int sm_count, cudaStream_t st, float* calib);
+// What a checking run finds (tuned_core.cuh Check; the errors as the bits of
+// floats).
+struct CheckOut {
+    int fp32, fp64;
+    unsigned long long pairs, differ;
+};
+// The forms' kernels with the nearest lookup, every decision compared with the
+// chain's (the TOD is written as well where the outputs are not null); *check
+// is added to.
+cudaError_t launch_tuned_check(const FwdArgs& a, int sm_count, cudaStream_t st, CheckOut* check);
+cudaError_t launch_exact_check(const FwdArgs& a, bool f64, int sm_count, cudaStream_t st,
+                               CheckOut* check);
 // Sky order of n < 2^31 samples (order.cu).  With tmp == NULL stores the
 // temporary bytes the sort needs in *tmp_bytes and does nothing else;
 // otherwise writes order[0..n): the positions 0..n-1 sorted by the Z-order

@@ -305,6 +305,14 @@ struct Out {
     int f64;
 };
 
+// What a checking run (kCheck) finds, per lane: the worst error of an FP32
+// decision and of one that quick_pair takes, each in units of its margin; the
+// pairs visited, and those whose beam pixel is not the chain's.
+struct Check {
+    float fp32 = 0.0f, fp64 = 0.0f;
+    unsigned long long pairs = 0, differ = 0;
+};
+
 __device__ __forceinline__ void store_out(void* out, int f64, long long i, double v)
 {
     if (!out) return;
@@ -876,12 +884,17 @@ __device__ __forceinline__ bool stencil_f32(const Beam& B, int qd, float tp, flo
 // The beam pixel and exp(2i chi) of a pair in FP64 without the chain's
 // arccosines and the sines and cosines of its angles: one sine and cosine (of
 // the longitude offset) and one arctangent, some 200 FP64 instructions against
-// 700.  false (nothing computed) where the chain itself has to decide: within
+// 700.  false where the chain itself has to decide: within
 // 1e-4 rad of the boresight (its own rounding shows there, and its degenerate
 // branch lies at 1e-6), a frame near a pole, or a decision within 1e-9 of an
 // integer.
+struct QuickPair {
+    long long bp;
+    double c2, s2;
+    double av, bv, cv, ir, m;  // the decisions (CapPixel) and their margin
+};
 __device__ __forceinline__ bool quick_pair(const Hpx& hs, const Hpx& hb, const Pend& P, int pix,
-                                           long long& bp, double& c2, double& s2)
+                                           QuickPair& q)
 {
     if (P.plain) return false;
     double z, phi, s;
@@ -906,13 +919,46 @@ __device__ __forceinline__ bool quick_pair(const Hpx& hs, const Hpx& hb, const P
     const double m = 1e-9 * (r + 2.0);
     const double ea = av - fa, eb = bv - fb, ec = cv - fc;
     if (!(fmin(fmin(ea, eb), ec) > m && fmax(fmax(ea, eb), ec) < 1.0 - m)) return false;
-    bp = (long long)(2.0 * ir * (ir - 1.0) + qd * ir + fc);
+    q.bp = (long long)(2.0 * ir * (ir - 1.0) + qd * ir + fc);
+    q.av = av;
+    q.bv = bv;
+    q.cv = cv;
+    q.ir = ir;
+    q.m = m;
     // phasor's w, turned by psi
     const double wr = fma(db, X, nb * Y), wi = fma(nb, X, -(db * Y));
     const double rr = wr * wr, iw = 1.0 / fma(wi, wi, rr);
-    c2 = fma(-wi, wi, rr) * iw;
-    s2 = wr * wi * (iw + iw);
+    q.c2 = fma(-wi, wi, rr) * iw;
+    q.s2 = wr * wi * (iw + iw);
     return true;
+}
+
+// Compares a pair's decisions with the chain's: the FP32 ones (av, bv, cv of
+// ring ir, beam pixel bp) where the pair is not queued, and quick_pair's, which
+// a queued pair would take, for every pair that it accepts.  r: the pair's FP32
+// ring position (the FP32 margin is kMarginRel (r + 2)).
+static __device__ __noinline__ void check_pair(const Hpx& hs, const Hpx& hb, const Pend& P, int pix,
+                                               float av, float bv, float cv, int ir, float r, int bp,
+                                               bool queued, Check& ck)
+{
+    double rho, sig, chi;
+    const long long want = pair_beam_pixel(hs, hb, pix, P.ra, P.dec, P.psi, &rho, &sig, &chi);
+    const double tt = fmodulo(sig * kInvHalfPi, 4.0), tp = tt - floor(tt);
+    // nside sqrt(3 (1 - cos rho))
+    const double rd = (double)hb.nside * 2.4494897427831781 * sin(0.5 * rho);
+    auto worst = [&](double a, double b, double c, double ring) {
+        return fmax(fmax(fabs(a - tp * rd), fabs(b - (1.0 - tp) * rd)), fabs(c - tp * ring));
+    };
+    ++ck.pairs;
+    if (!queued) {
+        ck.fp32 = fmaxf(ck.fp32, (float)(worst(av, bv, cv, (double)ir) / (kMarginRel * (r + 2.0))));
+        ck.differ += bp != want;
+    }
+    QuickPair q;
+    if (quick_pair(hs, hb, P, pix, q)) {
+        ck.fp64 = fmaxf(ck.fp64, (float)(worst(q.av, q.bv, q.cv, q.ir) / q.m));
+        ck.differ += queued && q.bp != want;
+    }
 }
 
 // Redoes queued pair e of the warp whose state S is, in FP64: the beam pixel
@@ -925,13 +971,15 @@ __device__ __forceinline__ void redo(const Hpx& hs, const Smem& S, int e, unsign
     const Pend& P = S.p[S.qs[e]];
     const int pix = S.q[e];
     const Hpx hb = hpx_make(P.nside_beam);
-    double rho = 0.0, sig = 0.0, c2, s2;
-    long long bp = -1;
-    if (kBil || !quick_pair(hs, hb, P, pix, bp, c2, s2)) {
+    double rho = 0.0, sig = 0.0;
+    QuickPair q;
+    if (kBil || !quick_pair(hs, hb, P, pix, q)) {
         double chi;
-        bp = pair_beam_pixel(hs, hb, pix, P.ra, P.dec, P.psi, &rho, &sig, &chi);
-        sincos(2.0 * chi, &s2, &c2);
+        q.bp = pair_beam_pixel(hs, hb, pix, P.ra, P.dec, P.psi, &rho, &sig, &chi);
+        sincos(2.0 * chi, &q.s2, &q.c2);
     }
+    const long long bp = q.bp;
+    const double c2 = q.c2, s2 = q.s2;
     if constexpr (kBil && Action::kStencil) {
         int px[4];
         float w[4];
@@ -1226,9 +1274,14 @@ __device__ __forceinline__ Spot2 locate2(float kf, const Frame& F, const float4&
     p.r = pack2(__fmul_rn(p.q0, rsqrt_approx(p.q0)), __fmul_rn(p.q1, rsqrt_approx(p.q1)));
     return p;
 }
-__device__ __forceinline__ void cap_pixel2(const Spot2& p, int& bp0, int& bp1, bool& near0,
-                                           bool& near1)
+struct CapPixel2 {
+    F32x2 av, bv, cv;
+    int ir0, ir1, bp0, bp1;
+    bool near0, near1;
+};
+__device__ __forceinline__ CapPixel2 cap_pixel2(const Spot2& p)
 {
+    CapPixel2 c;
     const F32x2 k23 = both(kTwo23), khalf = both(8388607.5f);
     // (products that sums take are scalar: ptxas fuses a packed product into
     // a packed sum, which the scalar form does not)
@@ -1242,12 +1295,16 @@ __device__ __forceinline__ void cap_pixel2(const Spot2& p, int& bp0, int& bp1, b
     const F32x2 tc = add2_rd(cv, k23);
     const F32x2 fc = sub2(cv, sub2(tc, khalf));
     const F32x2 edge = fma2(p.r, both(-kMarginRel), both(0.5f - 2.0f * kMarginRel));
-    near0 = fmaxf(fmaxf(fabsf(lo2(fa)), fabsf(lo2(fb))), fabsf(lo2(fc))) > lo2(edge);
-    near1 = fmaxf(fmaxf(fabsf(hi2(fa)), fabsf(hi2(fb))), fabsf(hi2(fc))) > hi2(edge);
-    const int i0 = (__float_as_int(lo2(ta)) - kTwo23Bits) + (__float_as_int(lo2(tb)) - kTwo23Bits) + 1;
-    const int i1 = (__float_as_int(hi2(ta)) - kTwo23Bits) + (__float_as_int(hi2(tb)) - kTwo23Bits) + 1;
-    bp0 = i0 * (2 * i0 - 2 + p.qd0) + (__float_as_int(lo2(tc)) - kTwo23Bits);
-    bp1 = i1 * (2 * i1 - 2 + p.qd1) + (__float_as_int(hi2(tc)) - kTwo23Bits);
+    c.near0 = fmaxf(fmaxf(fabsf(lo2(fa)), fabsf(lo2(fb))), fabsf(lo2(fc))) > lo2(edge);
+    c.near1 = fmaxf(fmaxf(fabsf(hi2(fa)), fabsf(hi2(fb))), fabsf(hi2(fc))) > hi2(edge);
+    c.ir0 = (__float_as_int(lo2(ta)) - kTwo23Bits) + (__float_as_int(lo2(tb)) - kTwo23Bits) + 1;
+    c.ir1 = (__float_as_int(hi2(ta)) - kTwo23Bits) + (__float_as_int(hi2(tb)) - kTwo23Bits) + 1;
+    c.bp0 = c.ir0 * (2 * c.ir0 - 2 + p.qd0) + (__float_as_int(lo2(tc)) - kTwo23Bits);
+    c.bp1 = c.ir1 * (2 * c.ir1 - 2 + p.qd1) + (__float_as_int(hi2(tc)) - kTwo23Bits);
+    c.av = av;
+    c.bv = bv;
+    c.cv = cv;
+    return c;
 }
 // (the signs of wr and of its factors are turned around: no packed negation)
 __device__ __forceinline__ void phasor2(const Spot2& p, float s0, float Wz, float Di, F32x2& c2,
@@ -1491,22 +1548,21 @@ __device__ __forceinline__ SamplePlan make_plan(const Hpx& hs, const Beam& B, do
 // Processes one sample from its plan.  A non-finite pointing gives NaN TOD
 // (kSums) and no pairs.  With kSums the TOD is written to `o` now, or by the
 // drain that redoes the sample's last queued pair.  nfall counts queued pairs
-// and npairs the disc pairs (lane 0 only); cmax (kCalib) is the worst FP32
-// decision error over the non-queued pairs, in units of the margin.  kBil:
-// bilinear beam lookup (bilinear_f32; only the degenerate pairs are queued).
-template <bool kCalib, bool kBil = false, class Smem, class Action>
+// (lane 0 only).  kCheck: the pairs' decisions are compared with the chain's
+// (ck).  kBil: bilinear beam lookup (bilinear_f32; only the degenerate pairs are
+// queued).
+template <bool kCheck, bool kBil = false, class Smem, class Action>
 __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& hs,
                                                const RingT* rings, const Hpx& hb, const Beam& B,
                                                double ra, double dec, double pa, const Out& o,
                                                Smem& S, Queue& Qs, int lane,
                                                unsigned int* err, Action& act,
-                                               unsigned long long& nfall, float& cmax,
-                                               unsigned long long& npairs)
+                                               unsigned long long& nfall, Check& ck)
 {
     RingC* W = S.r;
     const unsigned lt_mask = (1u << lane) - 1u, le_mask = 2u * lt_mask + 1u;
     // two pixels per lane (actions with pair2, nearest lookup)
-    constexpr bool kUnits = HasPair2<Action>::value && !kBil && !kCalib;
+    constexpr bool kUnits = HasPair2<Action>::value && !kBil;
     if (SP.flags & kPlanBad) {
         if (Action::kSums && lane == 0) {
             store_out(o.a, o.f64, o.idx, CUDART_NAN);
@@ -1651,18 +1707,12 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
             }
         }
         int incl = items;
-        int all = cnt;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(kFull, incl, o);
             if (lane >= o) incl += v;
         }
         const int total = __shfl_sync(kFull, incl, 31);
-        if (kCalib) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(kFull, all, o);
-            if (lane == 0) npairs += (unsigned long long)all;
-        }
         // the rings with pixels, packed in order: a lane's ring is then the
         // number of ring starts up to its slot, counted with one warp
         // reduction per iteration instead of a search through shared memory
@@ -1696,24 +1746,35 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 const bool v0 = t < total && j >= (R3.z & 0xffff);
                 const bool v1 = t < total && j < (int)((unsigned)R3.z >> 16);
                 const Spot2 p = locate2(kf, F, R0, R1.y, narrow);
-                int bp0, bp1;
-                bool near0, near1;
-                cap_pixel2(p, bp0, bp1, near0, near1);
-                const bool fb0 = v0 && (near0 || p.q0 < tiny);
-                const bool fb1 = v1 && (near1 || p.q1 < tiny);
-                const bool in0 = v0 && !fb0 && (unsigned)bp0 < npix_beam;
-                const bool in1 = v1 && !fb1 && (unsigned)bp1 < npix_beam;
+                const CapPixel2 c = cap_pixel2(p);
+                const bool fb0 = v0 && (c.near0 || p.q0 < tiny);
+                const bool fb1 = v1 && (c.near1 || p.q1 < tiny);
+                if constexpr (kCheck) {
+                    const Pend& P = S.p[slot];
+                    if (v0)
+                        check_pair(hs, hb, P, pix, lo2(c.av), lo2(c.bv), lo2(c.cv), c.ir0, lo2(p.r),
+                                   c.bp0, fb0, ck);
+                    if (v1)
+                        check_pair(hs, hb, P, pix + 1, hi2(c.av), hi2(c.bv), hi2(c.cv), c.ir1,
+                                   hi2(p.r), c.bp1, fb1, ck);
+                }
+                const bool in0 = v0 && !fb0 && (unsigned)c.bp0 < npix_beam;
+                const bool in1 = v1 && !fb1 && (unsigned)c.bp1 < npix_beam;
                 Unit U;
                 U.in0 = in0;
                 U.in1 = in1;
                 U.pix = pix;
-                U.bp0 = in0 ? bp0 : 0;
-                U.bp1 = in1 ? bp1 : 0;
+                U.bp0 = in0 ? c.bp0 : 0;
+                U.bp1 = in1 ? c.bp1 : 0;
                 U.B0 = load_beam<Action::kL1>(beam + U.bp0);
                 U.B1 = load_beam<Action::kL1>(beam + U.bp1);
                 act.fetch2(pix, U.S0, U.S1);
                 phasor2(p, F.s0, R1.x, R1.y, U.c, U.s);
                 act.pair2(U);
+                if constexpr (HasOutside<Action>::value) {
+                    if (v0 && !fb0 && !in0) act.outside(pix, c.bp0);
+                    if (v1 && !fb1 && !in1) act.outside(pix + 1, c.bp1);
+                }
                 if (__any_sync(kFull, fb0 || fb1)) {
 #pragma unroll 1
                     for (int e = 0; e < 2; ++e) queue(e ? fb1 : fb0, pix + e);
@@ -1754,17 +1815,8 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 } else {
                     const CapPixel c = cap_pixel(p);
                     fb |= c.near;
-                    if (kCalib && !fb) {
-                        double rho, sig, chi;
-                        (void)pair_beam_pixel(hs, hb, pix, ra, dec, -pa, &rho, &sig, &chi);
-                        const double tt = fmodulo(sig * kInvHalfPi, 4.0);
-                        const double tpd = tt - floor(tt);
-                        const double rd = (double)B.nside * sqrt(3.0 * (1.0 - cos(rho)));
-                        const double e1 = fabs(c.av - tpd * rd) / (p.r + 1.0);
-                        const double e2 = fabs(c.bv - (1.0 - tpd) * rd) / (p.r + 1.0);
-                        const double e3 = fabs(c.cv - tpd * (double)c.ir) / ((double)c.ir + 1.0);
-                        cmax = fmaxf(cmax, (float)fmax(fmax(e1, e2), e3) / kMarginRel);
-                    }
+                    if constexpr (kCheck)
+                        check_pair(hs, hb, S.p[slot], pix, c.av, c.bv, c.cv, c.ir, p.r, c.bp, fb, ck);
                     if (!fb) {
                         if constexpr (IsExact<Action>::value) {
                             if ((unsigned)c.bp < (unsigned)B.npix) {
@@ -1817,15 +1869,25 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
 }
 
 // Processes one sample, its plan built here by the warp.
-template <bool kCalib, bool kBil = false, class Smem, class Action>
+template <bool kCheck, bool kBil = false, class Smem, class Action>
 __device__ __forceinline__ void sample(const Hpx& hs, const RingT* rings, const Hpx& hb,
                                        const Beam& B, double ra, double dec, double pa,
                                        const Out& o, Smem& S, Queue& Qs, int lane,
                                        unsigned int* err, Action& act, unsigned long long& nfall,
-                                       float& cmax, unsigned long long& npairs)
+                                       Check& ck)
 {
-    sample_planned<kCalib, kBil>(make_plan(hs, B, ra, dec, pa), hs, rings, hb, B, ra, dec, pa, o,
-                                 S, Qs, lane, err, act, nfall, cmax, npairs);
+    sample_planned<kCheck, kBil>(make_plan(hs, B, ra, dec, pa), hs, rings, hb, B, ra, dec, pa, o,
+                                 S, Qs, lane, err, act, nfall, ck);
+}
+
+// Adds a lane's findings to *out (every lane of the warp calls).
+__device__ __forceinline__ void report(const Check& ck, CheckOut* out)
+{
+    // both errors are >= 0, so their bits order as they do
+    atomicMax(&out->fp32, __float_as_int(ck.fp32));
+    atomicMax(&out->fp64, __float_as_int(ck.fp64));
+    atomicAdd(&out->pairs, ck.pairs);
+    atomicAdd(&out->differ, ck.differ);
 }
 
 // Forward action: gather the sky, multiply by the beam, compensated sums of
