@@ -1410,22 +1410,32 @@ __device__ __forceinline__ RingF ring_two_float(float near, float f, float e, co
 // exp(2i chi) rounded to FP32: its error before that rounding, some 1e-12 at
 // rho of a degree, is far below what moves the rounded value.  About 260 FP32
 // instructions, the time of four FP64 ones; the 45 FP64 instructions of
-// phasor_exact took two thirds of a PLAIN launch.  narrow: |x| <= 1/2, where the
-// series' FP32 terms leave 2e-10 of sin x (8e-12 at 1/8).
-__device__ __forceinline__ void phasor_two_float(const RingF& R, float kf, bool narrow, FF s0,
-                                                 FF c2p, FF s2p, float& c2, float& s2)
+// phasor_exact took two thirds of a PLAIN launch.  Within 1/8 rad (narrow) and
+// within 1/2 (middle) sin x and 1 - cos x are good to 4e-13, by one series whose
+// third term takes a second float in the middle range (with one it left 1e-10
+// there); beyond, FP64's sincos (20,000 samples at 60 to 74 degrees, 5 degree
+// beam: 145 us with one float, 147 with two, 350 with sincos from 1/8 on).
+__device__ __forceinline__ void phasor_two_float(const RingF& R, float kf, bool narrow, bool middle,
+                                                 FF s0, FF c2p, FF s2p, float& c2, float& s2)
 {
     const FF x = kf * R.dphi + R.dc;
     FF sn, h;
-    if (narrow) {
+    if (narrow || middle) {
         const FF x2 = x * x;
-        // sin x = x + x (x2 (-1/6 + x2 p)), 1 - cos x = x2 (1/2 + x2 (-1/24 + x2 q))
-        const float p = fmaf(x2.h, fmaf(x2.h, fmaf(x2.h, -2.50521084e-8f, 2.75573192e-6f),
-                                        -1.98412698e-4f), 8.33333333e-3f);
-        const float q = fmaf(x2.h, fmaf(x2.h, fmaf(x2.h, -2.08767570e-9f, 2.75573192e-7f),
-                                        -2.48015873e-5f), 1.38888889e-3f);
-        const FF a = ff_quick(-0.16666667f, fmaf(x2.h, p, 4.9670537e-9f));
-        const FF b = ff_quick(-0.041666668f, fmaf(x2.h, q, 1.2417634e-9f));
+        // sin x = x + x (x2 (-1/6 + x2 (1/120 + x2 p)))
+        // 1 - cos x = x2 (1/2 + x2 (-1/24 + x2 (1/720 + x2 q)))
+        const float p = fmaf(x2.h, fmaf(x2.h, -2.50521084e-8f, 2.75573192e-6f), -1.98412698e-4f);
+        const float q = fmaf(x2.h, fmaf(x2.h, -2.08767570e-9f, 2.75573192e-7f), -2.48015873e-5f);
+        FF a, b;
+        if (narrow) {
+            a = ff_quick(-0.16666667f, fmaf(x2.h, fmaf(x2.h, p, 8.33333333e-3f), 4.9670537e-9f));
+            b = ff_quick(-0.041666668f, fmaf(x2.h, fmaf(x2.h, q, 1.38888889e-3f), 1.2417634e-9f));
+        } else {
+            a = FF{-0.16666667f, 4.9670537e-9f} +
+                x2 * ff_quick(8.33333377e-3f, fmaf(x2.h, p, -4.346172e-10f));
+            b = FF{-0.041666668f, 1.2417634e-9f} +
+                x2 * ff_quick(1.38888892e-3f, fmaf(x2.h, q, -3.3631094e-11f));
+        }
         sn = x + x * (x2 * a);
         h = x2 * (FF{0.5f, 0.0f} + x2 * b);
     } else {
@@ -1649,6 +1659,7 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
         const int ring = r0 + lane;
         int cnt = 0, items = 0;  // the ring's disc pixels; its lane slots
         bool wide = false;
+        [[maybe_unused]] bool beyond = false;
         RingC rc;
         [[maybe_unused]] std::conditional_t<IsTwoFloat<Action>::value, RingF, RingD> rd;
         if (ring <= PL.full_hi) {
@@ -1703,7 +1714,7 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                 // (the anchor is within half a pixel of the boresight's longitude)
                 const float far = ((float)max(-kk, kk + cnt - 1) + 0.5f) * rt.dphi;
                 wide = far > kShortOffset;
-                if constexpr (IsTwoFloat<Action>::value) wide = far > 0.5f;
+                beyond = far > 0.5f;
             }
         }
         int incl = items;
@@ -1725,6 +1736,8 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
             if constexpr (IsExact<Action>::value) S.rd[__popc(some & lt_mask)] = rd;
         }
         const bool narrow = !__any_sync(kFull, wide);
+        [[maybe_unused]] bool middle = false;
+        if constexpr (IsTwoFloat<Action>::value) middle = !__any_sync(kFull, beyond);
         __syncwarp();
         int k0 = -1;  // ring of the slot before this iteration's
         const int iters = (total + 31) >> 5;
@@ -1822,7 +1835,7 @@ __device__ __forceinline__ void sample_planned(const SamplePlan& SP, const Hpx& 
                             if ((unsigned)c.bp < (unsigned)B.npix) {
                                 if constexpr (IsTwoFloat<Action>::value) {
                                     float c2, s2;
-                                    phasor_two_float(S.rd[k], kf, narrow, S.s0, S.c2p, S.s2p, c2, s2);
+                                    phasor_two_float(S.rd[k], kf, narrow, middle, S.s0, S.c2p, S.s2p, c2, s2);
                                     act.pair64(pix, c.bp, c2, s2);
                                 } else {
                                     double c2, s2;

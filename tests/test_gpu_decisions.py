@@ -26,7 +26,7 @@ def convolver(nside, nside_beam, radius, decs, n, seed=11):
     return conv
 
 
-@pytest.mark.parametrize("form", ["tuned", "fp64"])
+@pytest.mark.parametrize("form", ["tuned", "fp64", "plain"])
 @pytest.mark.parametrize("shape", SHAPES, ids=str)
 def test_decisions_are_the_chains(gpu, shape, form):
     conv = convolver(*shape)
