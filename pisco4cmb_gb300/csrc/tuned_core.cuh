@@ -884,10 +884,11 @@ __device__ __forceinline__ bool stencil_f32(const Beam& B, int qd, float tp, flo
 // The beam pixel and exp(2i chi) of a pair in FP64 without the chain's
 // arccosines and the sines and cosines of its angles: one sine and cosine (of
 // the longitude offset) and one arctangent, some 200 FP64 instructions against
-// 700.  false where the chain itself has to decide: within
-// 1e-4 rad of the boresight (its own rounding shows there, and its degenerate
-// branch lies at 1e-6), a frame near a pole, or a decision within 1e-9 of an
-// integer.
+// 700.  false where the chain itself has to decide: within 1e-3 rad of the
+// boresight, a frame near a pole, or a decision within the margin of an integer.
+// The chain takes rho as acos(cos rho), which moves it by some 1e-16 / rho and a
+// decision by nside_b times as much: on a beam grid of nside 8192 up to 7.6
+// margins at 1e-4 rad, 0.22 from 1e-3 on.  (Its degenerate branch lies at 1e-6.)
 struct QuickPair {
     long long bp;
     double c2, s2;
@@ -906,7 +907,7 @@ __device__ __forceinline__ bool quick_pair(const Hpx& hs, const Hpx& hb, const P
     const double u = s * sd, v = z * P.s0 - s * P.z0 * cd;
     const double nb = P.s0 * sd, db = s * P.z0 - z * P.s0 * cd;
     const double sin2 = fma(u, u, v * v);
-    if (!(sin2 > 1e-8)) return false;
+    if (!(sin2 > 1e-6)) return false;
     // r = nside sqrt(3 (1 - cos rho)), 1 - cos rho = sin^2 rho / (1 + cos rho)
     const double r = (double)hb.nside * sqrt(3.0 * sin2 / (1.0 + z * P.z0 + s * P.s0 * cd));
     const double X = u * P.spsi - v * P.cpsi, Y = u * P.cpsi + v * P.spsi;
