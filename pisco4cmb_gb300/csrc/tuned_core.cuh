@@ -1916,13 +1916,17 @@ struct Gather {
     F32x2 sum, cmp;  // halves: detector a, detector b
     __device__ __forceinline__ void reset() { sum = cmp = pack2(0.0f, 0.0f); }
     __device__ __forceinline__ float4 fetch(int pix) const { return __ldg(&sky[pix]); }
-    // the sky's polarisation turned into the beam's frame once for both detectors
+    // the sky's polarisation turned into the beam's frame once for both detectors;
+    // I, mostly the largest, comes last, so that a pair is rounded once at its
+    // magnitude: with I of 100 and Q, U of 10 at nside 64 and 5 degrees the totals
+    // are off by 6.9e-9 of the TOD's spread, with I first 1.15e-8, for 0.3 % of
+    // the time (400,000 samples at nside 1024: 16.63 -> 16.68 ms)
     __device__ __forceinline__ static void contrib(const float4& S, const F8& B, float c2, float s2,
                                                   float& ta, float& tb)
     {
         const float q = fmaf(S.y, c2, S.z * s2), u = fmaf(S.z, c2, -(S.y * s2));
-        ta = fmaf(u, B.a.z, fmaf(q, B.a.y, fmaf(S.w, B.a.w, S.x * B.a.x)));
-        tb = fmaf(-u, B.b.z, fmaf(-q, B.b.y, fmaf(S.w, B.b.w, S.x * B.b.x)));
+        ta = fmaf(S.x, B.a.x, fmaf(q, B.a.y, fmaf(u, B.a.z, S.w * B.a.w)));
+        tb = fmaf(S.x, B.b.x, fmaf(-q, B.b.y, fmaf(-u, B.b.z, S.w * B.b.w)));
     }
     __device__ __forceinline__ void pair(int, const float4& S, const F8& B, int, float c2, float s2)
     {
