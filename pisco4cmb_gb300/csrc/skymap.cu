@@ -127,17 +127,20 @@ __device__ __forceinline__ void split(double x, float& h, float& l)
 //
 // The error: sin(dec) is good to 1.2e-7, the positions (at most nside in the
 // caps, 3/4 nside from the equator) to nside (0.75 x 1.2e-7 + 2^-24) or, in the
-// caps, nside (3e-7 + 2^-24); the margin is 5e-7 nside + 1e-6.
+// caps, nside (3e-7 + 2^-24): 1.2e-7 and 2.9e-7 nside at worst of 3 million each;
+// the margin is 5e-7 nside + 1e-6.
 template <class T>
 __device__ __forceinline__ int quick_ang2pix(int ns, T ra, T dec)
 {
     float rh, rl, dh, dl;
     split(ra, rh, rl);
     split(dec, dh, dl);
-    // quarter turns mod 4, tt + tl: ra 2 / pi with the product's rounding error
-    const float th = __fmul_rn(rh, 0.63661975f);
-    const float tl = fmaf(rl, 0.63661975f, fmaf(rh, 2.5682e-8f, fmaf(rh, 0.63661975f, -th)));
-    const float tt = fmaf(-4.0f, floorf(0.25f * th), th);
+    // quarter turns mod 4, tt + tl: ra 2 / pi with the product's rounding error,
+    // and that of th + turns (th in (-2, 0); elsewhere the sum is exact)
+    const float th = __fmul_rn(rh, 0.63661975f), turns = -4.0f * floorf(0.25f * th);
+    const float tt = __fadd_rn(th, turns);
+    const float tl = fmaf(rl, 0.63661975f, fmaf(rh, 2.56825533e-8f, fmaf(rh, 0.63661975f, -th))) +
+                     __fsub_rn(th, __fsub_rn(tt, turns));
     const float n = (float)ns, m = fmaf(n, 5e-7f, 1e-6f);
     const float z = sinf(dh);
     auto near = [&](float f) { return f < m || f > 1.0f - m; };
