@@ -172,10 +172,7 @@ __global__ void ring_table_kernel(int nside, RingT* rings)
     }
 }
 
-// A short launch's warps per block, and its blocks per SM.
-template <bool kBil>
-constexpr int kShortWarps = kBil ? PISCO_BIL_WARPS : PISCO_FWD_WARPS / 2;
-constexpr int kShortBlocks = 2;
+constexpr int kShortBlocks = 2;  // a short launch's blocks per SM
 
 }  // namespace
 
@@ -229,20 +226,28 @@ void launch_shape(const FwdArgs& a, int sm_count, cudaStream_t st, CheckOut* che
 
 // kTW: the planned launch's block.  A short launch (tuned_plans_itself: at most
 // 64 samples per SM, 32 to a block) gives two blocks per SM an equal share of
-// the samples each, and plans in the block.  2,003 samples of nside 1024 and 3
-// degrees: 184 us in full 20-warp blocks with plan_kernel before them, 155 in
-// full blocks of 8 that plan themselves, which leave a third of the SMs with
-// half the work of the others, 151 with equal shares of 10 warps (20 per SM);
-// 3,040 samples 184, 229 and 181 us; 4,000 samples 314, 257 and 261; 6,000
-// samples 317, 350 and 309; 7,000 samples 445, 362 and 387.  Without plans the warps build their own (FP64 disc
-// plan in the loop's registers).
+// the samples each, and plans in the block (2,003 samples of nside 1024 and 3
+// degrees spent 11 us of 178 in plan_kernel and 3 between the launches).  Its
+// blocks have 10 warps, all that fit at 96 registers, where that takes fewer
+// rounds over a block's samples than 8, or both take one; otherwise 8, which
+// have 128 registers and share L1 among fewer.  Times of 10 and 8 warps in us
+// (nside 1024, 3 degrees, cold caches; 304 blocks): 2,003 samples 170 and 167,
+// 3,040 193 and 254, 4,000 273 and 274, 6,080 324 and 364, 7,000 401 and 385,
+// 9,120 452 and 489, 9,728 519 and 494; nside 2048, 1 degree: 4,864 194 and 184,
+// 7,296 268 and 234, 9,728 335 and 285.  The bilinear lookup has 8.  Without
+// plans the warps build their own (FP64 disc plan in the loop's registers).
 template <bool kBil, int kTW>
 void launch_lookup(const FwdArgs& a, int sm_count, cudaStream_t st, tuned::SamplePlan* plans,
                    long long plan_cap)
 {
     constexpr int kUnplanned = kTW > 16 ? 16 : kTW;
-    if (tuned_plans_itself(a.n, sm_count))
-        launch_shape<false, kBil, kShortWarps<kBil>, kBlockPlans>(a, sm_count, st, nullptr, nullptr, 0);
+    constexpr int kFew = 8, kMany = PISCO_FWD_WARPS / 2;
+    const long long share = (a.n + kShortBlocks * sm_count - 1) / (kShortBlocks * sm_count);
+    const bool many = share <= kFew || (share + kMany - 1) / kMany < (share + kFew - 1) / kFew;
+    if (tuned_plans_itself(a.n, sm_count) && !kBil && many)
+        launch_shape<false, kBil, kMany, kBlockPlans>(a, sm_count, st, nullptr, nullptr, 0);
+    else if (tuned_plans_itself(a.n, sm_count))
+        launch_shape<false, kBil, kFew, kBlockPlans>(a, sm_count, st, nullptr, nullptr, 0);
     else if (plans && plan_cap > 0)
         launch_shape<false, kBil, kTW, kArrayPlans>(a, sm_count, st, nullptr, plans, plan_cap);
     else
