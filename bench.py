@@ -355,14 +355,14 @@ def run_gpu_arm(args, rank, world, local):
     torch.cuda.synchronize()
     plain_sps = m_plain / (e0.elapsed_time(e1) / 1e3)
 
-    # accuracy of TUNED vs FP64 on a bounded prefix (untimed)
+    # accuracy of TUNED vs the FP64 chain on a bounded prefix (untimed)
     m_acc = min(n, args.accuracy_samples)
     ta = torch.empty(m_acc, dtype=torch.float64, device=dev)
     tb = torch.empty(m_acc, dtype=torch.float64, device=dev)
     fa = torch.empty(m_acc, dtype=torch.float64, device=dev)
     fb = torch.empty(m_acc, dtype=torch.float64, device=dev)
     conv.forward_device(ta.data_ptr(), tb.data_ptr(), out_f64=True, n=m_acc, form="tuned")
-    conv.forward_device(fa.data_ptr(), fb.data_ptr(), out_f64=True, n=m_acc, form="fp64")
+    conv.debug_forward_chain(fa.data_ptr(), fb.data_ptr(), n=m_acc)
     conv.sync()
     rms = torch.sqrt(torch.mean(torch.cat([fa, fb]) ** 2)).item()
     err = torch.cat([ta - fa, tb - fb])
@@ -565,6 +565,10 @@ def run_c3_precision(args):
     e1.record()
     torch.cuda.synchronize()
     t_fp64 = e0.elapsed_time(e1) / 1e3
+    fp64 = [x.cpu().numpy() for x in ref]
+    # the reference of both forms: the chain, which shares nothing with them
+    conv.debug_forward_chain(ref[0].data_ptr(), ref[1].data_ptr(), n=m, stream=cs)
+    conv.sync()
     ref = [x.cpu().numpy() for x in ref]
     rms = float(np.sqrt(np.mean(np.concatenate(ref) ** 2)))
     err = np.concatenate([tuned[0][:m] - ref[0], tuned[1][:m] - ref[1]])
@@ -578,7 +582,7 @@ def run_c3_precision(args):
                                  sky.astype(np.float64), w["nside_beam"], ba.astype(np.float64),
                                  bb.astype(np.float64), nthreads=host_cores())
     errc = np.concatenate([tuned[0][:mc] - oa, tuned[1][:mc] - ob])
-    errf = np.concatenate([ref[0][:mc] - oa, ref[1][:mc] - ob])
+    errf = np.concatenate([fp64[0][:mc] - oa, fp64[1][:mc] - ob])
     line = {"workload": "c3_precision_nside2048_beam1deg", "nsamples": n, "pairs": pairs,
             "tuned_samples_per_s": n / t_tuned, "fp64_gpu_samples_per_s": m / t_fp64,
             "tuned_sky_order": {"samples_per_s": n / t_sky, "over_scan_order": t_tuned / t_sky,

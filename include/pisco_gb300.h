@@ -179,6 +179,13 @@ typedef struct pisco_decision_check {
 } pisco_decision_check;
 pisco_status pisco_debug_decisions(pisco_ctx* ctx, pisco_form form, long begin, long n,
                                    pisco_decision_check* out);
+/* pisco_forward_device on the reference's per-pair chain itself, in PLAIN's or
+ * FP64's arithmetic: what the forward runs with the bilinear lookup and for beams
+ * outside the TUNED domain, here for every lookup and beam.  With the nearest
+ * lookup it shares neither disc nor decisions with the forms. */
+pisco_status pisco_debug_forward_chain(pisco_ctx* ctx, pisco_form form, long begin, long n,
+                                       void* d_tod_a, void* d_tod_b, pisco_dtype out_dtype,
+                                       void* stream);
 
 /* ---- per-pair record of a form's decisions (diagnostic; no reference
  *      counterpart as an entry point -- the reference checks the same
@@ -206,9 +213,10 @@ typedef struct pisco_pair_dump {
 #define PISCO_PAIR_OUTSIDE_BEAM 2 /* beam pixel (every stencil pixel) beyond the
                                      stored map: the pair adds nothing */
 /* Runs the per-sample body of `form` (with the context's beam lookup; PLAIN
- * and FP64: the reference's chain) over samples [begin, begin+n) of the
- * current scan and records every (sample,
- * disc pixel) pair it visits: each sample's pairs appear together, in no
+ * and FP64: the reference's chain, which their forward runs with the bilinear
+ * lookup; with the nearest one pisco_debug_decisions holds what it decides
+ * against the chain) over samples [begin, begin+n) of the current scan and
+ * records every (sample, disc pixel) pair it visits: each sample's pairs appear together, in no
  * particular order within the sample.  *npairs = the number of disc pairs of
  * the range (HEALPix query_disc).  out == NULL only sizes the record;
  * out->capacity below *npairs is PISCO_ERR_INVALID_ARGUMENT.  Synchronous;

@@ -133,6 +133,7 @@ SIGNATURES = [
     ("pisco_tuned_calibrate", _S, [_P, _L, _L, ctypes.POINTER(ctypes.c_double),
                                    ctypes.POINTER(ctypes.c_longlong)]),
     ("pisco_debug_decisions", _S, [_P, _I, _L, _L, ctypes.POINTER(DecisionCheck)]),
+    ("pisco_debug_forward_chain", _S, [_P, _I, _L, _L, _P, _P, _I, _P]),
     ("pisco_debug_pairs", _S, [_P, _I, _L, _L, ctypes.POINTER(PairDump),
                                ctypes.POINTER(ctypes.c_longlong)]),
     ("pisco_hpx_pix2ang_device", _S, [_I, ctypes.c_longlong, _P, _P, _P, _P]),

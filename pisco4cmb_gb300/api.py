@@ -509,6 +509,14 @@ class GPUConvolver:
                                            ctypes.byref(out)), self.ctx, "debug_decisions")
         return out
 
+    def debug_forward_chain(self, d_a: int, d_b: int, out_f64: bool = True, begin: int = 0,
+                            n: int | None = None, stream: int = 0, form: str = "fp64") -> None:
+        """forward_device on the reference's chain itself (form: "plain" or "fp64")."""
+        n = self._n - begin if n is None else n
+        check(load().pisco_debug_forward_chain(self.ctx, FORMS[form], begin, n, d_a or None, d_b or None,
+                                               FLOAT64 if out_f64 else FLOAT32, stream or None),
+              self.ctx, "debug_forward_chain")
+
     def debug_pairs(self, form: str | None = None, begin: int = 0, n: int | None = None) -> dict:
         """Every (sample, disc pixel) pair the kernels of ``form`` visit over
         samples [begin, begin+n), with their decisions (pisco_debug_pairs):

@@ -259,6 +259,91 @@ pisco_status pisco_ctx::check_device()
     return PISCO_OK;
 }
 
+namespace {
+
+// A forward of samples [begin, begin + n) into device arrays; chain: PLAIN and
+// FP64 on the reference's chain whatever the lookup and the beam.
+pisco_status forward(pisco_ctx* c, pisco_form form, bool chain, long begin, long n, void* d_a,
+                     void* d_b, pisco_dtype out_dtype, void* stream)
+{
+    if (!c) return PISCO_ERR_INVALID_ARGUMENT;
+    if (!c->sky32 || !c->nside_sky) return fail(c, PISCO_ERR_NOT_READY, "no sky set");
+    if (!c->beam32 || !c->nside_beam) return fail(c, PISCO_ERR_NOT_READY, "no beam set");
+    if (c->nsamples < 0 || (!c->ra && c->nsamples > 0)) return fail(c, PISCO_ERR_NOT_READY, "no scan set");
+    if (begin < 0 || n < 0 || begin + n > c->nsamples)
+        return fail(c, PISCO_ERR_INVALID_ARGUMENT, "sample range outside the scan");
+    if (out_dtype != PISCO_FLOAT32 && out_dtype != PISCO_FLOAT64)
+        return fail(c, PISCO_ERR_INVALID_ARGUMENT, "bad output dtype");
+    if (form != PISCO_FORM_PLAIN && form != PISCO_FORM_TUNED && form != PISCO_FORM_FP64)
+        return fail(c, PISCO_ERR_INVALID_ARGUMENT, "bad form");
+    pisco_status st = c->activate();
+    if (st != PISCO_OK) return st;
+    cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
+    FwdArgs a{};
+    a.nside_sky = c->nside_sky;
+    a.sky32 = c->sky32;
+    a.rings = c->rings;
+    a.sky64 = nullptr;
+    a.nside_beam = c->nside_beam;
+    a.npix_beam = (int)c->npix_beam;
+    a.beam32 = c->beam32;
+    a.beam64 = nullptr;
+    a.rho_max = c->rho_max;
+    a.begin = begin;
+    a.n = n;
+    a.ra = c->ra;
+    a.dec = c->dec;
+    a.pa = c->pa;
+    a.out_a = d_a;
+    a.out_b = d_b;
+    st = c->range_order(begin, n, s, &a.order);
+    if (st != PISCO_OK) return st;
+    a.out_f64 = out_dtype == PISCO_FLOAT64;
+    a.interp = (int)c->interp;
+    a.err = c->d_err;
+    a.fallbacks = c->d_fallbacks;
+    cudaError_t e;
+    const bool tuned = tuned_supported(c->nside_beam, (int)c->npix_beam, c->rho_max);
+    // PLAIN and FP64 with the nearest lookup walk the TUNED geometry's pairs
+    // (fwd_exact.cu); the bilinear lookup, and beams outside that geometry's
+    // domain (reaching beyond the polar cap of their grid), take the chain
+    const bool exact = tuned && !chain && c->interp == PISCO_BEAM_NEAREST;
+    void* plans = nullptr;
+    long long plan_cap = 0;
+    if (form == PISCO_FORM_FP64) {
+        st = wide_maps(c, s, a);
+        if (st != PISCO_OK) return st;
+        if (exact) {
+            c->plan_scratch(n, s, &plans, &plan_cap);
+            e = launch_forward_exact(a, true, c->sm_count, s, plans, plan_cap);
+        } else {
+            e = launch_forward_plain(a, true, c->sm_count, s);
+        }
+    } else if (form == PISCO_FORM_TUNED && tuned) {
+        CK(cudaMemsetAsync(c->d_fallbacks, 0, sizeof(unsigned long long), s), "reset fallbacks");
+        if (!tuned_plans_itself(n, c->sm_count)) c->plan_scratch(n, s, &plans, &plan_cap);
+        e = launch_forward_tuned(a, c->sm_count, s, plans, plan_cap);
+    } else if (exact) {
+        c->plan_scratch(n, s, &plans, &plan_cap);
+        e = launch_forward_exact(a, false, c->sm_count, s, plans, plan_cap);
+    } else {
+        e = launch_forward_plain(a, false, c->sm_count, s);
+    }
+    if (plans) c->plans_used(s);
+    if (a.order) c->order_used(s);
+    if (e != cudaSuccess) return cuda_fail(c, e, "forward launch");
+    if (s != c->stream) {
+        cudaEvent_t ev;
+        CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
+        cudaEventRecord(ev, s);
+        cudaStreamWaitEvent(c->stream, ev, 0);
+        cudaEventDestroy(ev);
+    }
+    return PISCO_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 int pisco_abi_version(void) { return PISCO_ABI_VERSION; }
@@ -614,80 +699,15 @@ pisco_status pisco_set_scan_device(pisco_ctx* c, long n, const double* d_ra, con
 pisco_status pisco_forward_device(pisco_ctx* c, pisco_form form, long begin, long n, void* d_a,
                                   void* d_b, pisco_dtype out_dtype, void* stream)
 {
+    return forward(c, form, false, begin, n, d_a, d_b, out_dtype, stream);
+}
+
+pisco_status pisco_debug_forward_chain(pisco_ctx* c, pisco_form form, long begin, long n, void* d_a,
+                                       void* d_b, pisco_dtype out_dtype, void* stream)
+{
     if (!c) return PISCO_ERR_INVALID_ARGUMENT;
-    if (!c->sky32 || !c->nside_sky) return fail(c, PISCO_ERR_NOT_READY, "no sky set");
-    if (!c->beam32 || !c->nside_beam) return fail(c, PISCO_ERR_NOT_READY, "no beam set");
-    if (c->nsamples < 0 || (!c->ra && c->nsamples > 0)) return fail(c, PISCO_ERR_NOT_READY, "no scan set");
-    if (begin < 0 || n < 0 || begin + n > c->nsamples)
-        return fail(c, PISCO_ERR_INVALID_ARGUMENT, "sample range outside the scan");
-    if (out_dtype != PISCO_FLOAT32 && out_dtype != PISCO_FLOAT64)
-        return fail(c, PISCO_ERR_INVALID_ARGUMENT, "bad output dtype");
-    if (form != PISCO_FORM_PLAIN && form != PISCO_FORM_TUNED && form != PISCO_FORM_FP64)
-        return fail(c, PISCO_ERR_INVALID_ARGUMENT, "bad form");
-    pisco_status st = c->activate();
-    if (st != PISCO_OK) return st;
-    cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
-    FwdArgs a{};
-    a.nside_sky = c->nside_sky;
-    a.sky32 = c->sky32;
-    a.rings = c->rings;
-    a.sky64 = nullptr;
-    a.nside_beam = c->nside_beam;
-    a.npix_beam = (int)c->npix_beam;
-    a.beam32 = c->beam32;
-    a.beam64 = nullptr;
-    a.rho_max = c->rho_max;
-    a.begin = begin;
-    a.n = n;
-    a.ra = c->ra;
-    a.dec = c->dec;
-    a.pa = c->pa;
-    a.out_a = d_a;
-    a.out_b = d_b;
-    st = c->range_order(begin, n, s, &a.order);
-    if (st != PISCO_OK) return st;
-    a.out_f64 = out_dtype == PISCO_FLOAT64;
-    a.interp = (int)c->interp;
-    a.err = c->d_err;
-    a.fallbacks = c->d_fallbacks;
-    cudaError_t e;
-    const bool tuned = tuned_supported(c->nside_beam, (int)c->npix_beam, c->rho_max);
-    // PLAIN and FP64 with the nearest lookup walk the TUNED geometry's pairs
-    // (fwd_exact.cu); the bilinear lookup, and beams outside that geometry's
-    // domain (reaching beyond the polar cap of their grid), take the chain
-    const bool exact = tuned && c->interp == PISCO_BEAM_NEAREST;
-    void* plans = nullptr;
-    long long plan_cap = 0;
-    if (form == PISCO_FORM_FP64) {
-        st = wide_maps(c, s, a);
-        if (st != PISCO_OK) return st;
-        if (exact) {
-            c->plan_scratch(n, s, &plans, &plan_cap);
-            e = launch_forward_exact(a, true, c->sm_count, s, plans, plan_cap);
-        } else {
-            e = launch_forward_plain(a, true, c->sm_count, s);
-        }
-    } else if (form == PISCO_FORM_TUNED && tuned) {
-        CK(cudaMemsetAsync(c->d_fallbacks, 0, sizeof(unsigned long long), s), "reset fallbacks");
-        if (!tuned_plans_itself(n, c->sm_count)) c->plan_scratch(n, s, &plans, &plan_cap);
-        e = launch_forward_tuned(a, c->sm_count, s, plans, plan_cap);
-    } else if (exact) {
-        c->plan_scratch(n, s, &plans, &plan_cap);
-        e = launch_forward_exact(a, false, c->sm_count, s, plans, plan_cap);
-    } else {
-        e = launch_forward_plain(a, false, c->sm_count, s);
-    }
-    if (plans) c->plans_used(s);
-    if (a.order) c->order_used(s);
-    if (e != cudaSuccess) return cuda_fail(c, e, "forward launch");
-    if (s != c->stream) {
-        cudaEvent_t ev;
-        CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
-        cudaEventRecord(ev, s);
-        cudaStreamWaitEvent(c->stream, ev, 0);
-        cudaEventDestroy(ev);
-    }
-    return PISCO_OK;
+    if (form == PISCO_FORM_TUNED) return fail(c, PISCO_ERR_INVALID_ARGUMENT, "the chain runs in PLAIN or FP64");
+    return forward(c, form, true, begin, n, d_a, d_b, out_dtype, stream);
 }
 
 pisco_status pisco_memory_used(const pisco_ctx* c, size_t* bytes)
