@@ -134,11 +134,6 @@ struct ScatterBeam {
         scatter(p.ga, p.gb, pix, fetch(pix), B, bp, c2, s2);
     }
     __device__ __forceinline__ float4 fetch(int pix) const { return __ldg(&sky[pix]); }
-    __device__ __forceinline__ void pair(int pix, const float4& S, const F8& B, int bp, float c2,
-                                         float s2) const
-    {
-        scatter(ga, gb, pix, S, B, bp, c2, s2);
-    }
 
     // The pairs of a warp.  A scattered atomic costs the path from L1 to L2 a
     // sector each, a cycle and more, whatever it adds there, so lanes share
@@ -368,12 +363,6 @@ struct ScatterParams {
         }
         if (U.in0) add(ga, gb, U.S0, c0, s0, U.bp0, 1.0f);
         if (U.in1) add(ga, gb, U.S1, c1, s1, U.bp1, 1.0f);
-    }
-    __device__ __forceinline__ void pair(int pix, const float4& S, const F8& B, int bp, float c2,
-                                         float s2)
-    {
-        if (want_sky) sc.scatter(ga, gb, pix, B, c2, s2);
-        add(ga, gb, S, c2, s2, bp, 1.0f);
     }
     __device__ __forceinline__ void deferred(const tuned::Pend& p, int pix, const F8& B, int bp,
                                             float c2, float s2, float&, float&)

@@ -155,9 +155,13 @@ cudaError_t launch(int ndets, const double* dx, const double* dy, const double* 
                    double* yo, double* ro, cudaStream_t st)
 {
     if (ndets <= 0 || ns <= 0) return cudaSuccess;
-    // as many detectors per thread as leave about 16 warps for each of 152 SMs
+    int device = 0, sms = 1;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return e;
+    // as many detectors per thread as leave about 16 warps for each SM
     const long long parts = (ns + kThreads - 1) / kThreads;
-    long long group = parts * ndets / (152 * 16 * 32 / kThreads);
+    long long group = parts * ndets / (sms * 16LL * 32 / kThreads);
     group = group < 1 ? 1 : (group > kMostDets ? kMostDets : group);
     const long long items = parts * ((ndets + group - 1) / group);
     focal_plane_kernel<<<(int)(items < 16384 ? items : 16384), kThreads, 0, st>>>(

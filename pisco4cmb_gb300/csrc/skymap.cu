@@ -48,6 +48,7 @@ struct pisco_map {
     int device = 0;
     int nside = 0;
     long long npix = 0;
+    int sm_count = 1;
     cudaStream_t stream = nullptr;
     std::string error;
     double* acc = nullptr;  // kAcc x npix
@@ -519,7 +520,7 @@ pisco_status accumulate(pisco_map* m, long long ns, int ndet, const T* ra, const
     MCK(cudaMemsetAsync(bad, 0, sizeof(unsigned int), st), "reset check");
     // a persistent grid: a block's table takes as long as some of its values
     const long long blocks = std::min<long long>((total + 255) / 256, 8192);
-    map_keys_kernel<T><<<(int)std::min<long long>(blocks, 1216), kKeyThreads, 0, st>>>(
+    map_keys_kernel<T><<<(int)std::min<long long>(blocks, 8 * m->sm_count), kKeyThreads, 0, st>>>(
         total, ns, m->nside, ra, dec, pa, data, pol, keys, pos, rec, bad);
     MCK(cudaGetLastError(), "map keys");
     size_t tb = m->cap[kTmp];
@@ -571,6 +572,7 @@ pisco_status pisco_map_create(int nside, int device, pisco_map** out)
     m->nside = nside;
     m->npix = 12LL * nside * nside;
     cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&m->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&m->acc, sizeof(double) * kAcc * m->npix);
     if (e == cudaSuccess) e = cudaMalloc(&m->iqu, sizeof(float) * 3 * m->npix);

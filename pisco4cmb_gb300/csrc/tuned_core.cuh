@@ -60,9 +60,11 @@
 //   void reset(), total(a, b) main-pass sums (kSums)
 //   P fetch(int pix)          per-pixel data the action needs (Gather: the sky)
 //   void pair(int pix, P fetched, const F8& beam, int bp, float c2, float s2)
-//   void pair2(...)           optional: two neighbouring pixels at once
-//   void pair_all(...)        optional: every lane calls, with or without a
-//                             pair of its own (lanes share the atomics' sectors)
+//   void pair2(...)           in place of pair with the nearest lookup: two
+//                             neighbouring pixels at once
+//   void pair_all(...)        in place of pair: every lane calls, with or
+//                             without a pair of its own (lanes share the
+//                             atomics' sectors)
 //   void pair64(...)          optional: the phasor in FP64 or, with a member
 //                             type TwoFloat, in two-float arithmetic
 //   void stash(Pend&)         per-sample data a queued pair needs later
