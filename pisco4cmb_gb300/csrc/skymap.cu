@@ -121,6 +121,10 @@ __device__ __forceinline__ void split(double x, float& h, float& l)
     l = (float)(x - (double)h);
 }
 
+// |dec| <= pi/2 (a float is, if it is at most the largest one below pi/2).
+__device__ __forceinline__ bool is_latitude(float dec) { return fabsf(dec) <= 1.57079625f; }
+__device__ __forceinline__ bool is_latitude(double dec) { return fabs(dec) <= kHalfPi; }
+
 // ang2pix(pi/2 - dec, ra) for |ra| < 1e4 and |dec| <= pi/2 in FP32 (the
 // longitude in two-float arithmetic): -1 where a decision lies within the FP32
 // error of an integer (or |z| of 2/3), and ang2pix itself has to take it.  FP64
@@ -236,7 +240,8 @@ __device__ __forceinline__ Turn turn(int k)
 // rest in one double each 0.52 and 2.4).
 __device__ __forceinline__ void sincos_table(double x, const Turn* tab, double* s, double* c)
 {
-    if (!(fabs(x) < 1e5)) {
+    // |x| < 1e5 by its high word: FP64 comparisons queue for the FP64 pipe
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x40f86a00) {
         sincos(x, s, c);
         return;
     }
@@ -271,15 +276,15 @@ __global__ void __launch_bounds__(kKeyThreads) map_keys_kernel(long long total, 
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
         const int det = (int)((unsigned)e / (unsigned)ns);  // total < 2^31
-        const double r = (double)ra[e], dc = (double)dec[e];
         // the reference's arithmetic (skymap.cpp:85-101), FP64, no contraction
         const double psi = -PD_ADD((double)pol[det], (double)pa[e]);
         const double twopsi = PD_MUL(2.0, psi);
         double s, c;
         sincos_table(twopsi, tab, &s, &c);
         long long p = -1;
-        if (fabs(dc) <= kHalfPi && fabs((float)ra[e]) < 1e4f) p = quick_ang2pix(nside, ra[e], dec[e]);
+        if (is_latitude(dec[e]) && fabsf((float)ra[e]) < 1e4f) p = quick_ang2pix(nside, ra[e], dec[e]);
         if (p < 0) {
+            const double r = (double)ra[e], dc = (double)dec[e];
             const double theta = PD_SUB(kHalfPi, dc);
             p = h.npix;  // sentinel: sorted last, never accumulated
             if (isfinite(r) && isfinite(theta) && theta >= 0.0 && theta <= kPi) p = ang2pix(h, theta, r);
