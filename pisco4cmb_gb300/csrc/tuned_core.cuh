@@ -281,6 +281,13 @@ __device__ __forceinline__ FF operator*(float a, FF b)
     const float p = __fmul_rn(a, b.h);
     return ff_quick(p, fmaf(a, b.l, fmaf(a, b.h, -p)));
 }
+// c + a b for |c| >= |a b| (2^-47 of c; l is not reduced below half an ulp of h)
+__device__ __forceinline__ FF ff_horner(FF c, FF a, FF b)
+{
+    const float p = __fmul_rn(a.h, b.h);
+    const FF s = ff_quick(c.h, p);
+    return FF{s.h, __fadd_rn(s.l, fmaf(a.h, b.l, fmaf(a.l, b.h, fmaf(a.h, b.h, -p))) + c.l)};
+}
 
 // The same of a PLAIN sample: ring constants and frame.
 struct RingF {
@@ -1417,7 +1424,7 @@ __device__ __forceinline__ RingF ring_two_float(float near, float f, float e, co
 // within 1/2 (middle) sin x and 1 - cos x are good to 4e-13, by one series whose
 // third term takes a second float in the middle range (with one it left 1e-10
 // there); beyond, FP64's sincos (20,000 samples at 60 to 74 degrees, 5 degree
-// beam: 145 us with one float, 147 with two, 350 with sincos from 1/8 on).
+// beam: 145 us, 350 with sincos from 1/8 on).
 __device__ __forceinline__ void phasor_two_float(const RingF& R, float kf, bool narrow, bool middle,
                                                  FF s0, FF c2p, FF s2p, float& c2, float& s2)
 {
@@ -1434,13 +1441,13 @@ __device__ __forceinline__ void phasor_two_float(const RingF& R, float kf, bool 
             a = ff_quick(-0.16666667f, fmaf(x2.h, fmaf(x2.h, p, 8.33333333e-3f), 4.9670537e-9f));
             b = ff_quick(-0.041666668f, fmaf(x2.h, fmaf(x2.h, q, 1.38888889e-3f), 1.2417634e-9f));
         } else {
-            a = FF{-0.16666667f, 4.9670537e-9f} +
-                x2 * ff_quick(8.33333377e-3f, fmaf(x2.h, p, -4.346172e-10f));
-            b = FF{-0.041666668f, 1.2417634e-9f} +
-                x2 * ff_quick(1.38888892e-3f, fmaf(x2.h, q, -3.3631094e-11f));
+            a = ff_horner(FF{-0.16666667f, 4.9670537e-9f}, x2,
+                          ff_quick(8.33333377e-3f, fmaf(x2.h, p, -4.346172e-10f)));
+            b = ff_horner(FF{-0.041666668f, 1.2417634e-9f}, x2,
+                          ff_quick(1.38888892e-3f, fmaf(x2.h, q, -3.3631094e-11f)));
         }
-        sn = x + x * (x2 * a);
-        h = x2 * (FF{0.5f, 0.0f} + x2 * b);
+        sn = ff_horner(x, x, x2 * a);
+        h = x2 * ff_horner(FF{0.5f, 0.0f}, x2, b);
     } else {
         double s, c;
         sincos((double)x.h + (double)x.l, &s, &c);
