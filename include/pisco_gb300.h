@@ -294,7 +294,7 @@ pisco_status pisco_set_batched_config(pisco_ctx* ctx, int chunk, int warps_per_b
  * callbacks, services whose memory pool owns the whole GPU): the batched
  * TUNED forward with every buffer supplied by the caller and its own
  * working memory (sky ring table, work queue, descriptors, counters) in a
- * fixed array of about 2.6 MB compiled into the library, shared by all calls.  No context;
+ * fixed array of about 2.1 MB compiled into the library, shared by all calls.  No context;
  * calls no allocator.  Synchronous (returns when the TOD is written).
  * Limits: at most PISCO_NOALLOC_MAX_DETS detector pairs and at most
  * PISCO_NOALLOC_MAX_ITEMS work items, sum over pairs of

@@ -56,8 +56,11 @@ struct Scatter {
 
     // v 2^S rounded to the nearest integer.  The scale is a power of two, so
     // the FP32 product is exact and the FP32 -> int64 conversion gives what
-    // the FP64 route would, without two FP64 instructions per component (the
-    // FP64 pipe of this GPU issues a small fraction of the FP32 rate).
+    // the FP64 route would, without two FP64 instructions per component.  The
+    // conversion itself goes through the FP64 pipe, one instruction per value, and
+    // bounds the DETERMINISTIC kernels: 11 per warp and pair in the sky and
+    // beam-map gradient, which keep that pipe 73 % busy (its atomics the path
+    // from L1 to L2 48 %; 38.7M pairs 1.04 ms).
     __device__ __forceinline__ static unsigned long long fx(float v, float scale)
     {
         return (unsigned long long)__float2ll_rn(v * scale);
@@ -136,7 +139,8 @@ struct ScatterBeam {
     __device__ __forceinline__ float4 fetch(int pix) const { return __ldg(&sky[pix]); }
 
     // The pairs of a warp.  A scattered atomic costs the path from L1 to L2 a
-    // sector each, a cycle and more, whatever it adds there, so lanes share
+    // sector each, a cycle and more, whatever it adds there (which bounded this
+    // kernel before; now fx's conversions do), so lanes share
     // sectors: four lanes turn their 4 x 4 values around and add the four
     // 64-bit words of one detector's half pixel (a sector) at a time, two
     // lanes the two float4s of a pixel: 64 sectors for 32 pairs instead of 192.

@@ -10,13 +10,14 @@
 // in FP64.
 //
 // What bounds it: the FP64 pipe, which takes 16 cycles per warp instruction on
-// an SM.  plain_kernel (fwd_plain.cu) evaluates the chain's ten transcendental
-// functions for every pair, about 600 FP64 instructions; here a pair takes
-// about 60 (FP64 form) or, with some 260 FP32 ones, 4 (PLAIN).  nside 64, 5
-// degree beam, PLAIN, 20,000 samples: 1.9 ms in plain_kernel, 373 us with the
-// FP64 phasor, 124 us now; nside 2048, 1 degree, FP64 form, 6,001 samples: 21.3
-// -> 2.9 ms.  The bilinear lookup and beams outside the domain stay on
-// plain_kernel.
+// an SM (FP64 form 83 % busy).  plain_kernel (fwd_plain.cu) evaluates the chain's
+// ten transcendental functions for every pair, about 600 FP64 instructions; here
+// a pair takes about 56 (FP64 form) or, with some 240 FP32 ones, 4 (PLAIN), which
+// at 93 pairs per sample has the FP64 pipe 60 % busy and issues in 46 % of the
+// cycles.  nside 64, 5 degree beam, PLAIN, 20,000 samples: 2.1 ms in
+// plain_kernel, 373 us with the FP64 phasor, 120 us now; nside 2048, 1 degree,
+// FP64 form, 6,001 samples: 21.3 -> 2.9 ms.  The bilinear lookup and beams outside
+// the domain stay on plain_kernel.
 #include "tuned_core.cuh"
 
 namespace pisco {

@@ -185,7 +185,7 @@ void launch_plans(const FwdArgs& a, tuned::SamplePlan* plans, long long pos0, lo
                   cudaStream_t st)
 {
     // small blocks, so that a short launch's plans spread over the SMs: a plan
-    // is a chain of some 200 FP64 instructions, and the warps of an SM queue for
+    // is a chain of some 180 FP64 instructions, and the warps of an SM queue for
     // its FP64 pipe
     const long long b = (pos1 - pos0 + 127) / 128;
     plan_kernel<<<(int)(b < 65536 ? b : 65536), 128, 0, st>>>(a, plans, pos0, pos1);

@@ -12,9 +12,9 @@
 // library.
 //
 // The working memory is g_noalloc_scratch below: a file-scope
-// static __device__ array of kScratchBytes (about 2.6 MB).  Every GPU that
+// static __device__ array of kScratchBytes (about 2.1 MB).  Every GPU that
 // loads the library holds it until the process exits.  It holds the sky
-// ring table (2.1 MB, sized for nside 8192), the
+// ring table (1.6 MB, sized for nside 8192), the
 // detector descriptors (at most PISCO_NOALLOC_MAX_DETS), the work items (at
 // most PISCO_NOALLOC_MAX_ITEMS), the queue counter, the device error word
 // and the FP64-fallback counter.  All calls share it and it keeps the last
@@ -60,6 +60,7 @@ struct Scratch {
     unsigned long long fallbacks;
 };
 constexpr size_t kScratchBytes = sizeof(Scratch);
+static_assert(kScratchBytes > 2'000'000 && kScratchBytes < 2'200'000, "about 2.1 MB, as documented");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 

@@ -21,11 +21,11 @@
 // boresight-frame components, the beam grid's polar-cap indices and
 // exp(2i chi) as a product of unit phasors.  Any of the three floor decisions
 // lying within the margin of an integer, and any pair within 2e-6 rad of the
-// boresight, is queued and decided in FP64: by the small-offset form in FP64
-// with Newton steps instead of transcendental functions (quick_pair), or,
-// where that too is close to an edge, with the FP64 chain of the PLAIN form
-// (hpx.cuh pair_beam_pixel), so every pair lands on the same beam pixel as in
-// PLAIN.
+// boresight, is queued and decided in FP64: by the small-offset form with one
+// sine and cosine and one arctangent (quick_pair), or, where that too is close
+// to an edge or to the boresight, with the reference's FP64 chain (hpx.cuh
+// pair_beam_pixel), so every pair lands on the chain's beam pixel
+// (pisco_debug_decisions compares them).
 //
 // The queue outlives the sample: each entry names a per-warp slot holding its
 // sample's FP64 frame and output, and the warp redoes 32 entries at a time,
@@ -94,7 +94,8 @@
 // Warps per block of the adjoint's and the diagnostics' kernels, and the
 // minimum number of resident blocks per SM requested from the compiler (which
 // caps their registers at 65536 / (32 x warps x blocks)); the adjoint's
-// planned nearest-lookup instances take 4 blocks (adjoint_kernels.cuh).
+// planned nearest-lookup instances take 2, 3 or 4 (adjoint_kernels.cuh
+// adj_warps_per_sm).
 #ifndef PISCO_TUNED_WARPS
 #define PISCO_TUNED_WARPS 8
 #endif
@@ -136,8 +137,9 @@ template <class A, class = void>
 struct HasPair2 : std::false_type {};
 template <class A>
 struct HasPair2<A, std::void_t<decltype(&A::pair2)>> : std::true_type {};
-// Decisions whose FP32 value lies within kMarginRel * (value + 1) of an
-// integer are redone in FP64 (about 20 FP32 ulps).  The observed worst case
+// Decisions whose FP32 value lies within kMarginRel * (r + 2) of an integer (r:
+// the pair's ring position; the values are at most r + 1) are redone in FP64
+// (about 20 FP32 ulps).  The observed worst case
 // over a workload is measured by pisco_tuned_calibrate and must stay well
 // below this bound.
 constexpr float kMarginRel = 1.2e-6f;
@@ -198,7 +200,7 @@ struct alignas(16) Pend {
 // edge formula's constants), the boresight frame and the psi phasors.  Built
 // by make_plan, either inside the pair kernel (one warp per sample, every
 // lane redundantly) or beforehand by plan_kernel with one thread per sample:
-// it is FP64 work (about three hundred FP64 instructions), which GB300 runs
+// it is FP64 work (some 180 FP64 instructions), which GB300 runs
 // at a small fraction of its FP32 rate.  96 bytes.
 struct alignas(16) SamplePlan {
     // disc, for disc_ring's exact formula: cos(theta), 1 / sin(theta), longitude
@@ -492,8 +494,9 @@ __device__ __forceinline__ int small_float_to_int(float f)
     return __float_as_int(f + 12582912.0f) - 0x4B400000;
 }
 
-// 1/x by the MUFU reciprocal approximation (relative error below 2^-22);
-// used only for values, never for an index decision.
+// 1/x by the MUFU reciprocal approximation (relative error below 2^-22).  What
+// it decides (sigma in quarter_turns, hence the beam pixel) has that error within
+// the margin of the decisions.
 __device__ __forceinline__ float rcp_approx(float x)
 {
     float r;
@@ -1418,7 +1421,7 @@ __device__ __forceinline__ RingF ring_two_float(float near, float f, float e, co
 }
 
 // exp(2i chi) rounded to FP32: its error before that rounding, some 1e-12 at
-// rho of a degree, is far below what moves the rounded value.  About 260 FP32
+// rho of a degree, is far below what moves the rounded value.  About 240 FP32
 // instructions, the time of four FP64 ones; the 45 FP64 instructions of
 // phasor_exact took two thirds of a PLAIN launch.  Within 1/8 rad (narrow) and
 // within 1/2 (middle) sin x and 1 - cos x are good to 4e-13, by one series whose
