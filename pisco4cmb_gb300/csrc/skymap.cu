@@ -123,7 +123,12 @@ __device__ __forceinline__ void split(double x, float& h, float& l)
 
 // |dec| <= pi/2 (a float is, if it is at most the largest one below pi/2).
 __device__ __forceinline__ bool is_latitude(float dec) { return fabsf(dec) <= 1.57079625f; }
-__device__ __forceinline__ bool is_latitude(double dec) { return fabs(dec) <= kHalfPi; }
+// A double by its words: FP64 comparisons queue for the FP64 pipe.
+__device__ __forceinline__ bool is_latitude(double dec)
+{
+    const int hi = __double2hiint(dec) & 0x7fffffff;
+    return hi < 0x3ff921fb || (hi == 0x3ff921fb && (unsigned)__double2loint(dec) <= 0x54442d18u);
+}
 
 // ang2pix(pi/2 - dec, ra) for |ra| < 1e4 and |dec| <= pi/2 in FP32 (the
 // longitude in two-float arithmetic): -1 where a decision lies within the FP32
@@ -233,11 +238,11 @@ __device__ __forceinline__ Turn turn(int k)
     }
 }
 
-// sin and cos of x in 22 FP64 instructions (CUDA's takes some 45): the nearest
+// sin and cos of x in 20 FP64 instructions (CUDA's takes some 45): the nearest
 // multiple k of pi/64 from a table, the rest, at most 0.0246, by the Taylor
 // series (truncated below 4e-18), the largest parts added last.  Against 128-bit
-// values 0.29 ulp rms and 0.78 at worst (CUDA's 0.37 and 1.4; with table and
-// rest in one double each 0.52 and 2.4).
+// values 0.29 ulp rms and 1.06 at worst (CUDA's 0.37 and 1.4; with the table in
+// one double 0.52 and 2.4).
 __device__ __forceinline__ void sincos_table(double x, const Turn* tab, double* s, double* c)
 {
     // |x| < 1e5 by its high word: FP64 comparisons queue for the FP64 pipe
@@ -249,10 +254,9 @@ __device__ __forceinline__ void sincos_table(double x, const Turn* tab, double* 
     const double k = t - 6755399441055744.0;
     const Turn v = tab[__double2loint(t) & 127];
     // pi/64 as the sum of two doubles
-    const double r1 = fma(-k, 0.04908738521234052, x), r = fma(-k, 1.9135106236677394e-18, r1);
-    const double rl = fma(-k, 1.9135106236677394e-18, r1 - r);  // what r leaves out
+    const double r = fma(-k, 1.9135106236677394e-18, fma(-k, 0.04908738521234052, x));
     const double r2 = r * r;
-    const double sr = fma(r * r2, fma(r2, fma(r2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), rl);  // sin - r
+    const double sr = r * r2 * fma(r2, fma(r2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0);  // sin r - r
     const double cr = r2 * fma(r2, fma(r2, -1.0 / 720.0, 1.0 / 24.0), -0.5);  // cos r - 1
     *s = v.s + fma(v.c, r, fma(v.c, sr, fma(v.s, cr, v.s_lo)));
     *c = v.c + fma(-v.s, r, fma(-v.s, sr, fma(v.c, cr, v.c_lo)));
