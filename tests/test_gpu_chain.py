@@ -86,3 +86,37 @@ def test_chain_is_the_bilinear_forms_own_kernel(gpu):
     with pytest.raises(PiscoInvalidArgument):
         conv.debug_forward_chain(0, 0, form="tuned")
     conv.close()
+
+
+def test_longest_rings_follow_the_chain(gpu):
+    """nside 8192, rings of 2^15 pixels: PLAIN and TUNED against PLAIN's chain (TUNED: both round to
+    FP32), and every pair's pixel."""
+    import torch
+
+    from pisco4cmb_gb300 import GPUConvolver, Scan, beam_npix_for_radius
+
+    nside, n = 8192, 300
+    g = torch.Generator("cuda").manual_seed(1)
+    sky = torch.randn((12 * nside * nside, 4), generator=g, device="cuda")
+    conv = GPUConvolver()
+    conv.set_sky_device(nside, sky.data_ptr(), False, stream=1)
+    torch.cuda.synchronize()
+    del sky
+    torch.cuda.empty_cache()
+    rng = np.random.default_rng(2)
+    npix = beam_npix_for_radius(8192, np.deg2rad(0.25))
+    maps = rng.normal(size=(8, npix)).astype(np.float32)
+    conv.set_beam_planes(8192, npix, maps[:4], maps[4:])
+    dec = np.concatenate([rng.uniform(-0.7, 0.7, n - 80), np.pi / 2 - rng.uniform(0, 5e-3, 40),
+                          rng.uniform(1.3, 1.55, 40)])
+    conv.update_scan(Scan(n, rng.uniform(-5e-3, 5e-3, n), dec, rng.uniform(0, np.pi, n)))
+    ref = _tod(lambda t: (conv.debug_forward_chain(t[0].data_ptr(), t[1].data_ptr(), form="plain"),
+                          conv.sync()), n)
+    for form in ("plain", "tuned"):
+        got = _tod(lambda t: (conv.forward_device(t[0].data_ptr(), t[1].data_ptr(), out_f64=True, form=form),
+                              conv.sync()), n)
+        assert (got - ref).abs().max().item() < TOL[form] * ref.std().item(), form
+        check = conv.debug_decisions(form)
+        assert check.pairs == conv.count_pairs() and check.differing == 0
+        assert check.worst_fp32 < 0.5 and check.worst_fp64 < 0.5
+    conv.close()
